@@ -275,35 +275,42 @@ int make_plan(const stc_HACApK_leafmtxp *st, int nd, int num_ctas, Plan &plan, s
       }
     }
   }
-  // D blocks (one per atom, possibly empty) and U blocks (atoms with low-rank rows)
+  // D blocks (one per atom, possibly empty) and U blocks (atoms with low-rank
+  // rows), in atom order, a D block's pieces before its U block's
   std::vector<uint32_t> dblock(natoms), ublock(natoms, 0xffffffffu);
   std::vector<uint64_t> acost(natoms, 0);
+  {
+    size_t nb = plan.blocks.size();
+    for (int a = 0; a < natoms; ++a) {
+      dblock[a] = (uint32_t)nb++;
+      if (ucnt[a + 1] > ucnt[a]) ublock[a] = (uint32_t)nb++;
+    }
+    plan.blocks.resize(nb);
+    plan.pieces.resize((size_t)dcnt[natoms] + ucnt[natoms]);
+  }
+#pragma omp parallel for schedule(dynamic, 64)
   for (int a = 0; a < natoms; ++a) {
-    Block b{kRunD, (uint16_t)atoms[a].h, (uint32_t)a, 0, 0, (uint32_t)plan.pieces.size(), 0};
+    uint32_t at = dcnt[a] + ucnt[a];
+    Block b{kRunD, (uint16_t)atoms[a].h, (uint32_t)a, 0, 0, at, dcnt[a + 1] - dcnt[a]};
     for (uint32_t q = dcnt[a]; q < dcnt[a + 1]; ++q) {
       const stc_HACApK_leafmtx *s = leaf_at(st, (int)dleaf[q]);
-      plan.pieces.push_back(Piece{dleaf[q], 0, (uint32_t)s->ndt, (uint32_t)(s->nstrtt - 1)});
+      plan.pieces[at++] = Piece{dleaf[q], 0, (uint32_t)s->ndt, (uint32_t)(s->nstrtt - 1)};
       b.W += (uint32_t)s->ndt;
-      b.npiece++;
     }
-    dblock[a] = (uint32_t)plan.blocks.size();
-    plan.blocks.push_back(b);
+    plan.blocks[dblock[a]] = b;
     acost[a] = block_cost(b.h, b.W, precision, costs);
-    if (ucnt[a + 1] > ucnt[a]) {
-      // zbu order, so that the segments of one column group merge
-      std::sort(uleaf.begin() + ucnt[a], uleaf.begin() + ucnt[a + 1],
-                [&](uint32_t x, uint32_t y) { return plan.zoff[x] < plan.zoff[y]; });
-      Block u{kRunU, (uint16_t)atoms[a].h, (uint32_t)a, 0, 0, (uint32_t)plan.pieces.size(), 0};
-      for (uint32_t q = ucnt[a]; q < ucnt[a + 1]; ++q) {
-        const stc_HACApK_leafmtx *s = leaf_at(st, (int)uleaf[q]);
-        plan.pieces.push_back(Piece{uleaf[q], 0, (uint32_t)s->kt, (uint32_t)plan.zoff[uleaf[q]]});
-        u.W += (uint32_t)s->kt;
-        u.npiece++;
-      }
-      ublock[a] = (uint32_t)plan.blocks.size();
-      plan.blocks.push_back(u);
-      acost[a] += block_cost(u.h, u.W, precision, costs);
+    if (ublock[a] == 0xffffffffu) continue;
+    // zbu order, so that the segments of one column group merge
+    std::sort(uleaf.begin() + ucnt[a], uleaf.begin() + ucnt[a + 1],
+              [&](uint32_t x, uint32_t y) { return plan.zoff[x] < plan.zoff[y]; });
+    Block u{kRunU, (uint16_t)atoms[a].h, (uint32_t)a, 0, 0, at, ucnt[a + 1] - ucnt[a]};
+    for (uint32_t q = ucnt[a]; q < ucnt[a + 1]; ++q) {
+      const stc_HACApK_leafmtx *s = leaf_at(st, (int)uleaf[q]);
+      plan.pieces[at++] = Piece{uleaf[q], 0, (uint32_t)s->kt, (uint32_t)plan.zoff[uleaf[q]]};
+      u.W += (uint32_t)s->kt;
     }
+    plan.blocks[ublock[a]] = u;
+    acost[a] += block_cost(u.h, u.W, precision, costs);
   }
 
   // ---- balance: P slabs first (they gate the grid barrier), then atoms
@@ -322,33 +329,60 @@ int make_plan(const stc_HACApK_leafmtxp *st, int nd, int num_ctas, Plan &plan, s
     for (int a : aorder) cta_atoms[bins.take(acost[a])].push_back((uint32_t)a);
   }
 
-  // ---- emit run records and stream offsets per CTA
+  // ---- emit run records and stream offsets per CTA.  The CTAs' blocks and
+  // atoms first, one CTA after the other; then every CTA's records on its own
+  // (all host cores); then the records and streams back to back.
   plan.ctas.resize(num_ctas);
-  uint64_t off = 0;
-  std::vector<Seg> segs;
+  struct Cta {
+    std::vector<uint32_t> split;       // atoms with separate D and U blocks
+    std::vector<uint32_t> merged;      // atoms with one kRunDU block ...
+    uint32_t merged_block = 0;         // ... the first of these in plan.blocks
+    std::vector<RunRec> recs;
+    std::vector<RunLite> lite;
+    uint64_t bytes = 0, pad = 0;
+    bool failed = false;
+  };
+  std::vector<Cta> work(num_ctas);
+  plan.atoms.reserve(natoms);
   for (int c = 0; c < num_ctas; ++c) {
-    auto &pl = cta_p[c];
     auto &al = cta_atoms[c];
-    std::sort(pl.begin(), pl.end());
+    std::sort(cta_p[c].begin(), cta_p[c].end());
     std::sort(al.begin(), al.end());
-    CtaInfo info{};
-    info.stream_off = off;
-    info.rec_begin = (uint32_t)plan.recs.size();
-    info.atom_begin = (uint32_t)plan.atoms.size();
-    info.n_atoms = (uint32_t)al.size();
     // merge_keep >= 0: atoms with low-rank rows past the first merge_keep
     // take one kRunDU block; the atom list follows the blocks' order
-    std::vector<uint32_t> split, merged;
-    {
-      uint32_t with_u = 0;
-      for (uint32_t a : al) {
-        const bool has_u = ublock[a] != 0xffffffffu;
-        if (merge_keep >= 0 && has_u && with_u++ >= (uint32_t)merge_keep) merged.push_back(a);
-        else split.push_back(a);
-      }
+    Cta &w = work[c];
+    uint32_t with_u = 0;
+    for (uint32_t a : al) {
+      const bool has_u = ublock[a] != 0xffffffffu;
+      if (merge_keep >= 0 && has_u && with_u++ >= (uint32_t)merge_keep) w.merged.push_back(a);
+      else w.split.push_back(a);
     }
-    for (uint32_t a : split) plan.atoms.push_back(atoms[a]);
-    for (uint32_t a : merged) plan.atoms.push_back(atoms[a]);
+    CtaInfo &info = plan.ctas[c];
+    info = CtaInfo{};
+    info.atom_begin = (uint32_t)plan.atoms.size();
+    info.n_atoms = (uint32_t)al.size();
+    info.nblk_p = (uint32_t)cta_p[c].size();
+    for (uint32_t a : w.split) plan.atoms.push_back(atoms[a]);
+    for (uint32_t a : w.merged) plan.atoms.push_back(atoms[a]);
+    w.merged_block = (uint32_t)plan.blocks.size();
+    for (uint32_t a : w.merged) {
+      const Block d = plan.blocks[dblock[a]], u = plan.blocks[ublock[a]];
+      plan.blocks.push_back(Block{kRunDU, d.h, d.a, 0, d.W + u.W, (uint32_t)plan.pieces.size(), d.npiece + u.npiece});
+      plan.pieces.resize(plan.pieces.size() + d.npiece + u.npiece);
+    }
+  }
+  auto emit_cta = [&](int c) {
+    Cta &w = work[c];
+    CtaInfo &info = plan.ctas[c];
+    for (size_t k = 0; k < w.merged.size(); ++k) {
+      const Block &m = plan.blocks[w.merged_block + k], &d = plan.blocks[dblock[w.merged[k]]],
+                  &u = plan.blocks[ublock[w.merged[k]]];
+      Piece *o = &plan.pieces[m.piece_begin];
+      std::copy_n(&plan.pieces[d.piece_begin], d.npiece, o);
+      std::copy_n(&plan.pieces[u.piece_begin], u.npiece, o + d.npiece);
+      for (uint32_t q = 0; q < u.npiece; ++q) o[d.npiece + q].vsrc |= kSegZbu;
+    }
+    std::vector<Seg> segs;
     uint64_t pos = 0;
     uint32_t rot = 0, rot_step = 0;
     auto emit_block = [&](uint32_t bi) -> uint32_t {
@@ -395,7 +429,7 @@ int make_plan(const stc_HACApK_leafmtxp *st, int nd, int num_ctas, Plan &plan, s
         r.block = bi;
         r.col0 = col;
         std::copy(segs.begin(), segs.end(), rec.seg);
-        plan.recs.push_back(rec);
+        w.recs.push_back(rec);
         RunLite L{};
         L.pos = r.pos;
         L.out = r.out;
@@ -404,8 +438,8 @@ int make_plan(const stc_HACApK_leafmtxp *st, int nd, int num_ctas, Plan &plan, s
         L.rot = (uint8_t)r.rot;
         L.rot_step = (uint16_t)rot_step;
         L.flags = r.flags;
-        plan.lite.push_back(L);
-        plan.pad_bytes += (uint64_t)elem_bytes(precision) * b.h * (nc - r.vlen);
+        w.lite.push_back(L);
+        w.pad += (uint64_t)elem_bytes(precision) * b.h * (nc - r.vlen);
         pos += 16ull * b.h * r.npanel;
         rot = (rot + r.npanel) % kProductWarps;
         rot_step = (rot_step + r.npanel) % kStepWarps;
@@ -414,27 +448,31 @@ int make_plan(const stc_HACApK_leafmtxp *st, int nd, int num_ctas, Plan &plan, s
       } while (col < Wp);
       return nr;
     };
-    for (uint32_t b : pl) info.nr_p += emit_block(b);
-    info.nblk_p = (uint32_t)pl.size();
-    for (uint32_t a : split) info.nr_d += emit_block(dblock[a]);
-    for (uint32_t a : split)
+    for (uint32_t b : cta_p[c]) info.nr_p += emit_block(b);
+    for (uint32_t a : w.split) info.nr_d += emit_block(dblock[a]);
+    for (uint32_t a : w.split)
       if (ublock[a] != 0xffffffffu) info.nr_u += emit_block(ublock[a]);
-    for (uint32_t a : merged) {
-      const Block d = plan.blocks[dblock[a]], u = plan.blocks[ublock[a]];
-      Block m{kRunDU, d.h, d.a, 0, d.W + u.W, (uint32_t)plan.pieces.size(), d.npiece + u.npiece};
-      for (uint32_t q = 0; q < d.npiece; ++q) {
-        const Piece pc = plan.pieces[d.piece_begin + q];
-        plan.pieces.push_back(pc);
-      }
-      for (uint32_t q = 0; q < u.npiece; ++q) {
-        Piece pc = plan.pieces[u.piece_begin + q];
-        pc.vsrc |= kSegZbu;
-        plan.pieces.push_back(pc);
-      }
-      plan.blocks.push_back(m);
-      info.nr_u += emit_block((uint32_t)plan.blocks.size() - 1);
+    for (size_t k = 0; k < w.merged.size(); ++k) info.nr_u += emit_block(w.merged_block + (uint32_t)k);
+    w.bytes = pos;
+    info.stream_bytes = (uint32_t)pos;  // a multiple of 16 by construction
+  };
+#pragma omp parallel for schedule(dynamic, 1)
+  for (int c = 0; c < num_ctas; ++c) {
+    try {  // an exception must not leave the parallel region
+      emit_cta(c);
+    } catch (...) {
+      work[c].failed = true;
     }
-    if (pos > 0xfffffff0ull) {
+  }
+  uint64_t off = 0;
+  size_t nrec = 0;
+  for (int c = 0; c < num_ctas; ++c) {
+    CtaInfo &info = plan.ctas[c];
+    if (work[c].failed) {
+      err = "host memory for the run records";
+      return HBX_ERR_NOMEM;
+    }
+    if (work[c].bytes > 0xfffffff0ull) {
       err = "a CTA stream exceeds 4 GiB; use more CTAs";
       return HBX_ERR_INVALID;
     }
@@ -444,9 +482,18 @@ int make_plan(const stc_HACApK_leafmtxp *st, int nd, int num_ctas, Plan &plan, s
       err = "a CTA holds more than " + std::to_string(kMaxPairRuns) + " runs; use more CTAs";
       return HBX_ERR_INVALID;
     }
-    info.stream_bytes = (uint32_t)pos;  // a multiple of 16 by construction
-    plan.ctas[c] = info;
-    off += (pos + 255) & ~uint64_t(255);
+    info.stream_off = off;
+    info.rec_begin = (uint32_t)nrec;
+    off += (work[c].bytes + 255) & ~uint64_t(255);
+    nrec += work[c].recs.size();
+    plan.pad_bytes += work[c].pad;
+  }
+  plan.recs.resize(nrec);
+  plan.lite.resize(nrec);
+#pragma omp parallel for schedule(dynamic, 1)
+  for (int c = 0; c < num_ctas; ++c) {
+    std::copy(work[c].recs.begin(), work[c].recs.end(), plan.recs.begin() + plan.ctas[c].rec_begin);
+    std::copy(work[c].lite.begin(), work[c].lite.end(), plan.lite.begin() + plan.ctas[c].rec_begin);
   }
   plan.total_bytes = std::max<uint64_t>(off, 256);
   return HBX_OK;
