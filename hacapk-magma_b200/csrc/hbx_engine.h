@@ -209,6 +209,12 @@ constexpr size_t kNoallocCtlBytes = 256;
 constexpr uint64_t kNoallocZbuMax = (kNoallocScratchBytes - kNoallocCtlBytes) / sizeof(double);
 cudaError_t noalloc_scratch_address(void **ptr);
 
+// The packed stream of `plan` formed on the device from the host leaves
+// (hbx_pack.cu); a temporary of the leaves' size comes from `alloc`, whose
+// cudaErrorMemoryAllocation is returned with nothing written.
+cudaError_t pack_on_device(const stc_HACApK_leafmtxp *st, const Plan &plan, const RunRec *d_recs, const CtaInfo *d_ctas,
+                           uint8_t *d_stream, cudaError_t (*alloc)(void *, size_t));
+
 // Kernel launchers (hbx_kernels.cu).
 size_t kernel_smem_bytes();
 cudaError_t configure_kernels();

@@ -134,35 +134,35 @@ HBX_HD constexpr uint32_t stage_elem_bytes(int prec) { return prec == kFP64 ? 8u
 // significant bits whatever its magnitude.  Below 2^-126 the bfloat16
 // values are subnormal, multiples of 2^-133: the double is scaled to units
 // of 2^-133 (exactly) and rounded to the nearest integer, ties to even.
-inline uint16_t bf16_from_double(double v) {
+HBX_HD inline uint16_t bf16_from_double(double v) {
   uint64_t b;
-  std::memcpy(&b, &v, sizeof b);
+  memcpy(&b, &v, sizeof b);
   const uint64_t mag = b & 0x7fffffffffffffffull;
   const uint16_t sign = (uint16_t)((b >> 48) & 0x8000u);
   if (mag >= 0x7ff0000000000000ull) {  // inf / nan
     const float f = (float)v;
     uint32_t u;
-    std::memcpy(&u, &f, sizeof u);
+    memcpy(&u, &f, sizeof u);
     if ((u & 0x7fffffffu) > 0x7f800000u) return (uint16_t)((u >> 16) | 0x40u);  // quiet nan
     return (uint16_t)(u >> 16);
   }
   if (mag < 0x3810000000000000ull) {  // below 2^-126
     double m;
-    std::memcpy(&m, &mag, sizeof m);
-    const double q = std::ldexp(m, 133);  // < 128, exact
-    double k = std::floor(q);
+    memcpy(&m, &mag, sizeof m);
+    const double q = ldexp(m, 133);  // < 128, exact
+    double k = floor(q);
     const double f = q - k;                // exact
-    if (f > 0.5 || (f == 0.5 && std::fmod(k, 2.0) != 0.0)) k += 1.0;
+    if (f > 0.5 || (f == 0.5 && fmod(k, 2.0) != 0.0)) k += 1.0;
     return (uint16_t)(sign | (uint16_t)k);  // k == 128 is the smallest normal, 2^-126
   }
   // keep 7 fraction bits of the 52: round the low 45 bits to nearest, ties to even
   b += (1ull << 44) - 1ull + ((b >> 45) & 1ull);
   b &= ~((1ull << 45) - 1ull);
   double r;
-  std::memcpy(&r, &b, sizeof r);
+  memcpy(&r, &b, sizeof r);
   const float f = (float)r;  // exact, or +-inf past float's range
   uint32_t u;
-  std::memcpy(&u, &f, sizeof u);
+  memcpy(&u, &f, sizeof u);
   return (uint16_t)(u >> 16);
 }
 inline float bf16_to_float(uint16_t h) {  // host side (the kernels shift in registers)
