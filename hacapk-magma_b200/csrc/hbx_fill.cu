@@ -19,6 +19,7 @@
 // writes it; only the device's atan2 and log may differ from the host C
 // library's in the last bit.
 #include <cuda_runtime.h>
+#include <sys/mman.h>
 
 #include <algorithm>
 #include <cstdio>
@@ -31,16 +32,19 @@
 #include <vector>
 
 #include "../../include/hacapk_b200.h"
+#include "hbx_stage.h"
 
 namespace hbx {
 namespace {
 
+// The faces in cluster order, one array per value (kGeom arrays of n), so that
+// the entries of a row or a column read neighbouring words: vertices x0 x1 x2
+// y0 y1 y2 z0 z1 z2, centroid x y z, unit normal x y z.
+constexpr int kGeom = 15;
 struct FillGeom {
-  const double *fv;   // [nofc][9]: the face's vertex x0 x1 x2 y0 y1 y2 z0 z1 z2
-  const double *zg;   // [3][nofc]: centroids (column-major zgmid)
-  const int *lod;     // [nofc]: 1-based face id of each cluster-order position
-  int nofc;
-  int kernel;         // HBX_FILL_KERNEL_*
+  const double *f;
+  int n;
+  int kernel;  // HBX_FILL_KERNEL_*
 };
 
 __device__ __forceinline__ void cross3(const double u[3], const double v[3], double w[3]) {
@@ -49,27 +53,47 @@ __device__ __forceinline__ void cross3(const double u[3], const double v[3], dou
   w[2] = u[0] * v[1] - u[1] * v[0];
 }
 
+// What face_integral of m_ppohBEM_user_func.f90:49-99 derives from the face
+// alone -- the normal of its plane, and the centroid that a collocation at the
+// face uses -- formed once per face, in the reference's own operations, instead
+// of once per entry (a square root and three divisions of the 25).
+__global__ void k_fill_geom(const double *xyz, const int *face2node, const int *lod, int n, double *f) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const int *nodes = face2node + 3 * (size_t)(lod[i] - 1);
+    double xs[3], ys[3], zs[3];
+    for (int a = 0; a < 3; ++a) {
+      const double *p = xyz + 3 * (size_t)nodes[a];
+      xs[a] = p[0];
+      ys[a] = p[1];
+      zs[a] = p[2];
+    }
+    double u[3], v[3], w[3];
+    u[0] = xs[1] - xs[0];
+    v[0] = xs[2] - xs[1];
+    u[1] = ys[1] - ys[0];
+    v[1] = ys[2] - ys[1];
+    u[2] = zs[1] - zs[0];
+    v[2] = zs[2] - zs[1];
+    cross3(u, v, w);
+    const double wn = sqrt(w[0] * w[0] + w[1] * w[1] + w[2] * w[2]);
+    const double out[kGeom] = {xs[0], xs[1], xs[2], ys[0], ys[1], ys[2], zs[0], zs[1], zs[2],
+                               (xs[0] + xs[1] + xs[2]) / 3.0, (ys[0] + ys[1] + ys[2]) / 3.0,
+                               (zs[0] + zs[1] + zs[2]) / 3.0, w[0] / wn, w[1] / wn, w[2] / wn};
+    for (int k = 0; k < kGeom; ++k) f[(size_t)k * n + i] = out[k];
+  }
+}
+
 // face_integral of m_ppohBEM_user_func.f90:49-99: the analytic integral of
-// 1/r over the flat triangle (xs, ys, zs) seen from (x, y, z); |sum|.
-__device__ double face_integral_raw(const double *xs, const double *ys, const double *zs, double x, double y,
-                                    double z) {
+// 1/r over the flat triangle (xs, ys, zs) with unit normal w seen from
+// (x, y, z); |sum|.
+__device__ double face_integral_raw(const double *xs, const double *ys, const double *zs, const double *w, double x,
+                                    double y, double z) {
   double r[3];
   for (int a = 0; a < 3; ++a) {
     const double dx = xs[a] - x, dy = ys[a] - y, dz = zs[a] - z;
     r[a] = sqrt(dx * dx + dy * dy + dz * dz);
   }
-  double u[3], v[3], w[3];
-  u[0] = xs[1] - xs[0];
-  v[0] = xs[2] - xs[1];
-  u[1] = ys[1] - ys[0];
-  v[1] = ys[2] - ys[1];
-  u[2] = zs[1] - zs[0];
-  v[2] = zs[2] - zs[1];
-  cross3(u, v, w);
-  const double wn = sqrt(w[0] * w[0] + w[1] * w[1] + w[2] * w[2]);
-  w[0] = w[0] / wn;
-  w[1] = w[1] / wn;
-  w[2] = w[2] / wn;
+  double u[3], v[3];
   u[0] = x - xs[0];
   u[1] = y - ys[0];
   u[2] = z - zs[0];
@@ -103,14 +127,17 @@ __device__ double face_integral_raw(const double *xs, const double *ys, const do
   return fabs(sum);
 }
 
-// HACApK_entry_ij for 1-based face ids: collocation at the centroid of face
-// i, integration over face j (m_ppohBEM_matrix_element_ij.f90:60-74).  The
-// ppohBEM scale keeps the reference's single-precision literals PI and
-// EPSILON_0 (m_ppohBEM_user_func.f90:42-43).
-__device__ double entry(const FillGeom &g, int i, int j) {
-  const double x = g.zg[i - 1], y = g.zg[(size_t)g.nofc + (i - 1)], z = g.zg[2 * (size_t)g.nofc + (i - 1)];
-  const double *f = g.fv + 9 * (size_t)(j - 1);
-  const double s = face_integral_raw(f, f + 3, f + 6, x, y, z);
+// HACApK_entry_ij for 0-based positions in cluster order: collocation at the
+// centroid of face i, integration over face j
+// (m_ppohBEM_matrix_element_ij.f90:60-74).  The ppohBEM scale keeps the
+// reference's single-precision literals PI and EPSILON_0
+// (m_ppohBEM_user_func.f90:42-43).
+__device__ __noinline__ double entry(const FillGeom &g, int i, int j) {
+  const size_t n = (size_t)g.n;
+  const double *c = g.f + 9 * n + i, *f = g.f + j;
+  const double xs[3] = {f[0], f[n], f[2 * n]}, ys[3] = {f[3 * n], f[4 * n], f[5 * n]},
+               zs[3] = {f[6 * n], f[7 * n], f[8 * n]}, w[3] = {f[12 * n], f[13 * n], f[14 * n]};
+  const double s = face_integral_raw(xs, ys, zs, w, c[0], c[n], c[2 * n]);
   if (g.kernel == HBX_FILL_KERNEL_PPOHBEM) {
     const double pif = (double)3.141592653589793f, eps0 = (double)8.854187818f * 1e-12;
     return s / (4.0 * pif * eps0);
@@ -130,7 +157,7 @@ __global__ void k_fill_dense(FillGeom g, const DenseJob *jobs, int njobs, double
     const long long n = (long long)J.ndl * J.ndt;
     for (long long e = threadIdx.x; e < n; e += blockDim.x) {
       const int il = (int)(e / J.ndt), it = (int)(e % J.ndt);
-      out[J.off + e] = entry(g, g.lod[il + J.nstrtl - 1], g.lod[it + J.nstrtt - 1]);
+      out[J.off + e] = entry(g, il + J.nstrtl - 1, it + J.nstrtt - 1);
     }
   }
 }
@@ -260,10 +287,10 @@ struct LeafAca {
 
   // column jcol of the residual after k terms (calc_vec, m_HACApK_base.f90:677-698)
   __device__ void calc_col(int k, int jcol, double *vec) const {
-    const int fcol = g.lod[jcol + nstrtt - 2];
+    const int fcol = jcol + nstrtt - 2;
     for (int ii = T.r; ii < ndl; ii += NT) {
       double v = vec[ii];
-      if (rmsk[ii] == 0) v = entry(g, g.lod[ii + nstrtl - 1], fcol);
+      if (rmsk[ii] == 0) v = entry(g, ii + nstrtl - 1, fcol);
       if (k > 0) {
         double tmp = 0.0;
         for (int it = 1; it <= k; ++it) tmp = tmp + U[(size_t)ndl * (it - 1) + ii] * V[(size_t)ndt * (it - 1) + (jcol - 1)];
@@ -276,10 +303,10 @@ struct LeafAca {
   }
   // row irow of the residual after k terms
   __device__ void calc_row(int k, int irow, double *vec) const {
-    const int frow = g.lod[irow + nstrtl - 2];
+    const int frow = irow + nstrtl - 2;
     for (int ii = T.r; ii < ndt; ii += NT) {
       double v = vec[ii];
-      if (cmsk[ii] == 0) v = entry(g, frow, g.lod[ii + nstrtt - 1]);
+      if (cmsk[ii] == 0) v = entry(g, frow, ii + nstrtt - 1);
       if (k > 0) {
         double tmp = 0.0;
         for (int it = 1; it <= k; ++it) tmp = tmp + V[(size_t)ndt * (it - 1) + ii] * U[(size_t)ndl * (it - 1) + (irow - 1)];
@@ -465,6 +492,17 @@ __device__ int aca_plus(const LeafAca<NT> &C, const AcaParams &P, double *pa_ref
   return k;
 }
 
+// Threads of the team of a leaf whose longer side has m entries: about one
+// entry of a row or a column step a thread.  A step is a chain of latencies
+// (an entry's square roots, divisions and arctangents, a pass over the factors
+// so far, the reductions), and the leaves are many enough to fill the SMs with
+// any team size, so a short chain beats a small team: one warp for every leaf
+// below 4,096 rows and columns and 512 threads above took 126 ms for the 32,288
+// leaves of an 81,920-triangle sphere, most of it the tail of warps that had a
+// long leaf to themselves.
+constexpr int kTeams = 5;
+int team_class(int m) { return m <= 48 ? 0 : m <= 96 ? 1 : m <= 192 ? 2 : m <= 768 ? 3 : 4; }
+
 // One team per leaf: NT = 32 runs eight warps per CTA, each its own leaf;
 // NT > 32 one CTA per leaf.
 template <int NT>
@@ -472,20 +510,24 @@ __global__ void __launch_bounds__(NT == 32 ? 256 : NT) k_fill_aca(FillGeom g, Ac
                                                                  double *work, int *masks) {
   __shared__ double sd[NT == 32 ? 1 : NT / 32];
   __shared__ int si[NT == 32 ? 1 : NT / 32];
-  const int teams_per_cta = NT == 32 ? (int)(blockDim.x >> 5) : 1;
-  const int team = NT == 32 ? (int)(threadIdx.x >> 5) : 0;
+  const int q = NT == 32 ? (int)(blockIdx.x * 8 + (threadIdx.x >> 5)) : (int)blockIdx.x;
   const Team<NT> T{(int)(NT == 32 ? (threadIdx.x & 31) : threadIdx.x), sd, si};
-  for (int q = blockIdx.x * teams_per_cta + team; q < njobs; q += gridDim.x * teams_per_cta) {
-    AcaJob &J = jobs[q];
-    double *w = work + J.woff;
-    const LeafAca<NT> C{g, T, J.ndl, J.ndt, J.nstrtl, J.nstrtt, J.cap, w, w + (size_t)J.ndl * J.cap,
-                        masks + J.moff, masks + J.moff + J.ndl};
-    double *pa_ref = w + (size_t)(J.ndl + J.ndt) * J.cap;
-    double *pb_ref = pa_ref + J.ndl;
-    const int kt = aca_plus<NT>(C, P, pa_ref, pb_ref);
-    if (T.r == 0) J.kt = kt;
-    T.sync();
-  }
+  if (q >= njobs) return;
+  AcaJob &J = jobs[q];
+  double *w = work + J.woff;
+  const LeafAca<NT> C{g, T, J.ndl, J.ndt, J.nstrtl, J.nstrtt, J.cap, w, w + (size_t)J.ndl * J.cap,
+                      masks + J.moff, masks + J.moff + J.ndl};
+  double *pa_ref = w + (size_t)(J.ndl + J.ndt) * J.cap;
+  double *pb_ref = pa_ref + J.ndl;
+  const int kt = aca_plus<NT>(C, P, pa_ref, pb_ref);
+  if (T.r == 0) J.kt = kt;
+}
+
+template <int NT>
+void launch_aca(const FillGeom &g, AcaJob *jobs, int njobs, const AcaParams &P, double *work, int *masks,
+                cudaStream_t s) {
+  const int per = NT == 32 ? 8 : 1;
+  k_fill_aca<NT><<<(njobs + per - 1) / per, NT * per, 0, s>>>(g, jobs, njobs, P, work, masks);
 }
 
 // The factors of job q, columns 1..kt, from its workspace into the packed
@@ -521,10 +563,42 @@ namespace {
 
 thread_local std::string g_fill_error;
 
+// Host memory of the leaves: on 2 MB boundaries and, where the system gives
+// them, 2 MB pages (the first touch of 4 KB pages took as long as the copy).
+double *leaf_storage(size_t bytes) {
+  constexpr size_t kHuge = (size_t)2 << 20;
+  if (bytes < 4 * kHuge) return static_cast<double *>(std::malloc(bytes));
+  void *p = std::aligned_alloc(kHuge, (bytes + kHuge - 1) / kHuge * kHuge);
+#ifdef MADV_HUGEPAGE
+  if (p) madvise(p, bytes, MADV_HUGEPAGE);
+#endif
+  return static_cast<double *>(p);
+}
+
 struct DevBuf {
   void *p = nullptr;
   ~DevBuf() {
     if (p) cudaFree(p);
+  }
+};
+
+// One stream per team size, so that the sizes' kernels fill each other's gaps.
+// Blocking streams: their kernels follow the uploads on the default stream.
+struct Streams {
+  cudaStream_t s[hbx::kTeams + 1] = {};
+  cudaError_t open() {
+    for (cudaStream_t &x : s) {
+      cudaError_t e = cudaStreamCreate(&x);
+      if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+  }
+  ~Streams() {
+    for (cudaStream_t x : s)
+      if (x) {
+        cudaStreamSynchronize(x);
+        cudaStreamDestroy(x);
+      }
   }
 };
 
@@ -548,23 +622,10 @@ int hbx_fill_leaves(const double *xyz, int nond, const int *face2node, int nofc,
   auto leaf = [&](int ip) -> stc_HACApK_leafmtx & {
     return *reinterpret_cast<stc_HACApK_leafmtx *>(reinterpret_cast<char *>(st->st_lf) + (size_t)ip * st->st_lf_stride);
   };
-  // geometry: face vertices and centroids as hbx_build forms them
-  std::vector<double> fv(9 * (size_t)nofc), zg(3 * (size_t)nofc);
-  for (int f = 0; f < nofc; ++f) {
-    double *o = &fv[9 * (size_t)f];
-    for (int a = 0; a < 3; ++a) {
-      const int n = face2node[3 * (size_t)f + a];
-      if (n < 0 || n >= nond) return HBX_ERR_INVALID;
-      o[a] = xyz[3 * (size_t)n];
-      o[3 + a] = xyz[3 * (size_t)n + 1];
-      o[6 + a] = xyz[3 * (size_t)n + 2];
-    }
-    zg[f] = (o[0] + o[1] + o[2]) / 3.0;
-    zg[(size_t)nofc + f] = (o[3] + o[4] + o[5]) / 3.0;
-    zg[2 * (size_t)nofc + f] = (o[6] + o[7] + o[8]) / 3.0;
-  }
   for (int i = 0; i < nofc; ++i)
     if (lod[i] < 1 || lod[i] > nofc) return HBX_ERR_INVALID;
+  for (size_t k = 0; k < 3 * (size_t)nofc; ++k)
+    if (face2node[k] < 0 || face2node[k] >= nond) return HBX_ERR_INVALID;
   std::vector<DenseJob> dense;
   std::vector<int> dense_ip, aca_ip;
   long long dense_words = 0;
@@ -582,24 +643,48 @@ int hbx_fill_leaves(const double *xyz, int nond, const int *face2node, int nofc,
     }
   }
   cudaError_t e;
-  DevBuf d_fv, d_zg, d_lod;
-  if ((e = cudaMalloc(&d_fv.p, fv.size() * 8)) != cudaSuccess || (e = cudaMalloc(&d_zg.p, zg.size() * 8)) != cudaSuccess ||
-      (e = cudaMalloc(&d_lod.p, (size_t)nofc * 4)) != cudaSuccess)
-    return e == cudaErrorMemoryAllocation ? HBX_ERR_NOMEM : HBX_ERR_CUDA;
-  cudaMemcpy(d_fv.p, fv.data(), fv.size() * 8, cudaMemcpyHostToDevice);
-  cudaMemcpy(d_zg.p, zg.data(), zg.size() * 8, cudaMemcpyHostToDevice);
-  cudaMemcpy(d_lod.p, lod, (size_t)nofc * 4, cudaMemcpyHostToDevice);
-  const FillGeom g{static_cast<const double *>(d_fv.p), static_cast<const double *>(d_zg.p),
-                   static_cast<const int *>(d_lod.p), nofc, params->kernel};
   int dev = 0, nsm = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  // geometry: the faces in cluster order (xyz, the node ids and lod are only needed to form it)
+  DevBuf d_geom;
+  {
+    DevBuf d_xyz, d_f2n, d_lod;
+    const size_t bx = 3 * (size_t)nond * 8, bf = 3 * (size_t)nofc * 4, bl = (size_t)nofc * 4;
+    if ((e = cudaMalloc(&d_geom.p, (size_t)kGeom * nofc * 8)) != cudaSuccess || (e = cudaMalloc(&d_xyz.p, bx)) != cudaSuccess ||
+        (e = cudaMalloc(&d_f2n.p, bf)) != cudaSuccess || (e = cudaMalloc(&d_lod.p, bl)) != cudaSuccess)
+      return e == cudaErrorMemoryAllocation ? HBX_ERR_NOMEM : HBX_ERR_CUDA;
+    cudaMemcpy(d_xyz.p, xyz, bx, cudaMemcpyHostToDevice);
+    cudaMemcpy(d_f2n.p, face2node, bf, cudaMemcpyHostToDevice);
+    cudaMemcpy(d_lod.p, lod, bl, cudaMemcpyHostToDevice);
+    k_fill_geom<<<std::min((nofc + 127) / 128, nsm * 16), 128>>>(
+        static_cast<const double *>(d_xyz.p), static_cast<const int *>(d_f2n.p), static_cast<const int *>(d_lod.p), nofc,
+        static_cast<double *>(d_geom.p));
+    if ((e = cudaGetLastError()) != cudaSuccess || (e = cudaDeviceSynchronize()) != cudaSuccess) return HBX_ERR_CUDA;
+  }
+  const FillGeom g{static_cast<const double *>(d_geom.p), nofc, params->kernel};
 
   // largest leaves first, so that the warps that take them start at once
   std::stable_sort(aca_ip.begin(), aca_ip.end(), [&](int a, int b) {
     const stc_HACApK_leafmtx &x = leaf(a), &y = leaf(b);
     return (long long)x.ndl * x.ndt > (long long)y.ndl * y.ndt;
   });
+  Streams streams;
+  if (streams.open() != cudaSuccess) return HBX_ERR_CUDA;
+  // ---- dense leaves: their kernel runs beside the ACA+ kernels
+  DevBuf d_dense, d_djobs;
+  if (!dense.empty()) {
+    if ((e = cudaMalloc(&d_djobs.p, dense.size() * sizeof(DenseJob))) != cudaSuccess ||
+        (e = cudaMalloc(&d_dense.p, std::max<long long>(1, dense_words) * 8)) != cudaSuccess)
+      return e == cudaErrorMemoryAllocation ? HBX_ERR_NOMEM : HBX_ERR_CUDA;
+    cudaMemcpy(d_djobs.p, dense.data(), dense.size() * sizeof(DenseJob), cudaMemcpyHostToDevice);
+  }
+  auto launch_dense = [&]() -> cudaError_t {
+    if (dense.empty()) return cudaSuccess;
+    k_fill_dense<<<(int)std::min<size_t>(dense.size(), (size_t)nsm * 16), 256, 0, streams.s[kTeams]>>>(
+        g, static_cast<DenseJob *>(d_djobs.p), (int)dense.size(), static_cast<double *>(d_dense.p));
+    return cudaGetLastError();
+  };
   // ---- ACA+ in batches of leaves whose workspaces fit the budget; a leaf
   // whose rank outgrows its columns is run again with twice as many.  The
   // packed factors of every batch stay on the device until the end.
@@ -617,8 +702,8 @@ int hbx_fill_leaves(const double *xyz, int nond, const int *face2node, int nofc,
   const int first_cap = params->first_cap > 0 ? params->first_cap : 64;
   long long retried = 0;
   double t_aca = 0.0;
-  // leaves with more rows plus columns than this get a CTA, the rest a warp
-  constexpr int kBigLeaf = 4096, kBigTeam = 512;
+  bool dense_launched = false;
+  constexpr int kBigLeaf = 4096;  // leaves of this many rows and columns make batches of their own
   DevBuf d_work, d_mask, d_jobs;
   size_t work_cap = 0, mask_cap = 0, jobs_cap = 0;
   auto ensure = [&](DevBuf &b, size_t &cap, size_t bytes) -> cudaError_t {
@@ -635,8 +720,10 @@ int hbx_fill_leaves(const double *xyz, int nond, const int *face2node, int nofc,
     std::vector<size_t> again;
     size_t pos = 0;
     while (pos < todo.size()) {
+      // the batch: leaves [pos, ...) in size order, its jobs grouped by team size
       std::vector<AcaJob> jobs;
       std::vector<size_t> which;
+      std::vector<int> cls;
       long long wd = 0, wm = 0;
       bool big = false;
       while (pos < todo.size()) {
@@ -653,46 +740,65 @@ int hbx_fill_leaves(const double *xyz, int nond, const int *face2node, int nofc,
         big = b;
         jobs.push_back(AcaJob{L.nstrtl, L.ndl, L.nstrtt, L.ndt, cap, 0, wd, wm});
         which.push_back(todo[pos]);
+        cls.push_back(team_class(std::max(L.ndl, L.ndt)));
         wd += need;
         wm += L.ndl + L.ndt;
         ++pos;
       }
+      std::vector<int> at(jobs.size());  // place of each job in the grouped list
+      int first[kTeams + 1] = {0};
+      for (int c : cls) ++first[c + 1];
+      for (int c = 0; c < kTeams; ++c) first[c + 1] += first[c];
+      {
+        int next[kTeams];
+        std::copy(first, first + kTeams, next);
+        for (size_t q = 0; q < jobs.size(); ++q) at[q] = next[cls[q]]++;
+      }
+      std::vector<AcaJob> grouped(jobs.size());
+      for (size_t q = 0; q < jobs.size(); ++q) grouped[at[q]] = jobs[q];
       const double tb = now_s();
       if ((e = ensure(d_jobs, jobs_cap, jobs.size() * sizeof(AcaJob))) != cudaSuccess ||
           (e = ensure(d_work, work_cap, (size_t)wd * 8)) != cudaSuccess ||
           (e = ensure(d_mask, mask_cap, (size_t)wm * 4)) != cudaSuccess)
         return e == cudaErrorMemoryAllocation ? HBX_ERR_NOMEM : HBX_ERR_CUDA;
-      cudaMemcpy(d_jobs.p, jobs.data(), jobs.size() * sizeof(AcaJob), cudaMemcpyHostToDevice);
-      if (big) {
-        const int nblk = (int)std::min<size_t>(jobs.size(), (size_t)nsm * 4);
-        k_fill_aca<kBigTeam><<<nblk, kBigTeam>>>(g, static_cast<AcaJob *>(d_jobs.p), (int)jobs.size(), P,
-                                                 static_cast<double *>(d_work.p), static_cast<int *>(d_mask.p));
-      } else {
-        const int wpb = 8;
-        const int nblk = (int)std::min<size_t>((jobs.size() + wpb - 1) / wpb, (size_t)nsm * 16);
-        k_fill_aca<32><<<nblk, 32 * wpb>>>(g, static_cast<AcaJob *>(d_jobs.p), (int)jobs.size(), P,
-                                           static_cast<double *>(d_work.p), static_cast<int *>(d_mask.p));
+      cudaMemcpy(d_jobs.p, grouped.data(), grouped.size() * sizeof(AcaJob), cudaMemcpyHostToDevice);
+      for (int c = kTeams - 1; c >= 0; --c) {  // the longest leaves start first
+        const int n = first[c + 1] - first[c];
+        if (n == 0) continue;
+        AcaJob *dj = static_cast<AcaJob *>(d_jobs.p) + first[c];
+        double *wk = static_cast<double *>(d_work.p);
+        int *mk = static_cast<int *>(d_mask.p);
+        if (c == 0) launch_aca<32>(g, dj, n, P, wk, mk, streams.s[c]);
+        else if (c == 1) launch_aca<64>(g, dj, n, P, wk, mk, streams.s[c]);
+        else if (c == 2) launch_aca<128>(g, dj, n, P, wk, mk, streams.s[c]);
+        else if (c == 3) launch_aca<256>(g, dj, n, P, wk, mk, streams.s[c]);
+        else launch_aca<512>(g, dj, n, P, wk, mk, streams.s[c]);
       }
-      if ((e = cudaGetLastError()) != cudaSuccess || (e = cudaDeviceSynchronize()) != cudaSuccess) {
+      if ((e = cudaGetLastError()) == cudaSuccess && !dense_launched) {
+        e = launch_dense();
+        dense_launched = true;
+      }
+      if (e != cudaSuccess || (e = cudaDeviceSynchronize()) != cudaSuccess) {
         g_fill_error = cudaGetErrorString(e);
         return HBX_ERR_CUDA;
       }
-      cudaMemcpy(jobs.data(), d_jobs.p, jobs.size() * sizeof(AcaJob), cudaMemcpyDeviceToHost);
+      cudaMemcpy(grouped.data(), d_jobs.p, grouped.size() * sizeof(AcaJob), cudaMemcpyDeviceToHost);
       const double tk = now_s();
       // pack the finished leaves' factors into this batch's output buffer
       std::vector<PackJob> pk;
       long long ow = 0;
       const int ob = (int)outs.size();
       for (size_t q = 0; q < jobs.size(); ++q) {
-        if (jobs[q].kt < 0) {
+        const int kt = grouped[at[q]].kt;
+        if (kt < 0) {
           again.push_back(which[q]);
           continue;
         }
-        pk.push_back(PackJob{jobs[q].woff, ow, jobs[q].ndl, jobs[q].ndt, jobs[q].cap, jobs[q].kt});
-        kt_of[which[q]] = jobs[q].kt;
+        pk.push_back(PackJob{jobs[q].woff, ow, jobs[q].ndl, jobs[q].ndt, jobs[q].cap, kt});
+        kt_of[which[q]] = kt;
         out_buf[which[q]] = ob;
         out_off[which[q]] = ow;
-        ow += (long long)(jobs[q].ndl + jobs[q].ndt) * jobs[q].kt;
+        ow += (long long)(jobs[q].ndl + jobs[q].ndt) * kt;
       }
       if (!pk.empty()) {
         outs.emplace_back();
@@ -709,26 +815,14 @@ int hbx_fill_leaves(const double *xyz, int nond, const int *face2node, int nofc,
       }
       t_aca += tk - tb;
       if (verbose)
-        std::fprintf(stderr, "hbx_fill: round %d batch of %zu %s leaves, workspace %.2f GB, ACA+ %.3f s, pack %.3f s\n",
-                     round, jobs.size(), big ? "large" : "small", wd * 8e-9, tk - tb, now_s() - tk);
+        std::fprintf(stderr, "hbx_fill: round %d batch of %zu leaves, workspace %.2f GB, ACA+ %.3f s, pack %.3f s\n",
+                     round, jobs.size(), wd * 8e-9, tk - tb, now_s() - tk);
     }
     retried += round == 0 ? (long long)again.size() : 0;
     todo.swap(again);
   }
-  const double t1 = now_s();
-
-  // ---- dense leaves, on the device
-  DevBuf d_dense;
-  if (!dense.empty()) {
-    DevBuf d_jobs;
-    if ((e = cudaMalloc(&d_jobs.p, dense.size() * sizeof(DenseJob))) != cudaSuccess ||
-        (e = cudaMalloc(&d_dense.p, std::max<long long>(1, dense_words) * 8)) != cudaSuccess)
-      return e == cudaErrorMemoryAllocation ? HBX_ERR_NOMEM : HBX_ERR_CUDA;
-    cudaMemcpy(d_jobs.p, dense.data(), dense.size() * sizeof(DenseJob), cudaMemcpyHostToDevice);
-    k_fill_dense<<<(int)std::min<size_t>(dense.size(), (size_t)nsm * 16), 256>>>(
-        g, static_cast<DenseJob *>(d_jobs.p), (int)dense.size(), static_cast<double *>(d_dense.p));
-    if ((e = cudaGetLastError()) != cudaSuccess || (e = cudaDeviceSynchronize()) != cudaSuccess) return HBX_ERR_CUDA;
-  }
+  if (!dense_launched && ((e = launch_dense()) != cudaSuccess || (e = cudaDeviceSynchronize()) != cudaSuccess))
+    return HBX_ERR_CUDA;
   const double t2 = now_s();
 
   // ---- leaf storage in the reference layout: the dense entries, then every
@@ -738,7 +832,7 @@ int hbx_fill_leaves(const double *xyz, int nond, const int *face2node, int nofc,
   hbx_fill *F = new (std::nothrow) hbx_fill();
   if (!F) return HBX_ERR_NOMEM;
   F->words = words;
-  F->storage = static_cast<double *>(std::malloc(std::max<size_t>(1, words) * 8));
+  F->storage = leaf_storage(std::max<size_t>(1, words) * 8);
   if (!F->storage) {
     delete F;
     return HBX_ERR_NOMEM;
@@ -751,16 +845,17 @@ int hbx_fill_leaves(const double *xyz, int nond, const int *face2node, int nofc,
       o += (size_t)out_words[k];
     }
   }
-  // first touch of the destination pages by every host core (a pageable
-  // copy into untouched memory runs at a tenth of the speed)
   const double t3 = now_s();
-#pragma omp parallel for schedule(static)
-  for (long long i = 0; i < (long long)words; i += 512) F->storage[i] = 0.0;
-  const double t4 = now_s();
-  if (dense_words > 0) e = cudaMemcpy(F->storage, d_dense.p, (size_t)dense_words * 8, cudaMemcpyDeviceToHost);
-  for (size_t k = 0; k < outs.size() && e == cudaSuccess; ++k)
-    if (out_words[k] > 0) e = cudaMemcpy(F->storage + base[k], outs[k].p, (size_t)out_words[k] * 8, cudaMemcpyDeviceToHost);
-  if (verbose) std::fprintf(stderr, "hbx_fill: first touch %.3f s, copies %.3f s\n", t4 - t3, now_s() - t4);
+  {
+    Stager stager;
+    if (dense_words > 0)
+      e = stager.to_host({HostPiece{F->storage, 0, (uint64_t)dense_words}}, (uint64_t)dense_words,
+                         static_cast<const double *>(d_dense.p));
+    for (size_t k = 0; k < outs.size() && e == cudaSuccess; ++k)
+      e = stager.to_host({HostPiece{F->storage + base[k], 0, (uint64_t)out_words[k]}}, (uint64_t)out_words[k],
+                         static_cast<const double *>(outs[k].p));
+  }
+  if (verbose) std::fprintf(stderr, "hbx_fill: copies %.3f s\n", now_s() - t3);
   if (e != cudaSuccess) {
     hbx_fill_free(F);
     return HBX_ERR_CUDA;
@@ -787,8 +882,8 @@ int hbx_fill_leaves(const double *xyz, int nond, const int *face2node, int nofc,
   st->ktmax = ktmax;
   st->nlfkt = nlfkt;
   if (verbose)
-    std::fprintf(stderr, "hbx_fill: ACA+ %.3f s (kernels), all batches %.3f s, dense %.3f s, to the host %.3f s\n",
-                 t_aca, t1 - t0, t2 - t1, now_s() - t2);
+    std::fprintf(stderr, "hbx_fill: ACA+ %.3f s (kernels), all on the device %.3f s, to the host %.3f s\n", t_aca, t2 - t0,
+                 now_s() - t2);
   if (stats) {
     std::memset(stats, 0, sizeof(*stats));
     stats->n_lowrank = nlfkt;

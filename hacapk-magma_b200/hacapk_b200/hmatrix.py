@@ -187,10 +187,9 @@ class HostHMatrix:
         if st != 0:
             raise RuntimeError(f"hbx_fill_leaves failed: {abi.STATUS.get(st, st)}")
         self._fill = f
-        d, lr = self.storage_words()
         self.stats["ktmax"] = fs.ktmax
-        self.stats["mem_words"] = d + lr
-        self.stats["memh_words"] = d + lr + self.nlf
+        self.stats["mem_words"] = fs.words
+        self.stats["memh_words"] = fs.words + self.nlf
         return {k: getattr(fs, k) for k, _ in abi.FillStats._fields_ if k != "reserved"}
 
     def close(self):
