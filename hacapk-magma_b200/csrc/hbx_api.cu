@@ -97,6 +97,7 @@ void free_engine(hbx_hmat *h) {
   if (h->ggraph) cudaGraphExecDestroy(h->ggraph);
   cudaFree(h->d_f32);
   cudaFree(h->d_zbum);
+  cudaFree(h->d_mcols);
   cudaFree(h->d_mrv);
   cudaFree(h->d_mr32);
   cudaFree(h->d_mrpart);
@@ -397,6 +398,8 @@ static int create_engine(const stc_HACApK_leafmtxp *st, int nd, const hbx_option
   if (nrhs > 1 &&
       (e = dev_malloc(&h->d_zbum, std::max<uint64_t>(1, P.zbu_len) * hbx::kNrhs * sizeof(float))) != cudaSuccess)
     return bail(cuda_fail(e, "cudaMalloc(multi-RHS zbu)"));
+  if (nrhs > 1 && (e = dev_malloc(&h->d_mcols, std::max<uint64_t>(1, P.panel_cols) * sizeof(uint32_t))) != cudaSuccess)
+    return bail(cuda_fail(e, "cudaMalloc(multi-RHS columns)"));
   if ((e = dev_malloc(&h->d_gbar, 4 * sizeof(unsigned))) != cudaSuccess) return bail(cuda_fail(e, "cudaMalloc(gbar)"));
   if ((e = dev_malloc(&h->d_err, sizeof(int))) != cudaSuccess) return bail(cuda_fail(e, "cudaMalloc(err)"));
   if (!P.recs.empty() &&
@@ -429,6 +432,8 @@ static int create_engine(const stc_HACApK_leafmtxp *st, int nd, const hbx_option
     return bail(fail(HBX_ERR_NOMEM, "hbx_create: host staging buffer"));
   }
   if (e != cudaSuccess) return bail(cuda_fail(e, "pack stream"));
+  if (nrhs > 1 && (e = hbx::launch_matmat_cols(h->d_recs, h->d_ctas, nc, h->d_mcols, nullptr)) != cudaSuccess)
+    return bail(cuda_fail(e, "multi-RHS columns"));
   cudaMemset(h->d_gbar, 0, 4 * sizeof(unsigned));
   cudaMemset(h->d_err, 0, sizeof(int));
   cudaMemset(h->d_zbu, 0, 2 * std::max<uint64_t>(1, P.zbu_len) * sizeof(double));
@@ -600,9 +605,9 @@ int hbx_matmat(hbx_hmat *h, double alpha, const float *X, double beta, const dou
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   hbx::MatmatArgs a{};
   a.stream = h->d_stream;
-  a.recs = h->d_recs;
   a.ctas = h->d_ctas;
   a.lite = h->d_lite;
+  a.cols = h->d_mcols;
   a.x = X;
   a.yin = Yin;
   a.y = Y;
@@ -1427,9 +1432,9 @@ cudaError_t mr_matmat(void *ctx, const float *x, double *y, cudaStream_t s) {
   hbx_hmat *hm = static_cast<hbx_hmat *>(ctx);
   hbx::MatmatArgs a{};
   a.stream = hm->d_stream;
-  a.recs = hm->d_recs;
   a.ctas = hm->d_ctas;
   a.lite = hm->d_lite;
+  a.cols = hm->d_mcols;
   a.x = x;
   a.y = y;
   a.zbu = hm->d_zbum;

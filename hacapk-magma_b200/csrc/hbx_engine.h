@@ -89,9 +89,9 @@ struct BicgArgs {
 constexpr int kNrhs = 64;
 struct MatmatArgs {
   const uint8_t *stream;  // packed with pair_panels (FP32)
-  const RunRec *recs;
   const CtaInfo *ctas;
   const RunLite *lite;
+  const uint32_t *cols;  // vector row of every panel column (x, or zbu for U runs), kNoCol: a zero column
   const float *x;     // [nd][kNrhs]
   const double *yin;  // [nd][kNrhs], read when beta != 0
   double *y;          // [nd][kNrhs]
@@ -104,6 +104,9 @@ struct MatmatArgs {
 size_t matmat_smem_bytes();
 cudaError_t configure_matmat();
 cudaError_t launch_matmat(const MatmatArgs &a, int num_ctas, cudaStream_t s);
+constexpr uint32_t kNoCol = 0xffffffffu;
+// Forms MatmatArgs::cols from the run records (once per engine).
+cudaError_t launch_matmat_cols(const RunRec *recs, const CtaInfo *ctas, int num_ctas, uint32_t *cols, cudaStream_t s);
 
 // Multi-RHS BiCGSTAB (hbx_mrhs_solve.cu): scalars of one right-hand side.
 struct MrScal {
@@ -237,6 +240,7 @@ struct hbx_hmat {
   int num_ctas = 0;
   int transposed = 0;  // the packed stream holds H^T
   int nrhs = 1;        // right-hand sides per product (kNrhs: multi-RHS engine, hbx_matmat only)
+  uint32_t *d_mcols = nullptr;  // multi-RHS engine: MatmatArgs::cols
   float *d_zbum = nullptr;  // multi-RHS engine: zbu for all right-hand sides [zbu_len][kNrhs]
   // multi-RHS solver workspace (hbx_bicgstab_multi)
   double *d_mrv = nullptr;      // r, rh, p, ap, t, at, x, R, and two kNrhs x nd scratch arrays

@@ -3,31 +3,31 @@
 //
 // The packed stream is the FP32 engine's (panels of 4 columns x h rows, 16
 // bytes a row) with every run an even number of panels, so two panels make
-// the K = 8 of one TF32 step.  Per CTA (one per SM), 16 warps:
+// the K = 8 of one TF32 step.  Per CTA (one per SM), 23 warps:
 //
 //   warps 0-3   epilogue: TMEM accumulator -> zbu (P blocks) or Y (D, U)
-//   warp 4      tcgen05: allocates TMEM; one thread issues the MMAs of the
-//               even blocks
+//   warp 4      tcgen05: allocates TMEM; one thread issues the MMAs
 //   warp 5      bulk-copy producer of the stream ring (16 KB chunks)
-//   warps 6-13  gather: X (or zbu) columns of a run, 64 at a time, into a
-//               K-major operand stage [4-column chunk][rhs][4] (16 KB), one
-//               stage per warp
-//   warp 14     grid barrier between the P blocks and the U runs
-//   warp 15     one thread issues the MMAs of the odd blocks
+//   warps 6-21  gather: X (or zbu) columns of a run, 128 at a time, into a
+//               K-major operand stage [4-column chunk][rhs][4] (32 KB), four
+//               warps per stage
+//   warp 22     grid barrier between the P blocks and the U runs
 //
-// Two issuers because one thread's issue loop (descriptors, ring and stage
-// waits, commits: ~170 cycles an MMA of M = 64, N <= 64, K = 8) paced the
-// whole CTA; each has its own two accumulators, waits for its own slices'
-// stages, and hands every ring chunk back (the empty barriers count both).
+// The MMA thread is the one that elect.sync names: the compiler then knows that
+// one thread is active.  Under threadIdx.x % 32 == 0 it does not, and guards
+// every MMA with a loop over the active lanes: 107 cycles an MMA of M = 64,
+// N = 24, K = 8 with this kernel's descriptors, against 35 here, four at a time
+// (the tensor core takes 23).  Two threads of the first kind on alternate
+// blocks, which this replaces, kept the product on 81,920 unknowns at 513 us.
 //
 // One MMA: D[rhs][row] += Xs[rhs][k..k+8] * Panel[row][k..k+8]^T with
 // M = 64 right-hand sides, N = the block's rows rounded up to 8, A (the
 // staged X) and B (two panels straight from the ring) both K-major in the
 // canonical no-swizzle layout: 8-row core matrices of 16-byte rows, the next
 // 8 rows 128 bytes on (SBO), the next 4 columns LBO on (1 KB for A, 16h for
-// B).  D lives in TMEM (M = 64: rhs m in lane (m mod 16) + 32 (m / 16)); two
-// 64-column accumulators let the epilogue of one block overlap the MMAs of
-// the next.  The ring is smaller than k_matvec's (the product is bound by
+// B).  D lives in TMEM (M = 64: rhs m in lane (m mod 16) + 32 (m / 16)); four
+// 64-column accumulators let the epilogue of a block overlap the MMAs of
+// the next ones.  The ring is smaller than k_matvec's (the product is bound by
 // the X stages, not by the stream) and MMAs read it in place: a panel pair
 // that runs past the
 // ring's end reads a mirror of the first bytes of slot 0 that the producer
@@ -41,45 +41,45 @@
 namespace hbx {
 namespace {
 
-constexpr int kSliceCols = 64;                         // stage columns per slice
+constexpr int kSliceCols = 128;                        // stage columns per slice
 constexpr int kSliceChunks = kSliceCols / 4;           // 4-column K chunks per slice
 constexpr int kChunkXBytes = kNrhs * 16;               // one chunk, all right-hand sides: 1 KB
-constexpr int kSliceBytes = kSliceChunks * kChunkXBytes;  // 16 KB
+constexpr int kSliceBytes = kSliceChunks * kChunkXBytes;  // 32 KB
 constexpr int kMChunkLog = 14;  // ring chunk: 16 KB
 constexpr int kMChunkBytes = 1 << kMChunkLog;
-constexpr int kMRingChunks = 4;
+constexpr int kMRingChunks = 5;
 constexpr uint32_t kMRingBytes = (uint32_t)kMRingChunks * kMChunkBytes;
-constexpr int kXStages = 8;
+constexpr int kXStages = 4;
 constexpr int kMirrorBytes = 2304;  // >= 2 panels of 64 rows + 7 rows past them
 constexpr int kAccCols = 64;        // TMEM columns per accumulator (rows of a block <= 64)
-constexpr int kIssuers = 2;  // MMA-issuing threads (warps kMmaWarp and kMmaWarp2), alternate blocks
-constexpr int kTmemCols = 2 * kIssuers * kAccCols;  // two accumulators per issuer
-constexpr int kEpiWarps = 4, kMmaWarp = 4, kProdWarpM = 5, kGathWarp0 = 6, kGathWarps = 8, kSyncWarpM = 14,
-              kMmaWarp2 = 15;
-static_assert(kXStages == kGathWarps, "gather warp gi always fills stage gi");
-constexpr int kThreadsM = (kMmaWarp2 + 1) * 32;
+constexpr int kAccs = 4;            // accumulators: blocks in flight between the MMAs and the epilogue
+constexpr int kTmemCols = kAccs * kAccCols;
+constexpr int kEpiWarps = 4, kMmaWarp = 4, kProdWarpM = 5, kGathWarp0 = 6, kGathWarps = 16,
+              kSyncWarpM = kGathWarp0 + kGathWarps;
+constexpr int kSliceWarps = kGathWarps / kXStages;      // gather warps per stage, side by side
+constexpr int kWarpCols = kSliceCols / kSliceWarps;     // stage columns of one gather warp
+static_assert(kWarpCols == 32, "one column source a lane");
+constexpr int kThreadsM = (kSyncWarpM + 1) * 32;
 
 struct MLayout {
   static constexpr uint32_t ring = 0;
   static constexpr uint32_t xst = (kMRingBytes + kMirrorBytes + 1023) / 1024 * 1024;  // [kXStages] slices
-  static constexpr uint32_t rec = xst + kXStages * kSliceBytes;                       // [kGathWarps][2] records
-  static constexpr uint32_t lite = rec + 2 * kGathWarps * kRecBytes;                  // [kMaxPairRuns] summaries
+  static constexpr uint32_t lite = xst + kXStages * kSliceBytes;                      // [kMaxPairRuns] summaries
   static constexpr uint32_t full = lite + kMaxPairRuns * 16;
   static constexpr uint32_t empty = full + 8 * kMRingChunks;
   static constexpr uint32_t xfull = empty + 8 * kMRingChunks;
   static constexpr uint32_t xempty = xfull + 8 * kXStages;
   static constexpr uint32_t accfull = xempty + 8 * kXStages;
-  static constexpr uint32_t accempty = accfull + 8 * 2 * kIssuers;
-  static constexpr uint32_t pdone = accempty + 8 * 2 * kIssuers;
+  static constexpr uint32_t accempty = accfull + 8 * kAccs;
+  static constexpr uint32_t pdone = accempty + 8 * kAccs;
   static constexpr uint32_t gdone = pdone + 8;
   static constexpr uint32_t mdone = gdone + 8;
   static constexpr uint32_t tmem = mdone + 8;  // TMEM base address (tcgen05.alloc writes it)
   static constexpr uint32_t gen0 = tmem + 4;   // first grid-barrier generation of the launch
-  static constexpr uint32_t xcnt = (gen0 + 4 + 15) / 16 * 16;  // [kXStages] slices staged per slot
-  static constexpr uint32_t bytes = xcnt + 4 * kXStages;
+  static constexpr uint32_t bytes = gen0 + 4;
 };
 static_assert(MLayout::bytes <= 227 * 1024, "shared memory per CTA");
-static_assert(MLayout::xst % 1024 == 0 && MLayout::rec % 16 == 0 && MLayout::full % 8 == 0, "layout alignment");
+static_assert(MLayout::xst % 1024 == 0 && MLayout::lite % 16 == 0 && MLayout::full % 8 == 0, "layout alignment");
 
 // ---- tcgen05 ----------------------------------------------------------------
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -115,27 +115,31 @@ __device__ __forceinline__ void tc_commit(uint64_t *bar) {
 }
 
 // ---- producer with the ring-end mirror ------------------------------------
+// The factors pass through L2 with evict_first, and Y past it: X and zbu are
+// what is read again (86 MB on 81,920 unknowns; without the hints the gather
+// went to HBM, 473 us instead of 343).
 __device__ __forceinline__ void mr_issue(const uint8_t *src, uint32_t bytes, uint32_t g, uint8_t *ring,
-                                         uint64_t *full) {
+                                         uint64_t *full, uint64_t policy) {
   const uint32_t s = g % kMRingChunks;
   const uint32_t off = g << kMChunkLog;
   const uint32_t nb = min((uint32_t)kMChunkBytes, bytes - off);
   const uint32_t nm = s == 0 ? min(nb, (uint32_t)kMirrorBytes) : 0u;
   mbar_arrive_expect_tx(&full[s], nb + nm);
-  bulk_g2s(ring + ((size_t)s << kMChunkLog), src + off, nb, &full[s]);
-  if (nm) bulk_g2s(ring + kMRingBytes, src + off, nm, &full[s]);
+  bulk_g2s_hint(ring + ((size_t)s << kMChunkLog), src + off, nb, &full[s], policy);
+  if (nm) bulk_g2s_hint(ring + kMRingBytes, src + off, nm, &full[s], policy);
 }
 
 __device__ __forceinline__ void mr_producer(const uint8_t *src, uint32_t bytes, uint8_t *ring, uint64_t *full,
                                             uint64_t *empty, int *err, uint64_t tmo) {
   const uint32_t K = (bytes + kMChunkBytes - 1) >> kMChunkLog;
+  const uint64_t policy = l2_policy_stream();
   uint32_t issued = 0;
   for (uint32_t g = 0; g < K; ++g) {
     if (g >= (uint32_t)kMRingChunks && !mbar_wait(&empty[g % kMRingChunks], ((g / kMRingChunks) - 1) & 1, tmo)) {
       atomicOr(err, kErrProducer);
       break;
     }
-    mr_issue(src, bytes, g, ring, full);
+    mr_issue(src, bytes, g, ring, full, policy);
     issued = g + 1;
   }
   // copies still in flight land before the CTA exits
@@ -144,17 +148,16 @@ __device__ __forceinline__ void mr_producer(const uint8_t *src, uint32_t bytes, 
 }
 
 struct MSmem {
-  uint8_t *ring, *xst, *rec;
+  uint8_t *ring, *xst;
   RunLite *lite;
   uint64_t *full, *empty, *xfull, *xempty, *accfull, *accempty, *pdone, *gdone, *mdone;
-  uint32_t *tmem, *gen0, *xcnt;
+  uint32_t *tmem, *gen0;
 };
 
 __device__ __forceinline__ MSmem mlayout(uint8_t *b) {
   MSmem s;
   s.ring = b + MLayout::ring;
   s.xst = b + MLayout::xst;
-  s.rec = b + MLayout::rec;
   s.lite = reinterpret_cast<RunLite *>(b + MLayout::lite);
   s.full = reinterpret_cast<uint64_t *>(b + MLayout::full);
   s.empty = reinterpret_cast<uint64_t *>(b + MLayout::empty);
@@ -167,7 +170,6 @@ __device__ __forceinline__ MSmem mlayout(uint8_t *b) {
   s.mdone = reinterpret_cast<uint64_t *>(b + MLayout::mdone);
   s.tmem = reinterpret_cast<uint32_t *>(b + MLayout::tmem);
   s.gen0 = reinterpret_cast<uint32_t *>(b + MLayout::gen0);
-  s.xcnt = reinterpret_cast<uint32_t *>(b + MLayout::xcnt);
   return s;
 }
 
@@ -181,111 +183,123 @@ __device__ __forceinline__ uint32_t run_slices(const RunLite &L) {
   return (4u * L.npanel + kSliceCols - 1) / kSliceCols;
 }
 
-// ---- gather warp gi: slices q = gi, gi + kGathWarps, ... of the launch ----
-// Lane (c = lane & 3, m0 = lane >> 2) copies column c of every 4-column chunk
-// for right-hand sides m0, m0 + 8, ...: consecutive lanes write consecutive
-// words of the stage.  A stage column past the run's real columns is zero.
-// The record of the next run with a slice of this warp is fetched into the
-// other of the warp's two record buffers while it stages the current one.
+// ---- gather warp gi: its columns of slices q = gs, gs + kXStages, ... ----
+// A slice is a transpose: its columns are rows of X (or zbu), 64 consecutive
+// floats each, and the stage holds 16-byte groups of 4 columns per right-hand
+// side.  A lane loads its two right-hand sides (lane, lane + 32) of 4 columns
+// and stores two groups, so loads and stores are whole lines and no lane
+// exchanges anything; the loads of half its columns are in flight while it
+// waits for the stage.  What bounds the kernel is this gather (263 of its 287
+// us on 81,920 unknowns): 1.3 GB through L2 with 64 KB in flight per SM.
+// Measured there: 4-byte asynchronous copies into the stage, one per element,
+// 583 us in all (with the old issue loop); 16-byte loads transposed 4 x 4 in
+// registers on 8 warps 411; this with the stage waited for before the loads
+// 318; 3 stages, 64-, 96-, 160- or 192-column slices 302-375.  Which row a
+// column is comes from `cols`, one word a column, fetched a slice ahead.
+constexpr int kGathUnroll = 4;  // chunks of 4 columns whose loads are in flight together
+static_assert(kWarpCols % (4 * kGathUnroll) == 0, "whole batches of chunks");
+
 __device__ __forceinline__ void mr_gather(const MatmatArgs &a, const CtaInfo &ci, uint32_t nr, const MSmem &sm,
                                           uint32_t gi) {
   const int lane = threadIdx.x & 31;
-  const uint32_t c4 = lane & 3, m0 = lane >> 2;
-  const RunRec *recs = a.recs + ci.rec_begin;
-  uint8_t *rbuf = sm.rec + gi * 2 * kRecBytes;
-  // the next run at or after r (slice counter q at r) that holds a slice of this warp
-  auto next_own = [&](uint32_t &r, uint32_t &q) {
-    for (; r < nr; ++r) {
-      const uint32_t nsl = run_slices(sm.lite[r]);
-      if ((gi + kGathWarps - q % kGathWarps) % kGathWarps < nsl) return;
-      q += nsl;
+  const uint32_t gs = gi / kSliceWarps, col0 = (gi % kSliceWarps) * kWarpCols;  // this warp's stage and columns of it
+  // a place in the CTA's slices: slice s of run r, whose first slice is q and
+  // first panel column c
+  struct Place {
+    uint32_t r, q, s;
+    uint64_t c;
+  };
+  // on to the next slice of this warp's stage, from (r, s)
+  auto settle = [&](Place &p) {
+    for (; p.r < nr; ++p.r, p.s = 0) {
+      const uint32_t np = sm.lite[p.r].npanel, nsl = (4u * np + kSliceCols - 1) / kSliceCols;
+      p.s += (gs + kXStages - (p.q + p.s) % kXStages) % kXStages;
+      if (p.s < nsl) return;
+      p.q += nsl;
+      p.c += 4u * np;
     }
   };
-  auto fetch = [&](uint32_t r, uint32_t b) {
-    const uint8_t *src = reinterpret_cast<const uint8_t *>(recs + r);
-#pragma unroll
-    for (uint32_t o = 0; o < (uint32_t)kRecBytes; o += 512)
-      cp_async16cg(rbuf + b * kRecBytes + o + lane * 16, src + o + lane * 16);
+  // the vector row of its slice's column `lane` of this warp's
+  auto fetch = [&](const Place &p) {
+    const uint32_t ncol = p.r < nr ? 4u * sm.lite[p.r].npanel : 0u, sc = p.s * kSliceCols + col0 + lane;
+    return sc < ncol ? __ldg(a.cols + p.c + sc) : kNoCol;
   };
+  float4 *const st = reinterpret_cast<float4 *>(sm.xst + gs * kSliceBytes + (col0 / 4) * kChunkXBytes);
   bool ok = true, zbu_ready = false;
-  uint32_t r = 0, q = 0, b = 0;
-  next_own(r, q);
-  if (r < nr) fetch(r, 0);
-  while (ok && r < nr) {
-    const RunLite L = sm.lite[r];
-    const uint32_t nsl = run_slices(L), mine0 = (gi + kGathWarps - q % kGathWarps) % kGathWarps;
-    cp_async_wait_all();  // this run's record has landed
-    __syncwarp();
-    uint32_t rn = r + 1, qn = q + nsl;
-    next_own(rn, qn);
-    if (rn < nr) fetch(rn, b ^ 1u);
-    const uint8_t *rec = rbuf + b * kRecBytes;
-    const Run &hdr = *reinterpret_cast<const Run *>(rec);
-    const Seg *seg = reinterpret_cast<const Seg *>(rec + sizeof(Run));
-    const uint32_t kind = L.flags & 0xffu, vlen = hdr.vlen, nseg = hdr.nseg;
-    const float *vec = kind == kRunU ? a.zbu : a.x;
-    if (kind == kRunU && !zbu_ready) {
+  Place at{0, 0, 0, ci.col_begin};
+  settle(at);
+  uint32_t next_row = fetch(at);
+  while (at.r < nr) {
+    const RunLite L = sm.lite[at.r];
+    const uint32_t qs = at.q + at.s, cols = min((uint32_t)kSliceCols, 4u * L.npanel - at.s * kSliceCols);
+    const bool zbu = (L.flags & 0xffu) == kRunU;
+    if (zbu && !zbu_ready) {
       ok = warp_wait(sm.gdone, 0, a.timeout_ns);  // every CTA's zbu rows are written
       __threadfence();
       zbu_ready = true;
       if (!ok) break;
     }
-    uint32_t si = 0;  // this lane's segment cursor (segments are in stage order)
-    for (uint32_t s = mine0; s < nsl && ok; s += kGathWarps) {
-      const uint32_t qs = q + s, slot = qs % kXStages;
-      if (qs >= (uint32_t)kXStages) ok = warp_wait(&sm.xempty[slot], ((qs / kXStages) - 1) & 1, a.timeout_ns);
-      if (!ok) break;
-      float *st = reinterpret_cast<float *>(sm.xst + slot * kSliceBytes);
-      const uint32_t ncol = min((uint32_t)kSliceCols, 4u * L.npanel - s * kSliceCols);
-      for (uint32_t k = 0; k < ncol / 4; ++k) {
-        const uint32_t sc = s * kSliceCols + 4 * k + c4;  // stage column of this lane
-        while (si < nseg && (uint32_t)seg[si].dst + seg[si].len <= sc) ++si;
-        float *dst = st + k * (kChunkXBytes / 4) + c4;
-        if (sc < vlen && si < nseg && seg[si].dst <= sc) {
-          const float *src = vec + (size_t)(seg[si].src + (sc - seg[si].dst)) * kNrhs;
+    const float *vec = (zbu ? a.zbu : a.x) + lane;
+    const uint32_t row = next_row;
+    ++at.s;
+    settle(at);
+    next_row = fetch(at);
+    const uint32_t nchunk = (min(max(cols, col0), col0 + kWarpCols) - col0) / 4;  // of this warp
+    // the MMAs have left the stage's previous slice (a warp without columns in
+    // this slice waits too: its arrival below belongs to this slice's phase)
+    auto stage_free = [&]() {
+      return qs < (uint32_t)kXStages || warp_wait(&sm.xempty[gs], ((qs / kXStages) - 1) & 1, a.timeout_ns);
+    };
+    if (nchunk == 0) ok = stage_free();
+    for (uint32_t k0 = 0; k0 < nchunk; k0 += kGathUnroll) {
+      float v[kGathUnroll][4][2];
 #pragma unroll
-          for (uint32_t t = 0; t < 8; ++t) cp_async4(dst + (m0 + 8 * t) * 4, src + m0 + 8 * t);
-        } else {
+      for (uint32_t u = 0; u < kGathUnroll; ++u)
 #pragma unroll
-          for (uint32_t t = 0; t < 8; ++t) dst[(m0 + 8 * t) * 4] = 0.0f;
+        for (uint32_t c = 0; c < 4; ++c) {
+          const uint32_t src = __shfl_sync(0xffffffffu, row, 4 * (k0 + u) + c);  // kNoCol past the slice's columns
+          v[u][c][0] = v[u][c][1] = 0.0f;
+          if (src != kNoCol) {  // through L2: zbu is written by this launch
+            const float *p = vec + (size_t)src * kNrhs;
+            v[u][c][0] = __ldcg(p);
+            v[u][c][1] = __ldcg(p + 32);
+          }
         }
-      }
-      cp_async_wait_all();
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // visible to the tensor cores
-      __syncwarp();
-      if (lane == 0) {
-        st_release_s(&sm.xcnt[slot], qs / kXStages + 1);
-        mbar_arrive(&sm.xfull[slot]);
+      if (k0 == 0 && !(ok = stage_free())) break;  // the loads need no stage, the stores do
+#pragma unroll
+      for (uint32_t u = 0; u < kGathUnroll; ++u) {
+        if (k0 + u >= nchunk) break;
+        float4 *dst = st + (k0 + u) * kNrhs + lane;
+        dst[0] = make_float4(v[u][0][0], v[u][1][0], v[u][2][0], v[u][3][0]);
+        dst[32] = make_float4(v[u][0][1], v[u][1][1], v[u][2][1], v[u][3][1]);
       }
     }
-    r = rn;
-    q = qn;
-    b ^= 1u;
+    if (!ok) break;
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // visible to the tensor cores
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&sm.xfull[gs]);
   }
   if (!ok && lane == 0) atomicOr(a.err, kErrPipeline);
-  cp_async_wait_all();
 }
 
-// One thread's bounded wait until a shared counter reaches `need`.
-__device__ __forceinline__ bool thread_count_wait(const unsigned *cnt, unsigned need, uint64_t timeout_ns) {
-  if (ld_acquire_s(cnt) >= need) return true;
-  const uint64_t t0 = gtimer();
-  while (ld_acquire_s(cnt) < need)
-    if (gtimer() - t0 > timeout_ns) return false;
-  return true;
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
 }
 
-// ---- MMA thread ---------------------------------------------------------------
+constexpr uint32_t kMmaUnroll = 4;  // 1: 356 us, 2: 321, 4: 318, 8: 318 (81,920 unknowns)
+// ---- MMA thread (the elected one of warp kMmaWarp) ------------------------------
 // Per slice: wait for its X stage and for every ring chunk its panel pairs
-// touch (at most 16 KB of pairs, two chunks), then issue its MMAs back to
+// touch (at most 32 KB of pairs, three chunks), then issue its MMAs back to
 // back with the descriptors advanced in place, and commit the stage back.
-__device__ __forceinline__ void mr_mma(const MatmatArgs &a, uint32_t nr, uint32_t K, const MSmem &sm, uint32_t me) {
+__device__ __forceinline__ void mr_mma(const MatmatArgs &a, uint32_t nr, uint32_t K, const MSmem &sm) {
   const RunLite *lite = sm.lite;
   const uint64_t tmo = a.timeout_ns;
   const uint32_t tbase = *sm.tmem;
   const uint32_t ring_s = smem_u32(sm.ring), xst_s = smem_u32(sm.xst);
-  uint32_t waited = 0, released = 0, q = 0, nb = 0, nbk = 0;  // nb: blocks so far, nbk: this issuer's
-  bool ok = true, first = true;
+  uint32_t waited = 0, released = 0, q = 0, nb = 0;  // nb: blocks so far
+  bool ok = true;
   // Releases ring chunks below c once the MMAs issued so far are done with
   // them; a chunk is waited for (full) before its release, so the empty
   // phases stay in order.
@@ -303,27 +317,19 @@ __device__ __forceinline__ void mr_mma(const MatmatArgs &a, uint32_t nr, uint32_
   for (uint32_t r = 0; r < nr && ok; ++r) {
     const RunLite L = lite[r];
     if (empty_block(L)) continue;
-    if ((nb & 1u) != me) {  // the other issuer's block: count its slices
-      q += run_slices(L);
-      if (L.flags & kLast) ++nb;
-      continue;
-    }
     const uint32_t h = L.nrow, n8 = (h + 7u) & ~7u, pb = 16u * h;
     const uint32_t idesc = idesc_tf32(kNrhs, n8);
-    const uint32_t buf = 2u * me + (nbk & 1u);
+    const uint32_t buf = nb % kAccs;
     const uint32_t dtm = tbase + buf * kAccCols;
-    if (L.flags & kFirst) {
-      // Hand back the ring chunks below this block first: the epilogue takes
-      // the blocks in order, so the other issuer's earlier block (which may
-      // still need those chunks refilled) must not wait on this issuer.
-      release_below(L.pos >> kMChunkLog);
+    uint32_t acc = (L.flags & kFirst) ? 0u : 1u;
+    if (!acc) {
       // the epilogue has read this accumulator's previous block
-      if (nbk >= 2 && !(ok = mbar_wait(&sm.accempty[buf], ((nbk >> 1) - 1) & 1, tmo))) break;
+      if (nb >= (uint32_t)kAccs && !(ok = mbar_wait(&sm.accempty[buf], ((nb / kAccs) - 1) & 1, tmo))) break;
       tc_fence_after();  // the epilogue's TMEM reads come before these MMAs' writes
-      first = true;
     }
     const uint32_t nsl = run_slices(L), npair = L.npanel / 2u;
-    for (uint32_t s = 0; s < nsl && ok; ++s, ++q) {
+    const uint64_t bhi = smem_desc(0, pb, 128);  // the descriptor without its address
+    for (uint32_t s = 0; s < nsl; ++s, ++q) {
       const uint32_t slot = q % kXStages;
       const uint32_t p0 = s * (kSliceCols / 8), p1 = min(npair, p0 + kSliceCols / 8);
       const uint32_t pos0 = L.pos + 2u * p0 * pb, pos1 = L.pos + 2u * p1 * pb;
@@ -333,31 +339,45 @@ __device__ __forceinline__ void mr_mma(const MatmatArgs &a, uint32_t nr, uint32_
         ok = mbar_wait(&sm.full[waited % kMRingChunks], (waited / kMRingChunks) & 1, tmo);
         waited += ok ? 1u : 0u;
       }
-      // The stage's fill count first: the other issuer may not have taken
-      // the slot's previous slice yet, and a parity wait two phases ahead
-      // would return at once.
-      if (ok) ok = thread_count_wait(&sm.xcnt[slot], q / kXStages + 1, tmo);
       if (ok) ok = mbar_wait(&sm.xfull[slot], (q / kXStages) & 1, tmo);
       if (!ok) break;
       uint64_t adesc = smem_desc(xst_s + slot * kSliceBytes, kChunkXBytes, 128);
       uint32_t baddr = ring_s + ((pos0 >> kMChunkLog) % kMRingChunks) * kMChunkBytes + (pos0 & (kMChunkBytes - 1));
-      const uint64_t bhi = smem_desc(0, pb, 128);  // the descriptor without its address
-      for (uint32_t p = p0; p < p1; ++p) {
-        mma_tf32(dtm, adesc, bhi | (uint64_t)((baddr >> 4) & 0x3fffu), idesc, first ? 0u : 1u);
-        first = false;
+      const uint32_t step = 2u * pb;
+      uint32_t p = p0;
+      for (; p + kMmaUnroll <= p1; p += kMmaUnroll) {
+        uint32_t ad[kMmaUnroll], bd[kMmaUnroll];
+#pragma unroll
+        for (uint32_t u = 0; u < kMmaUnroll; ++u) {
+          ad[u] = (uint32_t)adesc + u * ((2u * kChunkXBytes) >> 4);
+          uint32_t ba = baddr + u * step;
+          if (ba >= ring_s + kMRingBytes) ba -= kMRingBytes;  // a pair that starts past the ring's end
+          bd[u] = (uint32_t)bhi | (ba >> 4);
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < kMmaUnroll; ++u) {
+          mma_tf32(dtm, (adesc & 0xffffffff00000000ull) | ad[u], (bhi & 0xffffffff00000000ull) | bd[u], idesc, acc);
+          acc = 1;
+        }
+        adesc += kMmaUnroll * ((2u * kChunkXBytes) >> 4);
+        baddr += kMmaUnroll * step;
+        if (baddr >= ring_s + kMRingBytes) baddr -= kMRingBytes;
+      }
+      for (; p < p1; ++p) {
+        mma_tf32(dtm, adesc, bhi | (uint64_t)(baddr >> 4), idesc, acc);
+        acc = 1;
         adesc += (2u * kChunkXBytes) >> 4;  // the next two K chunks of the stage
-        baddr += 2u * pb;
-        if (baddr >= ring_s + kMRingBytes) baddr -= kMRingBytes;  // a pair that starts past the ring's end
+        baddr += step;
+        if (baddr >= ring_s + kMRingBytes) baddr -= kMRingBytes;
       }
       tc_commit(&sm.xempty[slot]);  // the stage slot is free once these MMAs are done
     }
     if (ok && (L.flags & kLast)) {
       tc_commit(&sm.accfull[buf]);
-      ++nbk;
       ++nb;
     }
   }
-  release_below(K);
+  if (ok) release_below(K);
   if (!ok) atomicOr(a.err, kErrPipeline);
   // every MMA has completed before TMEM is handed back
   tc_commit(sm.mdone);
@@ -397,9 +417,8 @@ __device__ __forceinline__ void mr_epilogue(const MatmatArgs &a, uint32_t nr, ui
       if (kind == kRunP && ++np_done == nblk_p && lane == 0) mbar_arrive(sm.pdone);
       continue;
     }
-    // block nb: issuer nb & 1, that issuer's block nbk = nb >> 1 in its accumulator nbk & 1
-    const uint32_t nbk = nb >> 1, buf = 2u * (nb & 1u) + (nbk & 1u);
-    ok = warp_wait(&sm.accfull[buf], (nbk >> 1) & 1, a.timeout_ns);
+    const uint32_t buf = nb % kAccs;
+    ok = warp_wait(&sm.accfull[buf], (nb / kAccs) & 1, a.timeout_ns);
     if (!ok) break;
     tc_fence_after();
     const uint32_t taddr = *sm.tmem + tlane + buf * kAccCols;
@@ -423,10 +442,10 @@ __device__ __forceinline__ void mr_epilogue(const MatmatArgs &a, uint32_t nr, ui
         } else {
           double old[16];
 #pragma unroll
-          for (uint32_t i = 0; i < 16; ++i) old[i] = (add && i < n) ? src[o0 + (size_t)i * kNrhs] : 0.0;
+          for (uint32_t i = 0; i < 16; ++i) old[i] = (add && i < n) ? __ldcs(src + o0 + (size_t)i * kNrhs) : 0.0;
 #pragma unroll
           for (uint32_t i = 0; i < 16; ++i)
-            if (i < n) a.y[o0 + (size_t)i * kNrhs] = fma(a.alpha, (double)__uint_as_float(v[i]), c * old[i]);
+            if (i < n) __stcs(a.y + o0 + (size_t)i * kNrhs, fma(a.alpha, (double)__uint_as_float(v[i]), c * old[i]));
         }
       }
     }
@@ -449,20 +468,19 @@ __global__ void __launch_bounds__(kThreadsM, 1) k_matmat(MatmatArgs a) {
   if (threadIdx.x == 0) {
     for (int i = 0; i < kMRingChunks; ++i) {
       mbar_init(&sm.full[i], 1);
-      mbar_init(&sm.empty[i], kIssuers);  // both issuers hand every chunk back
+      mbar_init(&sm.empty[i], 1);
     }
     for (int i = 0; i < kXStages; ++i) {
-      mbar_init(&sm.xfull[i], 1);
+      mbar_init(&sm.xfull[i], kSliceWarps);
       mbar_init(&sm.xempty[i], 1);
-      sm.xcnt[i] = 0;
     }
-    for (int i = 0; i < 2 * kIssuers; ++i) {
+    for (int i = 0; i < kAccs; ++i) {
       mbar_init(&sm.accfull[i], 1);
       mbar_init(&sm.accempty[i], kEpiWarps);
     }
     mbar_init(sm.pdone, kEpiWarps);
     mbar_init(sm.gdone, 1);
-    mbar_init(sm.mdone, kIssuers);
+    mbar_init(sm.mdone, 1);
     *sm.gen0 = grid_gen0(a.gbar);
     mbar_fence_init();
   }
@@ -505,12 +523,8 @@ __global__ void __launch_bounds__(kThreadsM, 1) k_matmat(MatmatArgs a) {
     }
     return;
   }
-  if (w == kMmaWarp2) {
-    if (lane == 0) mr_mma(a, nr, K, sm, 1);
-    return;  // its MMAs are complete (mdone) before warp kMmaWarp frees TMEM
-  }
   if (w == kMmaWarp) {
-    if (lane == 0) mr_mma(a, nr, K, sm, 0);
+    if (elect_one()) mr_mma(a, nr, K, sm);
     __syncwarp();
   } else {
     mr_epilogue(a, nr, ci.nblk_p, sm);
@@ -524,7 +538,37 @@ __global__ void __launch_bounds__(kThreadsM, 1) k_matmat(MatmatArgs a) {
                  : "memory");
 }
 
+// cols[CTA's col_begin + column] = the vector row of the run's column (kNoCol past its real ones).
+__global__ void k_matmat_cols(const RunRec *recs, const CtaInfo *ctas, uint32_t *cols) {
+  const CtaInfo ci = ctas[blockIdx.x];
+  const uint32_t nr = ci.nr_p + ci.nr_d + ci.nr_u;
+  uint64_t c = ci.col_begin;
+  for (uint32_t r = 0; r < nr; ++r) {
+    const RunRec &rec = recs[ci.rec_begin + r];
+    const uint32_t ncol = 4u * rec.hdr.npanel, vlen = rec.hdr.vlen;
+    for (uint32_t k = threadIdx.x; k < ncol; k += blockDim.x) {
+      uint32_t row = kNoCol;
+      if (k < vlen) {
+        uint32_t lo = 0, hi = rec.hdr.nseg;  // the last segment that starts at or before k (in stage order)
+        while (hi - lo > 1) {
+          const uint32_t mid = (lo + hi) >> 1;
+          if (rec.seg[mid].dst <= k) lo = mid;
+          else hi = mid;
+        }
+        row = rec.seg[lo].src + (k - rec.seg[lo].dst);
+      }
+      cols[c + k] = row;
+    }
+    c += ncol;
+  }
+}
+
 }  // namespace
+
+cudaError_t launch_matmat_cols(const RunRec *recs, const CtaInfo *ctas, int num_ctas, uint32_t *cols, cudaStream_t s) {
+  k_matmat_cols<<<num_ctas, 256, 0, s>>>(recs, ctas, cols);
+  return cudaGetLastError();
+}
 
 size_t matmat_smem_bytes() { return MLayout::bytes; }
 

@@ -464,7 +464,7 @@ int make_plan(const stc_HACApK_leafmtxp *st, int nd, int num_ctas, Plan &plan, s
       work[c].failed = true;
     }
   }
-  uint64_t off = 0;
+  uint64_t off = 0, ncol = 0;
   size_t nrec = 0;
   for (int c = 0; c < num_ctas; ++c) {
     CtaInfo &info = plan.ctas[c];
@@ -484,6 +484,10 @@ int make_plan(const stc_HACApK_leafmtxp *st, int nd, int num_ctas, Plan &plan, s
     }
     info.stream_off = off;
     info.rec_begin = (uint32_t)nrec;
+    if (pair_panels) {
+      info.col_begin = ncol;
+      for (const RunLite &L : work[c].lite) ncol += (uint64_t)G * L.npanel;
+    }
     off += (work[c].bytes + 255) & ~uint64_t(255);
     nrec += work[c].recs.size();
     plan.pad_bytes += work[c].pad;
@@ -496,6 +500,7 @@ int make_plan(const stc_HACApK_leafmtxp *st, int nd, int num_ctas, Plan &plan, s
     std::copy(work[c].lite.begin(), work[c].lite.end(), plan.lite.begin() + plan.ctas[c].rec_begin);
   }
   plan.total_bytes = std::max<uint64_t>(off, 256);
+  plan.panel_cols = ncol;
   return HBX_OK;
 }
 

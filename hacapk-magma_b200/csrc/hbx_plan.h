@@ -225,7 +225,8 @@ struct CtaInfo {
   uint32_t nr_p, nr_d, nr_u;
   uint32_t atom_begin, n_atoms;  // owned atoms (rows written by this CTA)
   uint32_t nblk_p;               // P blocks (slabs) of the CTA
-  uint32_t pad[6];
+  uint64_t col_begin;            // multi-RHS layout: panel columns of the CTAs before this one
+  uint32_t pad[4];
 };
 static_assert(sizeof(CtaInfo) == 64, "CtaInfo layout");
 
@@ -277,6 +278,7 @@ struct Plan {
   std::vector<uint64_t> zoff;       // zbu offset of each low-rank leaf
   uint64_t total_bytes = 0;         // packed buffer size
   uint64_t zbu_len = 0;
+  uint64_t panel_cols = 0;          // multi-RHS layout: panel columns of every run
   uint64_t dense_words = 0, lowrank_words = 0;
   uint64_t pad_bytes = 0;           // zero columns that fill a block's last panel
   uint64_t alg_bytes = 0, alg_flops = 0;
