@@ -108,6 +108,29 @@ constexpr uint32_t kNoCol = 0xffffffffu;
 // Forms MatmatArgs::cols from the run records (once per engine).
 cudaError_t launch_matmat_cols(const RunRec *recs, const CtaInfo *ctas, int num_ctas, uint32_t *cols, cudaStream_t s);
 
+// FP64 product with kNrhs right-hand sides of a single-vector FP64 engine
+// (hbx_mm64.cu).  A unit: runs [r0, r0 + n0) and [r1, r1 + n1) of CTA `cta`.
+struct Mm64Unit {
+  uint32_t cta, r0, n0, r1, n1;
+};
+struct Mm64Args {
+  const uint8_t *stream;
+  const RunRec *recs;
+  const CtaInfo *ctas;
+  const Mm64Unit *units;
+  uint32_t nunits;
+  unsigned *next;  // unit counters of the two launches
+  const double *x, *yin;
+  double *y, *zbu;  // zbu: [zbu_len][kNrhs]
+  double alpha, beta;
+};
+cudaError_t configure_mm64();
+// The P units and the row-atom units of a plan, each in descending cost.
+void mm64_units(const std::vector<CtaInfo> &ctas, const std::vector<RunLite> &lite, std::vector<Mm64Unit> &p,
+                std::vector<Mm64Unit> &rest);
+cudaError_t launch_mm64(const Mm64Args &a, const Mm64Unit *p, uint32_t np, const Mm64Unit *rest, uint32_t nrest,
+                        cudaStream_t s);
+
 // Multi-RHS BiCGSTAB (hbx_mrhs_solve.cu): scalars of one right-hand side.
 struct MrScal {
   double alpha, zeta, rho, beta, rr, rtol;
@@ -250,6 +273,12 @@ struct hbx_hmat {
   int *d_mrint = nullptr;       // any_active, mask[kNrhs]
   double *d_mrdbl = nullptr;    // thresholds[kNrhs], norms[kNrhs]
   void *h_mrpin = nullptr;      // pinned: MrScal[kNrhs], norms, thresholds, ints
+  // FP64 product with kNrhs right-hand sides (hbx_mm64.cu), made by the first
+  // multi-RHS solve that uses this engine: units, their counters, zbu
+  hbx::Mm64Unit *d_mm64 = nullptr;
+  uint32_t mm64_p = 0, mm64_rest = 0;
+  unsigned *d_mm64_next = nullptr;
+  double *d_mm64_zbu = nullptr;
   // block-diagonal batch of independent instances (hbx_create_batch)
   std::vector<int> inst_off;    // row offsets, count + 1 entries (empty: one instance)
   int *d_inst_off = nullptr;    // the same on the device
