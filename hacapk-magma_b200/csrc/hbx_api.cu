@@ -1413,19 +1413,24 @@ struct MrPinned {
   double norm[hbx::kNrhs];
   double thresh[hbx::kNrhs];
   int mask[hbx::kNrhs];
-  int any;
+  int any[2];  // any_active after the last two batches of steps
 };
 
 // Each buffer is tested on its own, so a call after a failed allocation
 // completes the set instead of running on a null pointer.
 int ensure_mr_workspace(hbx_hmat *hm) {
   const size_t n = (size_t)hm->plan.nd * hbx::kNrhs;
-  if (!hm->d_mrv) HBX_CUDA(dev_malloc(&hm->d_mrv, 10 * n * sizeof(double)));
+  if (!hm->d_mrv) HBX_CUDA(dev_malloc(&hm->d_mrv, 9 * n * sizeof(double)));
   if (!hm->d_mr32) HBX_CUDA(dev_malloc(&hm->d_mr32, n * sizeof(float)));
   if (!hm->d_mrpart)
     HBX_CUDA(dev_malloc(&hm->d_mrpart, (size_t)hbx::mr_row_blocks(hm->plan.nd) * 2 * hbx::kNrhs * sizeof(double)));
   if (!hm->d_mrsc) HBX_CUDA(dev_malloc(&hm->d_mrsc, hbx::kNrhs * sizeof(hbx::MrScal)));
-  if (!hm->d_mrint) HBX_CUDA(dev_malloc(&hm->d_mrint, (1 + hbx::kNrhs) * sizeof(int)));
+  if (!hm->d_mrint) {
+    int *d = nullptr;
+    HBX_CUDA(dev_malloc(&d, (2 + hbx::kNrhs) * sizeof(int)));
+    hm->d_mrint = d;
+    HBX_CUDA(cudaMemset(d, 0, (2 + hbx::kNrhs) * sizeof(int)));
+  }
   if (!hm->d_mrdbl) HBX_CUDA(dev_malloc(&hm->d_mrdbl, 2 * hbx::kNrhs * sizeof(double)));
   if (!hm->h_mrpin) HBX_CUDA(cudaMallocHost(&hm->h_mrpin, sizeof(MrPinned)));
   return HBX_OK;
@@ -1495,6 +1500,7 @@ cudaError_t mr_matmat(void *ctx, const float *x, double *y, cudaStream_t s) {
   a.gbar = hm->d_gbar;
   a.err = hm->d_err;
   a.timeout_ns = hm->timeout_ns;
+  a.go = hm->d_mrint;
   return hbx::launch_matmat(a, hm->num_ctas, s);
 }
 
@@ -1517,15 +1523,15 @@ int hbx_bicgstab_multi(hbx_hmat *h, hbx_hmat *hm, const double *B, double *U, co
   if (st != HBX_OK) return st;
   const int nd = h->plan.nd;
   const size_t n = (size_t)nd * hbx::kNrhs;
-  double *r = hm->d_mrv, *rh = r + n, *p = rh + n, *ap = p + n, *t = ap + n, *at = t + n, *x = at + n, *R = x + n,
+  double *r = hm->d_mrv, *rh = r + n, *p = rh + n, *ap = p + n, *at = ap + n, *x = at + n, *R = x + n,
          *T1 = R + n, *T2 = T1 + n;
   double *d_thr = hm->d_mrdbl, *d_norm = hm->d_mrdbl + hbx::kNrhs;
   int *d_any = hm->d_mrint, *d_mask = hm->d_mrint + 1;
+  unsigned *ticket = reinterpret_cast<unsigned *>(hm->d_mrint + 1 + hbx::kNrhs);
   MrPinned *pin = static_cast<MrPinned *>(hm->h_mrpin);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   auto norms = [&](const double *v) -> int {  // pin->norm[j] = ||v_j||^2
-    HBX_CUDA(hbx::mr_launch_dots(1, nd, v, v, nullptr, nullptr, hm->d_mrpart, s));
-    HBX_CUDA(hbx::mr_launch_colsum(nd, hm->d_mrpart, d_norm, s));
+    HBX_CUDA(hbx::mr_launch_norms(nd, v, hm->d_mrpart, ticket, d_norm, s));
     HBX_CUDA(cudaMemcpyAsync(pin->norm, d_norm, sizeof(pin->norm), cudaMemcpyDeviceToHost, s));
     HBX_CUDA(cudaStreamSynchronize(s));
     return HBX_OK;
@@ -1590,26 +1596,33 @@ int hbx_bicgstab_multi(hbx_hmat *h, hbx_hmat *hm, const double *B, double *U, co
     }
     HBX_CUDA(cudaMemcpyAsync(d_thr, pin->thresh, sizeof(pin->thresh), cudaMemcpyHostToDevice, s));
     HBX_CUDA(cudaMemcpyAsync(d_mask, pin->mask, sizeof(pin->mask), cudaMemcpyHostToDevice, s));
-    HBX_CUDA(hbx::mr_launch_setup(nd, R, r, rh, p, ap, x, s));
-    HBX_CUDA(hbx::mr_launch_dots(1, nd, r, r, nullptr, nullptr, hm->d_mrpart, s));
-    HBX_CUDA(hbx::mr_launch_init(nd, hm->d_mrpart, d_thr, d_mask, hm->d_mrsc, d_any, s));
-    launches += 3;
     hbx::MrStep a{};
     a.nd = nd;
     a.max_iter = std::max(1, max_iter - max_done_iters);
     a.sc = hm->d_mrsc;
     a.any_active = d_any;
-    a.r = r; a.rh = rh; a.p = p; a.ap = ap; a.t = t; a.at = at; a.x = x; a.part = hm->d_mrpart;
+    a.ticket = ticket;
+    a.r = r; a.rh = rh; a.p = p; a.ap = ap; a.at = at; a.x = x; a.part = hm->d_mrpart;
     a.f32 = hm->d_mr32;
     a.matmat = mr_matmat;
     a.ctx = hm;
-    for (int k = 0; k < a.max_iter; k += batch) {
-      HBX_CUDA(cudaMemcpyAsync(&pin->any, d_any, sizeof(int), cudaMemcpyDeviceToHost, s));
-      HBX_CUDA(cudaStreamSynchronize(s));
-      if (!pin->any) break;
+    HBX_CUDA(hbx::mr_launch_setup(a, R, d_thr, d_mask, s));
+    ++launches;
+    // A batch of steps is queued while the flag of the one before is read, so
+    // the device does not wait for the host; after the last RHS is done the
+    // queued launches return at once.
+    cudaEvent_t flag[2] = {hm->ev3, hm->ev4};
+    int nbatch = 0;
+    for (int k = 0; k < a.max_iter; k += batch, ++nbatch) {
       for (int b = 0; b < batch; ++b) HBX_CUDA(hbx::mr_launch_step(a, s));
-      launches += 10 * batch;
+      HBX_CUDA(cudaMemcpyAsync(&pin->any[nbatch & 1], d_any, sizeof(int), cudaMemcpyDeviceToHost, s));
+      HBX_CUDA(cudaEventRecord(flag[nbatch & 1], s));
+      launches += 7 * batch;
       steps += batch;
+      if (nbatch > 0) {
+        HBX_CUDA(cudaEventSynchronize(flag[(nbatch - 1) & 1]));
+        if (!pin->any[(nbatch - 1) & 1]) break;
+      }
     }
     HBX_CUDA(cudaMemcpyAsync(pin->sc, hm->d_mrsc, sizeof(pin->sc), cudaMemcpyDeviceToHost, s));
     HBX_CUDA(hbx::mr_launch_add(nd, d_mask, x, U, s));

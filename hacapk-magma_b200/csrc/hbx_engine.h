@@ -100,6 +100,7 @@ struct MatmatArgs {
   unsigned *gbar;
   int *err;
   unsigned long long timeout_ns;
+  const int *go;  // optional: the launch does nothing while *go is 0 (a solver's flag)
 };
 size_t matmat_smem_bytes();
 cudaError_t configure_matmat();
@@ -136,26 +137,22 @@ struct MrScal {
   double alpha, zeta, rho, beta, rr, rtol;
   int active, iters, status, pad;
 };
-// One step for every right-hand side still running (10 launches, two of
-// them the product through `matmat`).
+// One step for every right-hand side still running (7 launches, two of them
+// the product through `matmat`); nothing is done once *any_active is 0.
 struct MrStep {
   int nd, max_iter;
   MrScal *sc;
   int *any_active;
-  double *r, *rh, *p, *ap, *t, *at, *x, *part;
+  unsigned *ticket;  // last-block counter of the reductions, zero between launches
+  double *r, *rh, *p, *ap, *at, *x, *part;  // t lies in r between the step's two products
   float *f32;  // the product's input (p, then t, rounded to float)
   cudaError_t (*matmat)(void *ctx, const float *x, double *y, cudaStream_t s);
   void *ctx;
 };
 int mr_row_blocks(int nd);
-cudaError_t mr_launch_dots(int nq, int nd, const double *x0, const double *y0, const double *x1, const double *y1,
-                           double *part, cudaStream_t s);
-cudaError_t mr_launch_setup(int nd, const double *R, double *r, double *rh, double *p, double *ap, double *x,
-                            cudaStream_t s);
-cudaError_t mr_launch_init(int nd, const double *part, const double *thresh, const int *mask, MrScal *sc,
-                           int *any_active, cudaStream_t s);
+cudaError_t mr_launch_norms(int nd, const double *v, double *part, unsigned *ticket, double *out, cudaStream_t s);
+cudaError_t mr_launch_setup(const MrStep &a, const double *R, const double *thresh, const int *mask, cudaStream_t s);
 cudaError_t mr_launch_step(const MrStep &a, cudaStream_t s);
-cudaError_t mr_launch_colsum(int nd, const double *part, double *out, cudaStream_t s);
 cudaError_t mr_launch_transpose(int rows, int cols, const double *in, double *out, cudaStream_t s);
 cudaError_t mr_launch_resid(int nd, const double *B, const double *HU, double *R, cudaStream_t s);
 cudaError_t mr_launch_add(int nd, const int *mask, const double *D, double *U, cudaStream_t s);
@@ -266,11 +263,11 @@ struct hbx_hmat {
   uint32_t *d_mcols = nullptr;  // multi-RHS engine: MatmatArgs::cols
   float *d_zbum = nullptr;  // multi-RHS engine: zbu for all right-hand sides [zbu_len][kNrhs]
   // multi-RHS solver workspace (hbx_bicgstab_multi)
-  double *d_mrv = nullptr;      // r, rh, p, ap, t, at, x, R, and two kNrhs x nd scratch arrays
+  double *d_mrv = nullptr;      // r, rh, p, ap, at, x, R, and two kNrhs x nd scratch arrays
   float *d_mr32 = nullptr;      // nd x kNrhs
   double *d_mrpart = nullptr;   // [row blocks][2][kNrhs]
   hbx::MrScal *d_mrsc = nullptr;
-  int *d_mrint = nullptr;       // any_active, mask[kNrhs]
+  int *d_mrint = nullptr;       // any_active, mask[kNrhs], the reductions' ticket
   double *d_mrdbl = nullptr;    // thresholds[kNrhs], norms[kNrhs]
   void *h_mrpin = nullptr;      // pinned: MrScal[kNrhs], norms, thresholds, ints
   // FP64 product with kNrhs right-hand sides (hbx_mm64.cu), made by the first

@@ -460,6 +460,7 @@ __device__ __forceinline__ void mr_epilogue(const MatmatArgs &a, uint32_t nr, ui
 
 __global__ void __launch_bounds__(kThreadsM, 1) k_matmat(MatmatArgs a) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
+  if (a.go && !*(volatile const int *)a.go) return;  // set by an earlier launch: the same on every CTA
   const MSmem sm = mlayout(smem_raw);
   const CtaInfo ci = a.ctas[blockIdx.x];
   const uint32_t nr = ci.nr_p + ci.nr_d + ci.nr_u;
