@@ -113,7 +113,8 @@ void free_engine(hbx_hmat *h) {
   cudaFree(h->d_btv);
   cudaFree(h->d_btsc);
   cudaFree(h->d_btdbl);
-  cudaFree(h->d_btany);
+  cudaFree(h->d_btflags);
+  if (h->h_btany) cudaFreeHost(h->h_btany);
   if (h->h_pin) cudaFreeHost(h->h_pin);
   if (h->h_state) cudaFreeHost(h->h_state);
   if (h->ev0) cudaEventDestroy(h->ev0);
@@ -1696,9 +1697,20 @@ bool skip_disabled() {
   return v && std::atoi(v) != 0;
 }
 
+// One of the steps' products (the vector kernels have written the float copy
+// of x); nothing is done once no instance runs.
 cudaError_t bt_matvec(void *ctx, const double *x, double *y, cudaStream_t s) {
   hbx_hmat *h = static_cast<hbx_hmat *>(ctx);
-  return mv_launch(h, matvec_args(h, 1.0, x, 0.0, nullptr, y), s);
+  hbx::MatvecArgs a = matvec_args(h, 1.0, x, 0.0, nullptr, y);
+  a.skip = &h->d_btflags->done;
+  return hbx::launch_matvec(a, h->num_ctas, s, h->plan.precision);
+}
+
+// CTAs per instance of the vector kernels, by the largest instance.
+int bt_cluster_of(const hbx_hmat *h) {
+  int most = 0;
+  for (size_t k = 0; k + 1 < h->inst_off.size(); ++k) most = std::max(most, h->inst_off[k + 1] - h->inst_off[k]);
+  return hbx::bt_cluster(most);
 }
 
 // A plain engine is one instance.  Its tables are published (inst_off set)
@@ -1716,8 +1728,14 @@ int ensure_bt_workspace(hbx_hmat *h, int count) {
   }
   if (!h->d_btv) HBX_CUDA(dev_malloc(&h->d_btv, 6 * n * sizeof(double)));
   if (!h->d_btsc) HBX_CUDA(dev_malloc(&h->d_btsc, count * sizeof(hbx::MrScal)));
-  if (!h->d_btdbl) HBX_CUDA(dev_malloc(&h->d_btdbl, 5 * (size_t)count * sizeof(double)));
-  if (!h->d_btany) HBX_CUDA(dev_malloc(&h->d_btany, sizeof(int)));
+  if (!h->d_btdbl) HBX_CUDA(dev_malloc(&h->d_btdbl, 3 * (size_t)count * sizeof(double)));
+  if (!h->h_btany) HBX_CUDA(cudaMallocHost(&h->h_btany, 2 * sizeof(int)));
+  if (!h->d_btflags) {
+    hbx::BtFlags *f = nullptr;
+    HBX_CUDA(dev_malloc(&f, sizeof(hbx::BtFlags)));
+    h->d_btflags = f;
+    HBX_CUDA(cudaMemset(f, 0, sizeof(hbx::BtFlags)));
+  }
   return HBX_OK;
 }
 
@@ -1734,37 +1752,47 @@ static int batch_dev(hbx_hmat *h, const double *b, double *u, double tol, const 
   if (st != HBX_OK) return st;
   const size_t n = (size_t)h->plan.nd;
   double *r = h->d_btv, *rh = r + n, *p = rh + n, *ap = p + n, *t = ap + n, *at = t + n;
-  double *dots = h->d_btdbl, *bnorm = dots + 2 * (size_t)count, *tnorm = bnorm + count;
+  double *bnorm = h->d_btdbl, *tnorm = bnorm + count;
   HBX_CUDA(cudaEventRecord(h->ev0, s));
-  // r = b - H u, rh = r, p = Ap = 0; the stop test of every instance
+  // r = b - H u, rh = r, p = r; the stop test of every instance
   HBX_CUDA(mv_launch(h, matvec_args(h, -1.0, u, 1.0, b, r), s));
-  HBX_CUDA(hbx::bt_launch_setup(n, r, rh, p, ap, s));
-  HBX_CUDA(hbx::bt_launch_dots(2, count, h->d_inst_off, r, r, b, b, dots, s));
-  HBX_CUDA(hbx::bt_launch_init(count, dots, tol, rtol, max_iter, h->d_btsc, bnorm, h->d_btany, s));
   hbx::BtStep a{};
-  a.n = n;
   a.count = count;
   a.max_iter = max_iter;
+  a.cluster = bt_cluster_of(h);
   a.off = h->d_inst_off;
-  a.rinst = h->d_rinst;
   a.sc = h->d_btsc;
-  a.any_active = h->d_btany;
-  a.r = r; a.rh = rh; a.p = p; a.ap = ap; a.t = t; a.at = at; a.u = u; a.dots = dots; a.bnorm = bnorm;
+  a.flags = h->d_btflags;
+  a.x32 = h->d_f32;
+  a.r = r; a.rh = rh; a.p = p; a.ap = ap; a.t = t; a.at = at; a.u = u; a.bnorm = bnorm;
   a.matvec = bt_matvec;
   a.ctx = h;
   // products inside the steps stream only the chunks of running instances
   const bool skip = h->d_chunk_inst && !skip_disabled();
   a.pre = skip ? h->d_inst_pre : nullptr;
-  int any = 0, steps = 0, launches = 4;
+  HBX_CUDA(hbx::bt_launch_init(a, b, tol, rtol, s));
+  // A batch of steps is queued while the flag of the one before is read, so
+  // the device does not wait for the host; once no instance runs the queued
+  // launches return at once.
+  int steps = 0, launches = 2;
+  int *any = h->h_btany;
+  cudaEvent_t flag[2] = {h->ev3, h->ev4};
   h->skip_inactive = skip ? 1 : 0;
   cudaError_t le = cudaSuccess;
-  for (;;) {
-    le = cudaMemcpyAsync(&any, h->d_btany, sizeof(int), cudaMemcpyDeviceToHost, s);
-    if (le == cudaSuccess) le = cudaStreamSynchronize(s);
-    if (le != cudaSuccess || !any || steps >= max_iter) break;
-    for (int k = 0; k < batch && le == cudaSuccess; ++k) le = hbx::bt_launch_step(a, s);
-    steps += batch;
-    launches += (skip ? 13 : 11) * batch;
+  for (int nb = 0; le == cudaSuccess; ++nb) {
+    if (steps < max_iter) {
+      for (int k = 0; k < batch && le == cudaSuccess; ++k) le = hbx::bt_launch_step(a, s);
+      steps += batch;
+      launches += 4 * batch;
+    }
+    if (le == cudaSuccess) le = cudaMemcpyAsync(&any[nb & 1], &h->d_btflags->any, sizeof(int), cudaMemcpyDeviceToHost, s);
+    if (le == cudaSuccess) le = cudaEventRecord(flag[nb & 1], s);
+    if (le != cudaSuccess) break;
+    // the first wait is for the first batch itself when no second one may follow
+    const int seen = steps < max_iter ? nb - 1 : nb;
+    if (seen < 0) continue;
+    le = cudaEventSynchronize(flag[seen & 1]);
+    if (le == cudaSuccess && (!any[seen & 1] || steps >= max_iter)) break;
   }
   h->skip_inactive = 0;
   HBX_CUDA(le);
@@ -1772,7 +1800,7 @@ static int batch_dev(hbx_hmat *h, const double *b, double *u, double tol, const 
   if (true_res) {
     // the true residual of every instance: ||b - H u|| / ||b||
     HBX_CUDA(mv_launch(h, matvec_args(h, -1.0, u, 1.0, b, r), s));
-    HBX_CUDA(hbx::bt_launch_dots(1, count, h->d_inst_off, r, r, nullptr, nullptr, tnorm, s));
+    HBX_CUDA(hbx::bt_launch_norms(count, a.cluster, h->d_inst_off, r, tnorm, s));
     launches += 2;
   }
   std::vector<hbx::MrScal> sc(count);
@@ -1842,18 +1870,19 @@ static int batch_refined_dev(hbx_hmat *h, hbx_hmat *hl, const double *b, double 
   int *d_flag = reinterpret_cast<int *>(h->d_rflag);
   double *d_itol = reinterpret_cast<double *>(reinterpret_cast<char *>(h->d_rflag) +
                                               ((size_t)count * sizeof(int) + 15) / 16 * 16);
-  double *dots = h->d_btdbl;  // [count]: per-instance dots of the outer loop
+  double *dots = h->d_btdbl + 2 * (size_t)count;  // [count]: per-instance norms of the outer loop
+  const int cluster = bt_cluster_of(h);
   cudaEventRecord(h->ev2, s);
   std::vector<double> bb(count), rr(count), rel(count, 0.0), itol(count);
   std::vector<int> flag(count), inner(count, 0), status(count, HBX_ERR_NOT_CONVERGED), outer_k(count, 0);
-  HBX_CUDA(hbx::bt_launch_dots(1, count, h->d_inst_off, b, b, nullptr, nullptr, dots, s));
+  HBX_CUDA(hbx::bt_launch_norms(count, cluster, h->d_inst_off, b, dots, s));
   HBX_CUDA(cudaMemcpyAsync(bb.data(), dots, count * sizeof(double), cudaMemcpyDeviceToHost, s));
   HBX_CUDA(cudaStreamSynchronize(s));
   std::vector<hbx_solve_info> ii(count);
   int outer = 0, launches = 1;
   for (;;) {
     HBX_CUDA(mv_launch(h, matvec_args(h, -1.0, u, 1.0, b, r), s));
-    HBX_CUDA(hbx::bt_launch_dots(1, count, h->d_inst_off, r, r, nullptr, nullptr, dots, s));
+    HBX_CUDA(hbx::bt_launch_norms(count, cluster, h->d_inst_off, r, dots, s));
     HBX_CUDA(cudaMemcpyAsync(rr.data(), dots, count * sizeof(double), cudaMemcpyDeviceToHost, s));
     HBX_CUDA(cudaStreamSynchronize(s));
     launches += 2;
@@ -1927,17 +1956,16 @@ int hbx_bicgstab_batch_refined(hbx_hmat *h, hbx_hmat *hl, const double *b, doubl
 int hbx_bicgstab_batch_refined_host(hbx_hmat *h, hbx_hmat *hl, const double *b, double *u, const hbx_solve_opts *opts,
                                     hbx_solve_info *info) {
   if (!h || !hl || !b || !u) return fail(HBX_ERR_INVALID, "hbx_bicgstab_batch_refined_host: NULL argument");
-  const size_t bytes = (size_t)h->plan.nd * sizeof(double);
-  double *dv = nullptr;
-  HBX_CUDA(dev_malloc(&dv, 2 * bytes));
+  int st = ensure_solver(h, 0);
+  if (st != HBX_OK) return st;
+  const size_t n = (size_t)h->plan.nd, bytes = n * sizeof(double);
+  double *db = h->d_work + 6 * n, *du = h->d_work + 7 * n;
   cudaStream_t s = h->stream;
-  cudaError_t e = cudaMemcpyAsync(dv, b, bytes, cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(dv + h->plan.nd, u, bytes, cudaMemcpyHostToDevice, s);
-  if (e != cudaSuccess) { cudaFree(dv); return cuda_fail(e, "hbx_bicgstab_batch_refined_host upload"); }
-  int st = hbx_bicgstab_batch_refined(h, hl, dv, dv + h->plan.nd, opts, info, s);
-  e = cudaMemcpyAsync(u, dv + h->plan.nd, bytes, cudaMemcpyDeviceToHost, s);
+  HBX_CUDA(cudaMemcpyAsync(db, b, bytes, cudaMemcpyHostToDevice, s));
+  HBX_CUDA(cudaMemcpyAsync(du, u, bytes, cudaMemcpyHostToDevice, s));
+  st = hbx_bicgstab_batch_refined(h, hl, db, du, opts, info, s);
+  cudaError_t e = cudaMemcpyAsync(u, du, bytes, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  cudaFree(dv);
   if (e != cudaSuccess) return cuda_fail(e, "hbx_bicgstab_batch_refined_host download");
   return st;
 }
@@ -1945,17 +1973,16 @@ int hbx_bicgstab_batch_refined_host(hbx_hmat *h, hbx_hmat *hl, const double *b, 
 int hbx_bicgstab_batch_host(hbx_hmat *h, const double *b, double *u, const hbx_solve_opts *opts,
                             hbx_solve_info *info) {
   if (!h || !b || !u) return fail(HBX_ERR_INVALID, "hbx_bicgstab_batch_host: NULL argument");
-  const size_t bytes = (size_t)h->plan.nd * sizeof(double);
-  double *d = nullptr;
-  HBX_CUDA(dev_malloc(&d, 2 * bytes));
+  int st = ensure_solver(h, 0);
+  if (st != HBX_OK) return st;
+  const size_t n = (size_t)h->plan.nd, bytes = n * sizeof(double);
+  double *db = h->d_work + 6 * n, *du = h->d_work + 7 * n;
   cudaStream_t s = h->stream;
-  cudaError_t e = cudaMemcpyAsync(d, b, bytes, cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(d + h->plan.nd, u, bytes, cudaMemcpyHostToDevice, s);
-  if (e != cudaSuccess) { cudaFree(d); return cuda_fail(e, "hbx_bicgstab_batch_host upload"); }
-  int st = hbx_bicgstab_batch(h, d, d + h->plan.nd, opts, info, s);
-  e = cudaMemcpyAsync(u, d + h->plan.nd, bytes, cudaMemcpyDeviceToHost, s);
+  HBX_CUDA(cudaMemcpyAsync(db, b, bytes, cudaMemcpyHostToDevice, s));
+  HBX_CUDA(cudaMemcpyAsync(du, u, bytes, cudaMemcpyHostToDevice, s));
+  st = hbx_bicgstab_batch(h, db, du, opts, info, s);
+  cudaError_t e = cudaMemcpyAsync(u, du, bytes, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  cudaFree(d);
   if (e != cudaSuccess) return cuda_fail(e, "hbx_bicgstab_batch_host download");
   return st;
 }

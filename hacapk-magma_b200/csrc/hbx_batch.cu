@@ -7,10 +7,24 @@
 // HACApK_SOLVER.c:631 does.  A finished instance keeps u and r, and its p and
 // t are zero so its rows of the block-diagonal products are zero.
 //
-// Dot products: one block per instance sums its rows with compensated
-// (Dot2) accumulation, as the single-body solver does -- each thread in row
-// order, then a fixed tree over the block -- so every run sums in the same
-// order and the scalars match a body solved alone.
+// An instance's dots need its rows alone, so a cluster of CTAs takes an
+// instance and goes from the product to the next product's input in one
+// launch: k_bt_mid forms alpha and t, k_bt_end zeta, u, r, beta and p, the
+// float copy of t or p that an FP32 or BF16 product reads included.  Two
+// launches and two products a step; what bounds them is their chain of
+// reductions (one or two, through the cluster's shared memory), and the
+// cluster's size (1 to 8 CTAs by the largest instance) keeps a row or a few
+// per thread.  The step of 24 bodies of 320 to 5,120 rows took 17 launches
+// beside the products before (dots, scalars, updates, float copies, prefix
+// counts: 40 us, and the host could not launch them fast enough); these two
+// take 12.
+//
+// Dot products are compensated (Dot2), as the single-body solver's: each
+// thread in row order, a warp butterfly, the CTA's warps in order, the
+// cluster's CTAs in order, so every run sums in the same order.
+#include <cooperative_groups.h>
+
+#include <algorithm>
 #include <cmath>
 
 #include "../../include/hacapk_b200.h"
@@ -20,213 +34,257 @@
 namespace hbx {
 namespace {
 
-constexpr int kBt = 1024;  // threads of a per-body dot block
+namespace cg = cooperative_groups;
 
-// out[k][q] = x_q . y_q over the rows of instance k
+constexpr int kBt = 512;       // threads of a CTA
+constexpr int kBtRows = 4096;  // rows of the largest instance per 2x of cluster: about 4 to 8 a thread
+constexpr int kMaxCluster = 8;
+
+// The rows of the calling thread: its instance's, in turn over the cluster.
+struct Rows {
+  int k;        // instance
+  int i0, i1;   // first and end row of the instance
+  int first, step;
+};
+__device__ __forceinline__ Rows my_rows(const int *off, unsigned nrank, unsigned rank) {
+  Rows R;
+  R.k = blockIdx.x / nrank;
+  R.i0 = off[R.k];
+  R.i1 = off[R.k + 1];
+  R.first = R.i0 + (int)(rank * kBt + threadIdx.x);
+  R.step = (int)nrank * kBt;
+  return R;
+}
+
+// tot[q]: the sums of acc[q] over the cluster, the same in every thread.
+// `sh` is written again only after another cluster barrier.
 template <int NQ>
-__global__ void __launch_bounds__(kBt) k_bt_dots(const int *off, const double *x0, const double *y0, const double *x1,
-                                                 const double *y1, double *out) {
-  const int k = blockIdx.x, tid = threadIdx.x;
-  const int r0 = off[k], r1 = off[k + 1];
-  Acc2 acc[NQ];
+struct ClusterSums {
+  Acc2 warp[kBt / 32][NQ];
+  Acc2 cta[NQ];
+};
+template <int NQ>
+__device__ __forceinline__ void cluster_totals(cg::cluster_group &cl, const Acc2 (&acc)[NQ], ClusterSums<NQ> &sh,
+                                               double (&tot)[NQ]) {
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
-  for (int q = 0; q < NQ; ++q) acc[q] = Acc2{0.0, 0.0};
-  for (int i = r0 + tid; i < r1; i += kBt) {
-    dot2_add(acc[0], x0[i], y0[i]);
-    if (NQ > 1) dot2_add(acc[NQ - 1], x1[i], y1[i]);
+  for (int q = 0; q < NQ; ++q) {
+    const Acc2 m = warp_merge(acc[q]);
+    if (lane == 0) sh.warp[w][q] = m;
   }
-  __shared__ Acc2 red[NQ][kBt];
-#pragma unroll
-  for (int q = 0; q < NQ; ++q) red[q][tid] = acc[q];
   __syncthreads();
-  for (int w = kBt / 2; w > 0; w >>= 1) {
-    if (tid < w) {
+  if (threadIdx.x < NQ) {
+    Acc2 t = sh.warp[0][threadIdx.x];
+    for (int k = 1; k < kBt / 32; ++k) t = acc2_merge(t, sh.warp[k][threadIdx.x]);
+    sh.cta[threadIdx.x] = t;
+  }
+  cl.sync();
+  const unsigned n = cl.num_blocks();
 #pragma unroll
-      for (int q = 0; q < NQ; ++q) red[q][tid] = acc2_merge(red[q][tid], red[q][tid + w]);
-    }
-    __syncthreads();
-  }
-  if (tid < NQ) out[(size_t)k * NQ + tid] = red[tid][0].s + red[tid][0].c;
-}
-
-// Start of the solve: r = b - H u is formed; rh = r, p = Ap = 0 on every row.
-__global__ void k_bt_setup(size_t n, const double *r, double *rh, double *p, double *ap) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    rh[i] = r[i];
-    p[i] = 0.0;
-    ap[i] = 0.0;
+  for (int q = 0; q < NQ; ++q) {
+    Acc2 t = *cl.map_shared_rank(&sh.cta[q], 0);
+    for (unsigned c = 1; c < n; ++c) t = acc2_merge(t, *cl.map_shared_rank(&sh.cta[q], c));
+    tot[q] = t.s + t.c;
   }
 }
 
-// rho = rh.r = r.r, bnorm; an instance runs while ||r||/||b|| >= tol
-__global__ void k_bt_init(int count, const double *dots /*[k][2]: r.r, b.b*/, double tol, const double *rtol,
-                          int max_iter, MrScal *s, double *bnorm, int *any_active) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= count) return;
-  const double rr = dots[2 * k], bb = dots[2 * k + 1];
-  const double bn = std::sqrt(bb);
-  bnorm[k] = bn;
-  MrScal q{};
-  q.rho = rr;
-  q.rr = rr;
-  const double rel = bn > 0.0 ? std::sqrt(rr) / bn : 0.0;
-  if (rtol) tol = rtol[k];  // per-instance tolerance (the inner solves of a refined batch)
-  q.rtol = tol;
-  q.status = 0;
-  if (!isfinite(rel)) q.status = HBX_ERR_BREAKDOWN;
-  else if (rel >= tol) q.active = max_iter > 0 ? 1 : 0;
-  if (rel >= tol && max_iter <= 0) q.status = HBX_ERR_NOT_CONVERGED;
-  s[k] = q;
-  if (q.active) atomicOr(any_active, 1);
-}
-
-// p = r + beta (p - zeta Ap) (p = r on the first step); zero when finished
-__global__ void k_bt_p(size_t n, const int *rinst, const MrScal *s, const double *r, double *p, const double *ap) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const MrScal &q = s[rinst[i]];
-    if (!q.active) {
-      p[i] = 0.0;
-      continue;
-    }
-    p[i] = q.iters == 0 ? r[i] : fma(q.beta, fma(-q.zeta, ap[i], p[i]), r[i]);
+// The CTA that finishes last in the grid (one thread of each calls with its
+// results written) counts the active instances: pre[k] = those below k,
+// flags: any_active, done.
+__device__ __forceinline__ void count_active(int count, const MrScal *s, int *pre, BtFlags *f) {
+  __shared__ bool last;
+  __shared__ int part[kBt];
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    const unsigned t = atomicAdd(&f->ticket, 1u);
+    last = t == gridDim.x - 1;
+    if (last) f->ticket = 0;
   }
-}
-
-// alpha = rho / (rh . Ap)
-__global__ void k_bt_alpha(int count, const double *dots, MrScal *s) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= count || !s[k].active) return;
-  const double d = dots[k];
-  const double alpha = s[k].rho / d;
-  if (d == 0.0 || !isfinite(alpha)) {
-    s[k].active = 0;
-    s[k].status = HBX_ERR_BREAKDOWN;
-    return;
-  }
-  s[k].alpha = alpha;
-}
-
-// t = r - alpha Ap; zero when finished
-__global__ void k_bt_t(size_t n, const int *rinst, const MrScal *s, const double *r, const double *ap, double *t) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const MrScal &q = s[rinst[i]];
-    t[i] = q.active ? fma(-q.alpha, ap[i], r[i]) : 0.0;
-  }
-}
-
-// zeta = (At . t) / (At . At).  At . At == 0 means At = 0: zeta = 0 keeps
-// the step's BiCG half (u += alpha p, r = t); the stop test that follows
-// (k_bt_beta) then ends the instance as converged when that r is below the
-// tolerance and as a breakdown otherwise, before any further step.
-__global__ void k_bt_zeta(int count, const double *dots, MrScal *s) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= count || !s[k].active) return;
-  const double tt = dots[2 * k], aa = dots[2 * k + 1];
-  const double zeta = aa != 0.0 ? tt / aa : 0.0;
-  if (!isfinite(zeta)) {
-    s[k].active = 0;
-    s[k].status = HBX_ERR_BREAKDOWN;
-    return;
-  }
-  s[k].zeta = zeta;
-}
-
-// u += alpha p + zeta t;  r = t - zeta At  (running instances)
-__global__ void k_bt_xr(size_t n, const int *rinst, const MrScal *s, const double *p, const double *t,
-                        const double *at, double *u, double *r) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const MrScal &q = s[rinst[i]];
-    if (!q.active) continue;
-    const double tv = t[i];
-    u[i] = fma(q.zeta, tv, fma(q.alpha, p[i], u[i]));
-    r[i] = fma(-q.zeta, at[i], tv);
-  }
-}
-
-// the step is done: rho_new = rh . r, rr = r . r; the stop test; beta
-__global__ void k_bt_beta(int count, const double *dots, const double *bnorm, int max_iter, MrScal *s,
-                          int *any_active) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= count || !s[k].active) return;
-  MrScal q = s[k];
-  const double rho_new = dots[2 * k], rr = dots[2 * k + 1];
-  q.iters += 1;
-  q.rr = rr;
-  const double rel = bnorm[k] > 0.0 ? std::sqrt(rr) / bnorm[k] : 0.0;
-  if (!isfinite(rel)) {
-    q.active = 0;
-    q.status = HBX_ERR_BREAKDOWN;
-  } else if (rel < q.rtol) {
-    q.active = 0;
-  } else if (q.iters >= max_iter) {
-    q.active = 0;
-    q.status = HBX_ERR_NOT_CONVERGED;
-  } else {
-    const double beta = (q.alpha / q.zeta) * (rho_new / q.rho);
-    if (q.zeta == 0.0 || !isfinite(beta)) {
-      q.active = 0;
-      q.status = HBX_ERR_BREAKDOWN;
-    } else {
-      q.beta = beta;
-      q.rho = rho_new;
-    }
-  }
-  s[k] = q;
-  if (q.active) atomicOr(any_active, 1);
-}
-
-int vgrid(size_t n) { return (int)std::min<size_t>((n + 255) / 256, 148 * 8); }
-
-// pre[k] = active instances below k (count + 1 entries), one block: each
-// thread counts a contiguous share, a block scan of the shares, then each
-// thread writes its share's prefixes.
-constexpr int kPreThreads = 1024;
-__global__ void __launch_bounds__(kPreThreads) k_bt_prefix(int count, const MrScal *s, int *pre) {
-  __shared__ int part[kPreThreads];
-  const int t = threadIdx.x, per = (count + kPreThreads - 1) / kPreThreads;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const int t = threadIdx.x, per = (count + kBt - 1) / kBt;
   const int k0 = min(count, t * per), k1 = min(count, k0 + per);
   int c = 0;
-  for (int k = k0; k < k1; ++k) c += s[k].active ? 1 : 0;
+  for (int k = k0; k < k1; ++k) c += __ldcg(&s[k].active) ? 1 : 0;
   part[t] = c;
   __syncthreads();
-  for (int o = 1; o < kPreThreads; o <<= 1) {
+  for (int o = 1; o < kBt; o <<= 1) {
     const int v = t >= o ? part[t - o] : 0;
     __syncthreads();
     part[t] += v;
     __syncthreads();
   }
-  int run = part[t] - c;  // active instances below k0
-  for (int k = k0; k < k1; ++k) {
-    pre[k] = run;
-    run += s[k].active ? 1 : 0;
+  if (pre) {
+    int run = part[t] - c;  // active instances below k0
+    for (int k = k0; k < k1; ++k) {
+      pre[k] = run;
+      run += __ldcg(&s[k].active) ? 1 : 0;
+    }
+    if (t == kBt - 1) pre[count] = part[t];
   }
-  if (t == kPreThreads - 1) pre[count] = part[t];
+  if (t == kBt - 1) {
+    f->any = part[t] > 0;
+    f->done = part[t] == 0;
+  }
 }
 
-}  // namespace
-
-cudaError_t bt_launch_prefix(int count, const MrScal *sc, int *pre, cudaStream_t s) {
-  k_bt_prefix<<<1, kPreThreads, 0, s>>>(count, sc, pre);
-  return cudaGetLastError();
+// out[k] = x . x over the rows of instance k
+__global__ void __launch_bounds__(kBt) k_bt_norms(const int *off, const double *x, double *out) {
+  cg::cluster_group cl = cg::this_cluster();
+  __shared__ ClusterSums<1> sh;
+  const Rows R = my_rows(off, cl.num_blocks(), cl.block_rank());
+  Acc2 acc[1] = {{0.0, 0.0}};
+  for (int i = R.first; i < R.i1; i += R.step) dot2_add(acc[0], x[i], x[i]);
+  double tot[1];
+  cluster_totals<1>(cl, acc, sh, tot);
+  if (cl.block_rank() == 0 && threadIdx.x == 0) out[R.k] = tot[0];
+  cl.sync();  // every CTA has read the others' sums
 }
 
-cudaError_t bt_launch_dots(int nq, int count, const int *off, const double *x0, const double *y0, const double *x1,
-                           const double *y1, double *out, cudaStream_t s) {
-  if (nq == 1) k_bt_dots<1><<<count, kBt, 0, s>>>(off, x0, y0, nullptr, nullptr, out);
-  else k_bt_dots<2><<<count, kBt, 0, s>>>(off, x0, y0, x1, y1, out);
-  return cudaGetLastError();
+// Start of the solve, r = b - H u formed: rh = r, p = r, the stop test; an
+// instance runs while ||r||/||b|| >= tol (rtol: per instance).
+__global__ void __launch_bounds__(kBt) k_bt_init(BtStep a, const double *b, double tol, const double *rtol) {
+  cg::cluster_group cl = cg::this_cluster();
+  __shared__ ClusterSums<2> sh;
+  const Rows R = my_rows(a.off, cl.num_blocks(), cl.block_rank());
+  Acc2 acc[2] = {{0.0, 0.0}, {0.0, 0.0}};
+  for (int i = R.first; i < R.i1; i += R.step) {
+    const double rv = a.r[i], bv = b[i];
+    a.rh[i] = rv;
+    dot2_add(acc[0], rv, rv);
+    dot2_add(acc[1], bv, bv);
+  }
+  double tot[2];
+  cluster_totals<2>(cl, acc, sh, tot);
+  const double rr = tot[0], bn = std::sqrt(tot[1]);
+  MrScal q{};
+  q.rho = rr;
+  q.rr = rr;
+  const double rel = bn > 0.0 ? std::sqrt(rr) / bn : 0.0;
+  if (rtol) tol = rtol[R.k];  // per-instance tolerance (the inner solves of a refined batch)
+  q.rtol = tol;
+  q.status = 0;
+  if (!isfinite(rel)) q.status = HBX_ERR_BREAKDOWN;
+  else if (rel >= tol) q.active = a.max_iter > 0 ? 1 : 0;
+  if (rel >= tol && a.max_iter <= 0) q.status = HBX_ERR_NOT_CONVERGED;
+  for (int i = R.first; i < R.i1; i += R.step) {
+    const double pv = q.active ? a.r[i] : 0.0;
+    a.p[i] = pv;
+    if (a.x32) a.x32[i] = (float)pv;
+    if (!q.active) a.t[i] = 0.0;
+  }
+  if (cl.block_rank() == 0 && threadIdx.x == 0) {
+    a.bnorm[R.k] = bn;
+    a.sc[R.k] = q;
+  }
+  cl.sync();
+  count_active(a.count, a.sc, a.pre, a.flags);
 }
 
-cudaError_t bt_launch_setup(size_t n, const double *r, double *rh, double *p, double *ap, cudaStream_t s) {
-  k_bt_setup<<<vgrid(n), 256, 0, s>>>(n, r, rh, p, ap);
-  return cudaGetLastError();
+// After Ap: alpha = rho / (rh . Ap), t = r - alpha Ap
+__global__ void __launch_bounds__(kBt) k_bt_mid(BtStep a) {
+  cg::cluster_group cl = cg::this_cluster();
+  __shared__ ClusterSums<1> sh;
+  if (*(volatile const int *)&a.flags->done) return;
+  const Rows R = my_rows(a.off, cl.num_blocks(), cl.block_rank());
+  MrScal &S = a.sc[R.k];
+  if (!S.active) return;  // the same in the whole cluster
+  const double rho = S.rho;
+  Acc2 acc[1] = {{0.0, 0.0}};
+  for (int i = R.first; i < R.i1; i += R.step) dot2_add(acc[0], a.rh[i], a.ap[i]);
+  double tot[1];
+  cluster_totals<1>(cl, acc, sh, tot);
+  const double alpha = rho / tot[0];
+  const bool bad = tot[0] == 0.0 || !isfinite(alpha);
+  for (int i = R.first; i < R.i1; i += R.step) {
+    const double tv = bad ? 0.0 : fma(-alpha, a.ap[i], a.r[i]);
+    a.t[i] = tv;
+    if (a.x32) a.x32[i] = (float)tv;
+    if (bad) a.p[i] = 0.0;
+  }
+  cl.sync();  // the others' sums and S are read
+  if (cl.block_rank() == 0 && threadIdx.x == 0) {
+    if (bad) {
+      S.active = 0;
+      S.status = HBX_ERR_BREAKDOWN;
+    } else {
+      S.alpha = alpha;
+    }
+  }
 }
 
-cudaError_t bt_launch_init(int count, const double *dots, double tol, const double *rtol, int max_iter, MrScal *sc,
-                           double *bnorm, int *any_active, cudaStream_t s) {
-  cudaMemsetAsync(any_active, 0, sizeof(int), s);
-  k_bt_init<<<(count + 127) / 128, 128, 0, s>>>(count, dots, tol, rtol, max_iter, sc, bnorm, any_active);
-  return cudaGetLastError();
+// After At: zeta = (At . t) / (At . At), u += alpha p + zeta t, r = t - zeta
+// At, rho_new = rh . r, rr = r . r; the stop test; p = r + beta (p - zeta Ap).
+// At . At == 0 means At = 0: zeta = 0 keeps the step's BiCG half (u += alpha p,
+// r = t); the stop test then ends the instance as converged when that r is
+// below the tolerance and as a breakdown otherwise, before any further step.
+__global__ void __launch_bounds__(kBt) k_bt_end(BtStep a) {
+  cg::cluster_group cl = cg::this_cluster();
+  __shared__ ClusterSums<2> sh, sh2;
+  if (*(volatile const int *)&a.flags->done) return;
+  const Rows R = my_rows(a.off, cl.num_blocks(), cl.block_rank());
+  MrScal q = a.sc[R.k];
+  if (q.active) {
+    Acc2 acc[2] = {{0.0, 0.0}, {0.0, 0.0}};
+    for (int i = R.first; i < R.i1; i += R.step) {
+      const double av = a.at[i];
+      dot2_add(acc[0], av, a.t[i]);
+      dot2_add(acc[1], av, av);
+    }
+    double tot[2];
+    cluster_totals<2>(cl, acc, sh, tot);
+    const double zeta = tot[1] != 0.0 ? tot[0] / tot[1] : 0.0;
+    bool run = isfinite(zeta);
+    if (!run) {
+      q.status = HBX_ERR_BREAKDOWN;  // u and r of the previous step stay
+    } else {
+      q.zeta = zeta;
+      acc[0] = acc[1] = Acc2{0.0, 0.0};
+      for (int i = R.first; i < R.i1; i += R.step) {
+        const double tv = a.t[i];
+        a.u[i] = fma(zeta, tv, fma(q.alpha, a.p[i], a.u[i]));
+        const double rv = fma(-zeta, a.at[i], tv);
+        a.r[i] = rv;
+        dot2_add(acc[0], a.rh[i], rv);
+        dot2_add(acc[1], rv, rv);
+      }
+      cluster_totals<2>(cl, acc, sh2, tot);
+      const double rho_new = tot[0], rr = tot[1], bn = a.bnorm[R.k];
+      q.iters += 1;
+      q.rr = rr;
+      const double rel = bn > 0.0 ? std::sqrt(rr) / bn : 0.0;
+      if (!isfinite(rel)) {
+        run = false;
+        q.status = HBX_ERR_BREAKDOWN;
+      } else if (rel < q.rtol) {
+        run = false;
+      } else if (q.iters >= a.max_iter) {
+        run = false;
+        q.status = HBX_ERR_NOT_CONVERGED;
+      } else {
+        const double beta = (q.alpha / q.zeta) * (rho_new / q.rho);
+        if (q.zeta == 0.0 || !isfinite(beta)) {
+          run = false;
+          q.status = HBX_ERR_BREAKDOWN;
+        } else {
+          q.beta = beta;
+          q.rho = rho_new;
+        }
+      }
+    }
+    q.active = run ? 1 : 0;
+    for (int i = R.first; i < R.i1; i += R.step) {
+      const double pv = run ? fma(q.beta, fma(-q.zeta, a.ap[i], a.p[i]), a.r[i]) : 0.0;
+      a.p[i] = pv;
+      if (a.x32) a.x32[i] = (float)pv;
+      if (!run) a.t[i] = 0.0;
+    }
+    cl.sync();  // the others' sums and scalars are read
+    if (cl.block_rank() == 0 && threadIdx.x == 0) a.sc[R.k] = q;
+  }
+  count_active(a.count, a.sc, a.pre, a.flags);
 }
 
 // r[i] = 0 for the rows of instances whose flag is 0
@@ -235,29 +293,49 @@ __global__ void k_bt_mask(size_t n, const int *rinst, const int *flag, double *r
     if (!flag[rinst[i]]) r[i] = 0.0;
 }
 
+template <class... P, class... A>
+cudaError_t launch_clusters(void (*kern)(P...), int count, int cluster, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(count * cluster));
+  cfg.blockDim = dim3(kBt);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)cluster;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+
+}  // namespace
+
+int bt_cluster(int max_rows) {
+  int c = 1;
+  while (c < kMaxCluster && max_rows > c * kBtRows / 2) c *= 2;
+  return c;
+}
+
+cudaError_t bt_launch_norms(int count, int cluster, const int *off, const double *x, double *out, cudaStream_t s) {
+  return launch_clusters(k_bt_norms, count, cluster, s, off, x, out);
+}
+
+cudaError_t bt_launch_init(const BtStep &a, const double *b, double tol, const double *rtol, cudaStream_t s) {
+  return launch_clusters(k_bt_init, a.count, a.cluster, s, a, b, tol, rtol);
+}
+
 cudaError_t bt_launch_mask(size_t n, const int *rinst, const int *flag, double *r, cudaStream_t s) {
-  k_bt_mask<<<vgrid(n), 256, 0, s>>>(n, rinst, flag, r);
+  k_bt_mask<<<(int)std::min<size_t>((n + 255) / 256, 148 * 8), 256, 0, s>>>(n, rinst, flag, r);
   return cudaGetLastError();
 }
 
 cudaError_t bt_launch_step(const BtStep &a, cudaStream_t s) {
-  const int sg = (a.count + 127) / 128;
   cudaError_t e;
-  k_bt_p<<<vgrid(a.n), 256, 0, s>>>(a.n, a.rinst, a.sc, a.r, a.p, a.ap);
-  if (a.pre) k_bt_prefix<<<1, kPreThreads, 0, s>>>(a.count, a.sc, a.pre);
   if ((e = a.matvec(a.ctx, a.p, a.ap, s)) != cudaSuccess) return e;
-  k_bt_dots<1><<<a.count, kBt, 0, s>>>(a.off, a.rh, a.ap, nullptr, nullptr, a.dots);
-  k_bt_alpha<<<sg, 128, 0, s>>>(a.count, a.dots, a.sc);
-  k_bt_t<<<vgrid(a.n), 256, 0, s>>>(a.n, a.rinst, a.sc, a.r, a.ap, a.t);
-  if (a.pre) k_bt_prefix<<<1, kPreThreads, 0, s>>>(a.count, a.sc, a.pre);
+  if ((e = launch_clusters(k_bt_mid, a.count, a.cluster, s, a)) != cudaSuccess) return e;
   if ((e = a.matvec(a.ctx, a.t, a.at, s)) != cudaSuccess) return e;
-  k_bt_dots<2><<<a.count, kBt, 0, s>>>(a.off, a.at, a.t, a.at, a.at, a.dots);
-  k_bt_zeta<<<sg, 128, 0, s>>>(a.count, a.dots, a.sc);
-  k_bt_xr<<<vgrid(a.n), 256, 0, s>>>(a.n, a.rinst, a.sc, a.p, a.t, a.at, a.u, a.r);
-  k_bt_dots<2><<<a.count, kBt, 0, s>>>(a.off, a.rh, a.r, a.r, a.r, a.dots);
-  cudaMemsetAsync(a.any_active, 0, sizeof(int), s);
-  k_bt_beta<<<sg, 128, 0, s>>>(a.count, a.dots, a.bnorm, a.max_iter, a.sc, a.any_active);
-  return cudaGetLastError();
+  return launch_clusters(k_bt_end, a.count, a.cluster, s, a);
 }
 
 }  // namespace hbx

@@ -159,25 +159,26 @@ cudaError_t mr_launch_add(int nd, const int *mask, const double *D, double *U, c
 
 // Batched BiCGSTAB over the instances of a block-diagonal engine
 // (hbx_batch.cu); one MrScal per instance, rtol = the relative tolerance.
+struct BtFlags {
+  int any, done;    // some instance runs; none does (MatvecArgs::skip)
+  unsigned ticket;  // last-block counter, zero between launches
+};
 struct BtStep {
-  size_t n;
-  int count, max_iter;
-  int *pre;  // optional: prefix counts of active instances, refreshed before each product
-  const int *off, *rinst;  // instance row offsets [count + 1], instance of every row
+  int count, max_iter, cluster;  // cluster: CTAs per instance (bt_cluster)
+  const int *off;                // instance row offsets [count + 1]
   MrScal *sc;
-  int *any_active;
-  double *r, *rh, *p, *ap, *t, *at, *u, *dots, *bnorm;
+  BtFlags *flags;
+  int *pre;    // optional: prefix counts of active instances, refreshed by every step
+  float *x32;  // FP32 / BF16 engines: the products' input as float (p, then t)
+  double *r, *rh, *p, *ap, *t, *at, *u, *bnorm;
   cudaError_t (*matvec)(void *ctx, const double *x, double *y, cudaStream_t s);
   void *ctx;
 };
-cudaError_t bt_launch_dots(int nq, int count, const int *off, const double *x0, const double *y0, const double *x1,
-                           const double *y1, double *out, cudaStream_t s);
-cudaError_t bt_launch_setup(size_t n, const double *r, double *rh, double *p, double *ap, cudaStream_t s);
-cudaError_t bt_launch_init(int count, const double *dots, double tol, const double *rtol, int max_iter, MrScal *sc,
-                           double *bnorm, int *any_active, cudaStream_t s);
+int bt_cluster(int max_rows);
+cudaError_t bt_launch_norms(int count, int cluster, const int *off, const double *x, double *out, cudaStream_t s);
+cudaError_t bt_launch_init(const BtStep &a, const double *b, double tol, const double *rtol, cudaStream_t s);
 cudaError_t bt_launch_mask(size_t n, const int *rinst, const int *flag, double *r, cudaStream_t s);
 cudaError_t bt_launch_step(const BtStep &a, cudaStream_t s);
-cudaError_t bt_launch_prefix(int count, const MrScal *sc, int *pre, cudaStream_t s);
 
 // Dot products of up to kMaxDots vector pairs per launch (hbx_gcr.cu;
 // compensated per-block partials part[blocks][kMaxDots][2], summed in block
@@ -291,8 +292,9 @@ struct hbx_hmat {
   void *d_rflag = nullptr;  // refined batch: per-instance flags and inner tolerances
   double *d_btv = nullptr;      // r, rh, p, ap, t, at (6 nd)
   hbx::MrScal *d_btsc = nullptr;
-  double *d_btdbl = nullptr;    // dots [count][2], bnorm [count], true norms [count]
-  int *d_btany = nullptr;
+  double *d_btdbl = nullptr;    // bnorm [count], true norms [count], norms of the outer loop [count]
+  hbx::BtFlags *d_btflags = nullptr;
+  int *h_btany = nullptr;       // page-locked: any_active after the last two batches of steps
   hbx::Plan plan;
   uint8_t *d_stream = nullptr;
   hbx::RunRec *d_recs = nullptr;
