@@ -270,7 +270,7 @@ def run_ours(args, world, rank, local):
         "e2e": {"value": e2e_s, "unit": "s", "h2d_bytes_per_step": 16 * n, "d2h_bytes_per_step": 8 * n},
         "hmatvec": {"us": mv_us, "gbs": mv_gbs, "frac_of_" + peak_kind + "_peak": mv_gbs / peak},
         "roofline": {
-            "kernel": "k_bicg_iter (one BiCGSTAB step: 2 H-matvecs + vector updates + dots)",
+            "kernel": "k_bicg_steps (per BiCGSTAB step: 2 H-matvecs + vector updates + dots)",
             "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": achieved / peak, "peak_kind": peak_kind,
             "traffic": ncu_traffic("k_bicg_iter"),

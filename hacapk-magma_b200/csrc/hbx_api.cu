@@ -62,7 +62,6 @@ void free_engine(hbx_hmat *h) {
   int cur = -1;
   cudaGetDevice(&cur);
   if (cur != h->device) cudaSetDevice(h->device);
-  if (h->graph) cudaGraphExecDestroy(h->graph);
   cudaFree(h->d_stream);
   cudaFree(h->d_recs);
   cudaFree(h->d_ctas);
@@ -116,12 +115,13 @@ void free_engine(hbx_hmat *h) {
   cudaFree(h->d_btflags);
   if (h->h_btany) cudaFreeHost(h->h_btany);
   if (h->h_pin) cudaFreeHost(h->h_pin);
-  if (h->h_state) cudaFreeHost(h->h_state);
+  if (h->h_back) cudaFreeHost(h->h_back);
   if (h->ev0) cudaEventDestroy(h->ev0);
   if (h->ev1) cudaEventDestroy(h->ev1);
   if (h->ev2) cudaEventDestroy(h->ev2);
   if (h->ev3) cudaEventDestroy(h->ev3);
   if (h->ev4) cudaEventDestroy(h->ev4);
+  if (h->ev5) cudaEventDestroy(h->ev5);
   if (h->stream) cudaStreamDestroy(h->stream);
   if (cur >= 0 && cur != h->device) cudaSetDevice(cur);
   delete h;
@@ -198,7 +198,7 @@ int ensure_solver(hbx_hmat *h, int max_iter) {
   if (!h->d_part) HBX_CUDA(dev_malloc(&h->d_part, (size_t)h->num_ctas * hbx::kSlots * 2 * sizeof(double)));
   if (!h->d_dot) HBX_CUDA(dev_malloc(&h->d_dot, 4 * sizeof(double)));
   if (!h->d_state) HBX_CUDA(dev_malloc(&h->d_state, sizeof(hbx::BicgState)));
-  if (!h->h_state) HBX_CUDA(cudaHostAlloc(&h->h_state, sizeof(hbx::BicgState), cudaHostAllocDefault));
+  if (!h->h_back) HBX_CUDA(cudaHostAlloc(&h->h_back, sizeof(hbx::SolveBack), cudaHostAllocDefault));
   if (h->hist_cap < max_iter + 1) {
     cudaFree(h->d_hist);
     h->d_hist = nullptr;
@@ -384,6 +384,7 @@ static int create_engine(const stc_HACApK_leafmtxp *st, int nd, const hbx_option
   cudaEventCreate(&h->ev2);
   cudaEventCreate(&h->ev3);
   cudaEventCreate(&h->ev4);
+  cudaEventCreate(&h->ev5);
   if ((e = dev_malloc(&h->d_stream, P.total_bytes)) != cudaSuccess) return bail(cuda_fail(e, "cudaMalloc(stream)"));
   if ((e = dev_malloc(&h->d_recs, std::max<size_t>(1, P.recs.size()) * sizeof(hbx::RunRec))) != cudaSuccess)
     return bail(cuda_fail(e, "cudaMalloc(run records)"));
@@ -753,38 +754,6 @@ static hbx::BicgArgs bicg_args(hbx_hmat *h, const double *b, double *u, double t
   return a;
 }
 
-// Captures `batch` iteration launches into one graph (re-captured when the
-// vectors or the stopping parameters change).
-static int get_graph(hbx_hmat *h, const hbx::BicgArgs &a, int batch) {
-  const void *key[4] = {a.b, a.u, (const void *)(uintptr_t)a.max_iter, nullptr};
-  double tolkey = a.tol;
-  std::memcpy(&key[3], &tolkey, sizeof(double));
-  if (h->graph && h->graph_batch == batch && std::memcmp(key, h->graph_key, sizeof(key)) == 0) return HBX_OK;
-  if (h->graph) {
-    cudaGraphExecDestroy(h->graph);
-    h->graph = nullptr;
-  }
-  cudaGraph_t g = nullptr;
-  cudaStream_t s = h->stream;
-  if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return HBX_ERR_CUDA;
-  for (int i = 0; i < batch; ++i) hbx::launch_bicg_iter(a, h->num_ctas, s, h->plan.precision);
-  cudaError_t e = cudaStreamEndCapture(s, &g);
-  if (e != cudaSuccess || !g) {
-    cudaGetLastError();
-    return HBX_ERR_CUDA;
-  }
-  e = cudaGraphInstantiate(&h->graph, g, 0);
-  cudaGraphDestroy(g);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    h->graph = nullptr;
-    return HBX_ERR_CUDA;
-  }
-  h->graph_batch = batch;
-  std::memcpy(h->graph_key, key, sizeof(key));
-  return HBX_OK;
-}
-
 // BiCGSTAB on device vectors b, u (u: x0 in / solution out), all on h->stream.
 static int bicgstab_dev(hbx_hmat *h, const double *b, double *u, const hbx_solve_opts *opts, hbx_solve_info *info) {
   if (int rc = single_rhs(h, "hbx_bicgstab")) return rc;
@@ -796,42 +765,41 @@ static int bicgstab_dev(hbx_hmat *h, const double *b, double *u, const hbx_solve
   int st = ensure_solver(h, max_iter);
   if (st != HBX_OK) return st;
   cudaStream_t s = h->stream;
-  const hbx::BicgArgs a = bicg_args(h, b, u, tol, max_iter);
+  hbx::BicgArgs a = bicg_args(h, b, u, tol, max_iter);
+  a.steps = batch;
   HBX_CUDA(cudaEventRecord(h->ev0, s));
   // r = b - H u  (HACApK_SOLVER.c:562-573)
   HBX_CUDA(mv_launch(h, matvec_args(h, -1.0, u, 1.0, b, a.r), s));
   HBX_CUDA(hbx::launch_bicg_setup(a, h->num_ctas, s));
-  const bool use_graph = get_graph(h, a, batch) == HBX_OK;
-  int launched = 0;
-  double iter_s = 0.0;
+  HBX_CUDA(cudaEventRecord(h->ev5, s));
+  // One launch runs up to `batch` steps; the next is queued while the state
+  // after it is read, and returns at once when the solve has ended.
+  hbx::SolveBack *back = h->h_back;
+  cudaEvent_t read[2] = {h->ev3, h->ev4};
+  int launched = 0, seen = -1;
   for (;;) {
-    HBX_CUDA(cudaEventRecord(h->ev3, s));
-    if (use_graph) {
-      HBX_CUDA(cudaGraphLaunch(h->graph, s));
-    } else {
-      for (int i = 0; i < batch; ++i) HBX_CUDA(hbx::launch_bicg_iter(a, h->num_ctas, s, h->plan.precision));
-    }
-    HBX_CUDA(cudaEventRecord(h->ev4, s));
-    launched += batch;
-    HBX_CUDA(cudaMemcpyAsync(h->h_state, h->d_state, sizeof(hbx::BicgState), cudaMemcpyDeviceToHost, s));
-    HBX_CUDA(cudaStreamSynchronize(s));
-    float bms = 0.f;
-    cudaEventElapsedTime(&bms, h->ev3, h->ev4);
-    iter_s += bms * 1e-3;
-    if (h->h_state->done || launched > max_iter + batch) break;
-    int derr = 0;
-    HBX_CUDA(cudaMemcpy(&derr, h->d_err, sizeof(int), cudaMemcpyDeviceToHost));
-    if (derr) break;
+    const int k = launched & 1;
+    HBX_CUDA(hbx::launch_bicg_steps(a, h->num_ctas, s, h->plan.precision));
+    HBX_CUDA(cudaMemcpyAsync(&back->state[k], h->d_state, sizeof(hbx::BicgState), cudaMemcpyDeviceToHost, s));
+    HBX_CUDA(cudaEventRecord(read[k], s));
+    if (launched++ == 0) continue;
+    seen = k ^ 1;
+    HBX_CUDA(cudaEventSynchronize(read[seen]));
+    if (back->state[seen].done || (long long)(launched - 2) * batch > max_iter) break;
   }
+  float its = 0.f;
+  cudaEventElapsedTime(&its, h->ev5, read[seen]);
+  const double iter_s = its * 1e-3;
+  const hbx::BicgState S = back->state[seen];
   HBX_CUDA(cudaEventRecord(h->ev1, s));
-  const hbx::BicgState S = *h->h_state;
   // true residual ||b - H u|| (HACApK_SOLVER.c:737-746)
   HBX_CUDA(mv_launch(h, matvec_args(h, -1.0, u, 1.0, b, a.t), s));
   HBX_CUDA(hbx::launch_dot(a, a.t, a.t, hbx::kSlotAux, h->d_dot, h->num_ctas, s));
-  double tr2 = 0.0;
-  HBX_CUDA(cudaMemcpyAsync(&tr2, h->d_dot, sizeof(double), cudaMemcpyDeviceToHost, s));
+  HBX_CUDA(cudaMemcpyAsync(&back->dot, h->d_dot, sizeof(double), cudaMemcpyDeviceToHost, s));
+  HBX_CUDA(cudaMemcpyAsync(&back->err, h->d_err, sizeof(int), cudaMemcpyDeviceToHost, s));
   HBX_CUDA(cudaStreamSynchronize(s));
-  int dst = check_device_error(h, s);
+  const double tr2 = back->dot;
+  const int dst = back->err ? check_device_error(h, s) : HBX_OK;
   float ms = 0.f;
   cudaEventElapsedTime(&ms, h->ev0, h->ev1);
   if (info) {
@@ -843,8 +811,8 @@ static int bicgstab_dev(hbx_hmat *h, const double *b, double *u, const hbx_solve
     info->true_relres = S.bnorm > 0 ? std::sqrt(tr2) / S.bnorm : std::sqrt(tr2);
     info->seconds = ms * 1e-3;
     info->iter_kernel_seconds = iter_s;
-    info->iter_launches = launched;
-    info->launches = launched + 5;  // r0 matvec, setup, residual matvec, two dot kernels
+    info->iter_launches = S.iter + 1;  // steps, with the one that observes the end
+    info->launches = launched + 5;     // r0 matvec, setup, residual matvec, two dot kernels
   }
   if (verbose > 0) {
     std::vector<double> hist(S.iter + 1, 0.0);

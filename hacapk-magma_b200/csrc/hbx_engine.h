@@ -24,11 +24,19 @@ enum : int {
   kSlots = 8
 };
 
-// Solver scalars carried from one iteration launch to the next.
+// Solver scalars carried from one launch to the next.
 struct BicgState {
   double alpha, zeta, rho, beta;
   double relres, bnorm;
-  int iter, done, status, breakdown;
+  int iter, done, status, pad;
+};
+
+// What a solve reads back, in page-locked memory: the state after its last two
+// launches, the true residual's square, the device error word.
+struct SolveBack {
+  BicgState state[2];
+  double dot;
+  int err, pad;
 };
 
 struct MatvecArgs {
@@ -75,12 +83,13 @@ struct BicgArgs {
   const double *b;
   double *u, *r, *rh, *p, *ap, *t, *at;
   float *p32, *t32, *zbu32;  // FP32 engines: float copies of the matvec inputs (zbu32: [2][zbu_len])
-  double *part;   // [num_ctas][kSlots][2]
+  double *part;   // [kSlots][num_ctas][2]
   BicgState *state;
   double *hist;   // relres per iteration (max_iter + 1 entries)
   unsigned long long *prof;  // optional: per-CTA %globaltimer stamps [num_ctas][16], slots 8-15
   double tol;
   int max_iter;
+  int steps;           // steps of one launch, at most
   uint32_t keep_frac;  // as MatvecArgs::keep_frac
 };
 
@@ -244,13 +253,13 @@ size_t kernel_smem_bytes();
 cudaError_t configure_kernels();
 cudaError_t configure_step_kernels();     // the step kernels' translation unit
 cudaError_t configure_step_kernels_lp();  // the FP32 / BF16 step kernels' unit
-cudaError_t launch_bicg_iter_lp(const BicgArgs &a, int num_ctas, cudaStream_t s, int precision);
+cudaError_t launch_bicg_steps_lp(const BicgArgs &a, int num_ctas, cudaStream_t s, int precision);
 cudaError_t launch_matvec(const MatvecArgs &a, int num_ctas, cudaStream_t s, int precision);
 cudaError_t launch_bicg_setup(const BicgArgs &a, int num_ctas, cudaStream_t s);
-cudaError_t launch_bicg_iter(const BicgArgs &a, int num_ctas, cudaStream_t s, int precision);
-// part[.][slot] = sum over own rows of x.y; then out[0] = the total (one block).
+cudaError_t launch_bicg_steps(const BicgArgs &a, int num_ctas, cudaStream_t s, int precision);
 cudaError_t launch_axpy(double alpha, const double *x, double *y, size_t n, cudaStream_t s);
 cudaError_t launch_to_float(const double *x, float *y, size_t n, cudaStream_t s);
+// The slot's partials of x.y over own rows; then out[0] = the total (one block).
 cudaError_t launch_dot(const BicgArgs &a, const double *x, const double *y, int slot, double *out,
                        int num_ctas, cudaStream_t s);
 
@@ -311,7 +320,7 @@ struct hbx_hmat {
   unsigned long long *d_prof = nullptr;  // phase stamps of the last matvec (HBX_PROFILE=1)
   double setup_seconds = 0.0;
   cudaStream_t stream = nullptr;  // used by the host-vector calls
-  cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr, ev3 = nullptr, ev4 = nullptr;
+  cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr, ev3 = nullptr, ev4 = nullptr, ev5 = nullptr;
   // host-vector staging
   double *d_x = nullptr, *d_y = nullptr;
   double *h_pin = nullptr;        // pinned staging, 2*nd doubles
@@ -320,7 +329,7 @@ struct hbx_hmat {
   double *d_part = nullptr;
   double *d_dot = nullptr;
   hbx::BicgState *d_state = nullptr;
-  hbx::BicgState *h_state = nullptr;  // pinned
+  hbx::SolveBack *h_back = nullptr;  // page-locked: what a solve reads back
   double *d_hist = nullptr;
   double *d_refine = nullptr;     // mixed-precision solve: outer residual and correction (2*nd)
   float *d_f32 = nullptr;         // FP32 engines: x, p, t (3*nd) and zbu (zbu_len) rounded to float
@@ -343,8 +352,4 @@ struct hbx_hmat {
   cudaGraphExec_t pgraph = nullptr;
   int pgraph_batch = 0;
   const void *pgraph_key = nullptr;
-  // captured iteration batch
-  cudaGraphExec_t graph = nullptr;
-  int graph_batch = 0;
-  const void *graph_key[4] = {nullptr, nullptr, nullptr, nullptr};
 };

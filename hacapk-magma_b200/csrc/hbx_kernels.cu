@@ -5,18 +5,19 @@
 //               phase, no atomics, no zeroing of zbu/zau).
 // k_bicg_setup  r = b - H u has been formed by k_matvec; sets rh = r, p = Ap = 0
 //               and the first reduction partials (HACApK_SOLVER.c:533-594).
-// k_bicg_iter   one BiCGSTAB step of HACApK_SOLVER.c:602-732 in one launch:
-//               both H-matvecs, the vector updates and all dot products, with
-//               compensated (Dot2) partial sums reduced in a fixed order.
+// k_bicg_steps  BiCGSTAB steps of HACApK_SOLVER.c:602-732, several in one
+//               launch: both H-matvecs, the vector updates and all dot
+//               products, with compensated (Dot2) partial sums reduced in a
+//               fixed order.
 //
 // The file is compiled three times: as itself (k_matvec and the small vector
 // kernels, 16 consumer warps), with HBX_STEP_TU and HBX_CONSUMER_WARPS=13
-// (k_bicg_setup, the FP64 k_bicg_iter and the dot kernels): with fewer
+// (k_bicg_setup, the FP64 k_bicg_steps and the dot kernels): with fewer
 // threads per CTA the step kernel gets the registers it needs without
 // spilling, and its scalar phases synchronise fewer warps (C1 step 121.4 ->
 // 115 us, while the standalone product is fastest with 16); and with
 // HBX_STEP_TU, HBX_STEP_LP and HBX_CONSUMER_WARPS=kStepWarpsLp (the FP32 and
-// BF16 k_bicg_iter, whose consumer warps form two groups like the FP32 and
+// BF16 k_bicg_steps, whose consumer warps form two groups like the FP32 and
 // BF16 products').
 //
 // All kernels run one CTA per SM: consumer warps, a bulk-copy producer
@@ -110,6 +111,7 @@ __device__ __forceinline__ void init_cta_part(const Smem &s, const RunLite *lite
     s.rsum[1] = grid_gen0(gbar);
     s.rsum[2] = 0;
     s.rsum[3] = 0;
+    s.rsum[4] = 0;
     mbar_fence_init();
   }
   if (threadIdx.x < t0 || s.lite == lite) return;  // summaries read where they lie (see cta_smem)
@@ -137,17 +139,19 @@ __device__ __forceinline__ void init_cta(const Smem &s, const RunLite *lite, uin
 // ---- grid-barrier warp: once per pass, after the CTA's P blocks are summed
 // (pdone), arrive on the grid barrier, wait for it and release the U runs
 // (gdone).  The barrier latency stays off the consumer and gather warps.
-// Pass p uses grid-barrier instance k0 + p * kstep of the launch.
+// Pass p uses grid-barrier instance (p / 2) * kstep + (p odd ? k1 : k0) of the
+// launch.  It returns early once the solve has stopped (rsum[4]).
 // `beyond` > 0 (a test hook) waits for an instance that no launch of this
 // grid completes, so the bounded waits of the whole CTA expire.
-__device__ __forceinline__ void sync_warp(unsigned *gbar, uint32_t npass, uint32_t k0, uint32_t kstep, const Smem &sm,
-                                          int *err, uint64_t tmo, uint32_t beyond = 0) {
+__device__ __forceinline__ void sync_warp(unsigned *gbar, uint32_t npass, uint32_t k0, uint32_t k1, uint32_t kstep,
+                                          const Smem &sm, int *err, uint64_t tmo, uint32_t beyond = 0) {
   for (uint32_t p = 0; p < npass; ++p) {
     if (!mbar_wait(sm.pdone, p & 1, tmo)) {
       atomicOr(err, kErrPipeline);
       return;  // the waits on gdone are bounded too
     }
-    const unsigned target = grid_target(sm.rsum[1], k0 + p * kstep + beyond, gridDim.x);
+    if (ld_acquire_s(&sm.rsum[4])) return;
+    const unsigned target = grid_target(sm.rsum[1], (p / 2) * kstep + ((p & 1) ? k1 : k0) + beyond, gridDim.x);
     grid_arrive(gbar, target);  // a release: the CTA's zbu stores (before pdone) are visible grid-wide
     if (!grid_wait(gbar, target, tmo)) {
       atomicOr(err, kErrGridBarrier);
@@ -171,8 +175,6 @@ struct PassOut {
   const double *yin;
   double *y, *zbu;
   float *zbu32;     // FP32 engines: zbu rounded to float (what the U runs gather)
-  uint32_t pass;    // pass index within the launch (barrier parities)
-  uint32_t nblk_p;  // P blocks of the CTA
 };
 
 // End of a block for a consumer warp: park its row sums (rows lane and
@@ -183,19 +185,18 @@ __device__ __forceinline__ bool block_end(double t0, double t1, uint32_t &nb, co
                                           uint64_t tmo) {
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t slot = nb % kRedSlots;
-  int ok = 1;
-  if (nb >= kRedSlots && lane == 0 && ld_acquire_s(sm.rsum) + kRedSlots <= nb) {
+  auto free_slot = [&]() { return ld_acquire_s(sm.rsum) + kRedSlots > nb; };
+  if (nb >= kRedSlots && !__all_sync(0xffffffffu, free_slot())) {
     const uint64_t ts = gtimer();
-    while (ld_acquire_s(sm.rsum) + kRedSlots <= nb) {
-      if (gtimer() - ts > tmo) {
-        ok = 0;
-        atomicOr(err, kErrPipeline);
-        break;
+    while (!__all_sync(0xffffffffu, free_slot())) {
+      if (__any_sync(0xffffffffu, gtimer() - ts > tmo)) {
+        if (lane == 0) atomicOr(err, kErrPipeline);
+        ++nb;
+        return false;
       }
     }
   }
   ++nb;
-  if (!__shfl_sync(0xffffffffu, ok, 0)) return false;
   double *rb = sm.red + slot * (NW * 64) + w * 64;
   rb[lane] = t0;
   rb[32 + lane] = t1;
@@ -210,17 +211,22 @@ __device__ __forceinline__ bool block_end(double t0, double t1, uint32_t &nb, co
 // alpha*s (the atom's D block was summed before, in this same order) --
 // then free the slot.  After the pass's last P block it signals pdone (the
 // CTA's zbu rows are complete), after the pass's last block rdone.
-__device__ __forceinline__ void sum_warp(uint32_t nr, uint32_t npass, uint32_t nblk_p, const PassOut *outs,
-                                         const Smem &sm, int *err, uint64_t tmo) {
+template <class Outs>  // outs(pass): where that pass's sums go
+__device__ __forceinline__ void sum_warp(uint32_t nr, uint32_t npass, uint32_t nblk_p, Outs outs, const Smem &sm,
+                                         int *err, uint64_t tmo) {
   const int lane = threadIdx.x & 31;
   uint32_t nb = 0;
   for (uint32_t pass = 0; pass < npass; ++pass) {
-    const PassOut &o = outs[pass];
+    const PassOut o = outs(pass);
     // Not before the pass has started: rdone must not run a phase ahead of
     // the consumers' wait on it (a CTA without blocks would otherwise
     // complete both passes' phases at once).
     if (!warp_wait(sm.xready, pass & 1, tmo)) {
       if (lane == 0) atomicOr(err, kErrPipeline);
+      return;
+    }
+    if (ld_acquire_s(&sm.rsum[4])) {  // no such pass: wake the grid-barrier warp too
+      if (lane == 0) mbar_arrive(sm.pdone);
       return;
     }
     uint32_t np_done = 0;
@@ -312,12 +318,12 @@ __device__ __forceinline__ void consume_pass(Ring &R, uint32_t K, uint32_t nr, u
 // row of the pass is written) and, in warp 0, for the pass's grid barrier
 // (the caller's next grid barrier must not start before it completes).
 template <int kPrec>
-__device__ __forceinline__ void matvec_pass(Ring &R, uint32_t K, uint32_t nr, uint32_t &nb, const PassOut &o,
-                                            const Smem &sm, int *err, uint64_t tmo) {
-  if (o.nblk_p == 0 && threadIdx.x == 0) mbar_arrive(sm.pdone);
-  consume_pass<kPrec>(R, K, nr, nb, o.pass, sm, err, tmo);
-  if (!warp_wait(sm.rdone, o.pass & 1, tmo) && (threadIdx.x & 31) == 0) atomicOr(err, kErrPipeline);
-  if (threadIdx.x < 32 && !warp_wait(sm.gdone, o.pass & 1, tmo) && threadIdx.x == 0) atomicOr(err, kErrGridBarrier);
+__device__ __forceinline__ void matvec_pass(Ring &R, uint32_t K, uint32_t nr, uint32_t &nb, uint32_t pass,
+                                            uint32_t nblk_p, const Smem &sm, int *err, uint64_t tmo) {
+  if (nblk_p == 0 && threadIdx.x == 0) mbar_arrive(sm.pdone);
+  consume_pass<kPrec>(R, K, nr, nb, pass, sm, err, tmo);
+  if (!warp_wait(sm.rdone, pass & 1, tmo) && (threadIdx.x & 31) == 0) atomicOr(err, kErrPipeline);
+  if (threadIdx.x < 32 && !warp_wait(sm.gdone, pass & 1, tmo) && threadIdx.x == 0) atomicOr(err, kErrGridBarrier);
 }
 
 // Bytes at the head of a CTA's stream read with the evict_last policy: a
@@ -361,18 +367,19 @@ __global__ void __launch_bounds__(kThreads, 1) k_matvec(MatvecArgs a) {
     return;
   }
   if (w == kSyncWarp) {
-    if (lane == 0) sync_warp(a.gbar, 1, 0, 0, sm, a.err, a.timeout_ns, a.stall ? 1u : 0u);
+    if (lane == 0) sync_warp(a.gbar, 1, 0, 0, 0, sm, a.err, a.timeout_ns, a.stall ? 1u : 0u);
     return;
   }
-  const PassOut o{a.alpha, a.beta, a.yin, a.y, a.zbu, kF32 ? a.zbu32 : nullptr, 0, ci.nblk_p};
   if (w == kSumWarp) {
-    sum_warp(nr, 1, ci.nblk_p, &o, sm, a.err, a.timeout_ns);
+    sum_warp(nr, 1, ci.nblk_p,
+             [&](uint32_t) { return PassOut{a.alpha, a.beta, a.yin, a.y, a.zbu, kF32 ? a.zbu32 : nullptr}; }, sm, a.err,
+             a.timeout_ns);
     return;
   }
   if (threadIdx.x == 0) signal_xready(sm, 0);  // x is an input: ready from the start
   uint32_t nb = 0;
   Ring R{sm.ring, sm.full, sm.empty, 0, 0, 0, a.timeout_ns, a.err, false};
-  matvec_pass<kPrec>(R, K, nr, nb, o, sm, a.err, a.timeout_ns);
+  matvec_pass<kPrec>(R, K, nr, nb, 0, ci.nblk_p, sm, a.err, a.timeout_ns);
   if (a.prof && threadIdx.x == 0) {
     a.prof[blockIdx.x * 16 + 0] = t_start;
     a.prof[blockIdx.x * 16 + 5] = gtimer();
@@ -402,8 +409,16 @@ __device__ __forceinline__ void for_more_rows(const Atom *atoms, const CtaInfo &
   }
 }
 
+// The partials of a slot lie back to back over the CTAs, 16 bytes each: every
+// CTA reads all of them after a grid barrier, 148 warps at once, and with one
+// 128-byte line per CTA (all its slots together) that took 3.5 us, of which the
+// 19 lines of a slot take under one.
+__device__ __forceinline__ double2 *part_of(double *part, int ncta, int slot, int cta) {
+  return reinterpret_cast<double2 *>(part) + (size_t)slot * ncta + cta;
+}
+
 // Per-CTA compensated partial sums of NS dot products over the owned rows.
-// acc[] holds the calling thread's partials; the result goes to part[cta][slot0+k].
+// acc[] holds the calling thread's partials; the result goes to slots slot0+k.
 template <int NSL>
 __device__ __forceinline__ void cta_partials(Acc2 (&acc)[NSL], double *part, int slot0, const Smem &sm) {
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -422,9 +437,7 @@ __device__ __forceinline__ void cta_partials(Acc2 (&acc)[NSL], double *part, int
   if (w == 0 && lane < NSL) {
     Acc2 t{sc[lane * 2], sc[lane * 2 + 1]};
     for (int q = 1; q < NW; ++q) t = acc2_merge(t, Acc2{sc[(q * NSL + lane) * 2], sc[(q * NSL + lane) * 2 + 1]});
-    double *dst = part + ((size_t)blockIdx.x * kSlots + slot0 + lane) * 2;
-    dst[0] = t.s;
-    dst[1] = t.c;
+    *part_of(part, gridDim.x, slot0 + lane, blockIdx.x) = make_double2(t.s, t.c);
     __threadfence();
   }
   named_bar(1, kConsumerThreads);
@@ -444,8 +457,8 @@ __device__ __forceinline__ double reduce_slot(const double *part, int ncta, int 
       const int c = c0 + lane + 32 * k;
       v[k] = Acc2{0.0, 0.0};
       if (c < ncta) {
-        const double *src = part + ((size_t)c * kSlots + slot) * 2;
-        v[k] = Acc2{__ldcg(src), __ldcg(src + 1)};
+        const double2 x = __ldcg(part_of(const_cast<double *>(part), ncta, slot, c));
+        v[k] = Acc2{x.x, x.y};
       }
     }
 #pragma unroll
@@ -455,25 +468,94 @@ __device__ __forceinline__ double reduce_slot(const double *part, int ncta, int 
   return a.s + a.c;
 }
 
+// Totals of N slots at once (full warp), each as reduce_slot sums it: the
+// loads of all slots are under way together.
+template <int N>
+__device__ __forceinline__ void reduce_slots(const double *part, int ncta, const int (&slot)[N], double (&tot)[N]) {
+  constexpr int kBatch = 5;
+  const int lane = threadIdx.x & 31;
+  Acc2 a[N];
+#pragma unroll
+  for (int q = 0; q < N; ++q) a[q] = Acc2{0.0, 0.0};
+  for (int c0 = 0; c0 < ncta; c0 += 32 * kBatch) {
+    Acc2 v[N][kBatch];
+#pragma unroll
+    for (int q = 0; q < N; ++q)
+#pragma unroll
+      for (int k = 0; k < kBatch; ++k) {
+        const int c = c0 + lane + 32 * k;
+        v[q][k] = Acc2{0.0, 0.0};
+        if (c < ncta) {
+          const double2 x = __ldcg(part_of(const_cast<double *>(part), ncta, slot[q], c));
+          v[q][k] = Acc2{x.x, x.y};
+        }
+      }
+#pragma unroll
+    for (int q = 0; q < N; ++q)
+#pragma unroll
+      for (int k = 0; k < kBatch; ++k) a[q] = acc2_merge(a[q], v[q][k]);
+  }
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+    a[q] = warp_merge(a[q]);
+    tot[q] = a[q].s + a[q].c;
+  }
+}
+
 // Grid-barrier instances of one BiCGSTAB step, in order: p complete, zbu of
 // the first H-matvec complete, the r^.Ap partials, t complete, zbu of the
-// second H-matvec, the At.t / At.At partials.
-enum : unsigned { kGridP = 0, kGridPass0 = 1, kGridAlpha = 2, kGridT = 3, kGridPass1 = 4, kGridZeta = 5 };
+// second H-matvec, the At.t / At.At partials, the r^.r / r.r partials.
+enum : unsigned {
+  kGridP = 0, kGridPass0 = 1, kGridAlpha = 2, kGridT = 3, kGridPass1 = 4, kGridZeta = 5, kGridEnd = 6, kGridStep = 7
+};
+
+// Grid-barrier instance k of the launch for this CTA, by one whole warp.
+__device__ __forceinline__ void arrive_and_wait(unsigned *gbar, unsigned k, int *err, uint64_t timeout_ns,
+                                                const Smem &sm) {
+  const unsigned target = grid_target(sm.rsum[1], k, gridDim.x);
+  if ((threadIdx.x & 31) == 0) grid_arrive(gbar, target);
+  __syncwarp();
+  if (!grid_wait_warp(gbar, target, timeout_ns) && (threadIdx.x & 31) == 0) atomicOr(err, kErrGridBarrier);
+}
 
 // Full grid barrier (instance k of the launch) among the consumer warps of
-// every CTA.
-__device__ __forceinline__ bool grid_sync(unsigned *gbar, unsigned k, int *err, uint64_t timeout_ns, const Smem &sm) {
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+// every CTA: what their threads wrote before it is read after it (bar.sync,
+// then the arriving thread's release; no fence of their own).
+__device__ __forceinline__ void grid_sync(unsigned *gbar, unsigned k, int *err, uint64_t timeout_ns, const Smem &sm) {
   named_bar(1, kConsumerThreads);
-  if (w == 0 && lane == 0) {
-    const unsigned target = grid_target(sm.rsum[1], k, gridDim.x);
-    grid_arrive(gbar, target);
-    const bool ok = grid_wait(gbar, target, timeout_ns);
-    if (!ok) atomicOr(err, kErrGridBarrier);
-    sm.scal[62] = ok ? 1.0 : 0.0;
+  if (threadIdx.x < 32) arrive_and_wait(gbar, k, err, timeout_ns, sm);
+  named_bar(1, kConsumerThreads);
+}
+
+// The CTA's compensated partials of NSL dots to slots slot0 + k, then
+// grid-barrier instance `inst`, all in warp 0 after one barrier of the CTA: the
+// partials are all that the others wait for, and warp 0 goes straight on to
+// their totals (the other warps wait for those at the caller's next barrier).
+// The caller's warps have waited for the block-sum warp (rdone), so sm.red is
+// free.
+template <int NSL>
+__device__ __forceinline__ void share_partials(Acc2 (&acc)[NSL], double *part, int slot0, unsigned *gbar, unsigned inst,
+                                               int *err, uint64_t timeout_ns, const Smem &sm) {
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int k = 0; k < NSL; ++k) acc[k] = warp_merge(acc[k]);
+  double *sc = sm.red;  // reuse: [NW][NSL][2]
+  if (lane == 0) {
+#pragma unroll
+    for (int k = 0; k < NSL; ++k) {
+      sc[(w * NSL + k) * 2 + 0] = acc[k].s;
+      sc[(w * NSL + k) * 2 + 1] = acc[k].c;
+    }
   }
   named_bar(1, kConsumerThreads);
-  return sm.scal[62] != 0.0;
+  if (w != 0) return;
+  if (lane < NSL) {
+    Acc2 t{sc[lane * 2], sc[lane * 2 + 1]};
+    for (int q = 1; q < NW; ++q) t = acc2_merge(t, Acc2{sc[(q * NSL + lane) * 2], sc[(q * NSL + lane) * 2 + 1]});
+    *part_of(part, gridDim.x, slot0 + lane, blockIdx.x) = make_double2(t.s, t.c);
+  }
+  __syncwarp();
+  arrive_and_wait(gbar, inst, err, timeout_ns, sm);
 }
 
 #ifndef HBX_STEP_LP
@@ -505,113 +587,55 @@ __global__ void __launch_bounds__(kThreads, 1) k_bicg_setup(BicgArgs a) {
 }
 #endif
 
+// Up to a.steps BiCGSTAB steps.  One launch per step paid a launch boundary
+// and a cold start -- barriers, run summaries, the first chunks of the stream
+// -- every step; within a launch the ring stays full from step to step and a
+// grid barrier takes their place.  When the stop test ends the solve before
+// a.steps, the warps that run ahead are told (rsum[4]) and woken: the producer
+// by one more emptied slot, the gather and block-sum warps by the signal of a
+// pass that does not follow, the grid-barrier warp by the block-sum warp.
+// HBM bounds the passes; the six barriers between them bound small matrices.
+// Time of a step, one launch per step -> this: N = 320 27.3 -> 20.5 us, 1,280
+// 38.6 -> 31.1, 5,120 48.8 -> 41.8, 20,480 119 -> 109.5 (two passes of 265 MB
+// at 6.55 TB/s: 81).
 template <int kPrec>
-__global__ void __launch_bounds__(kThreads, 1) k_bicg_iter(BicgArgs a) {
+__global__ void __launch_bounds__(kThreads, 1) k_bicg_steps(BicgArgs a) {
   constexpr bool kF32 = kPrec != kFP64;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
+  if (*(volatile const int *)&a.state->done) return;  // an earlier launch ended the solve (or its waits ran out)
   const CtaInfo ci = a.ctas[blockIdx.x];
   const uint32_t nr = ci.nr_p + ci.nr_d + ci.nr_u;
   const Smem sm = cta_smem(smem_raw, a.lite + ci.rec_begin, nr);
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ncta = gridDim.x;
+  const uint32_t npass = 2u * (uint32_t)a.steps;
   auto stamp = [&](int k) {
     if (a.prof && threadIdx.x == 0) a.prof[blockIdx.x * 16 + 8 + k] = gtimer();
   };
-  const uint64_t t_start = a.prof ? gtimer() : 0;
-  // A consumer warp's first owned atom and this lane's row of it: its vector
-  // entries stay in registers through the step, loaded while the step's
-  // scalars are reduced (the rows of further atoms are read where needed).
+  // A consumer warp's first owned atom and this lane's row of it: r, p and t
+  // stay in registers through the launch, the other vectors' entries are read
+  // ahead of the barrier before their use (the rows of further atoms are read
+  // where needed).
   const Atom a0 = (w < NW && (uint32_t)w < ci.n_atoms) ? a.atoms[ci.atom_begin + w] : Atom{0, 0};
   const bool own0 = (uint32_t)lane < a0.h;
   const uint32_t row0 = a0.r0 + lane;
-  double c_r = 0.0, c_rh = 0.0, c_p = 0.0, c_ap = 0.0, c_u = 0.0, c_t = 0.0, c_at = 0.0;
+  double c_r = 0.0, c_p = 0.0, c_t = 0.0;
   if (own0) {
     c_r = a.r[row0];
-    c_rh = a.rh[row0];
     c_p = __ldcg(&a.p[row0]);  // see S1
-    c_ap = a.ap[row0];
-    c_u = a.u[row0];
   }
-  // the producer starts the stream of the first H-matvec, warps 4 and up set
-  // up the CTA and warps 0-3 reduce the scalars
+  // the producer starts the stream of the first H-matvec while the other
+  // threads set up the CTA
   const StreamSrc ss{a.stream + ci.stream_off, ci.stream_bytes, keep_bytes(ci.stream_bytes, a.keep_frac)};
   uint32_t issued0 = 0;
-  if (threadIdx.x == kProducerWarp * 32) issued0 = producer_start(ss, 2, sm.ring, sm.full, sm.empty);
+  if (threadIdx.x == kProducerWarp * 32) issued0 = producer_start(ss, npass, sm.ring, sm.full, sm.empty);
   init_cta_part(sm, a.lite + ci.rec_begin, nr, a.gbar, 128, NW / groups_of<kPrec>());
-
-  // ---- S0: scalars of the previous step; stop test at the top of the loop
-  // (HACApK_SOLVER.c:602-603).  Every CTA computes identical values: warps
-  // 0-2 reduce the three dot products side by side, warp 3 reads the state.
-  if (w < 3) {
-    const double v = reduce_slot(a.part, ncta, w == 0 ? kSlotRhoR : (w == 1 ? kSlotRR : kSlotBB));
-    if (lane == 0) sm.scal[10 + w] = v;
-  } else if (w == 3 && lane == 0) {
-    sm.scal[13] = __ldcg(&a.state->alpha);
-    sm.scal[14] = __ldcg(&a.state->zeta);
-    sm.scal[15] = __ldcg(&a.state->rho);
-    sm.scal[16] = (double)__ldcg(&a.state->iter);
-    sm.scal[17] = (double)__ldcg(&a.state->done);
-    sm.scal[18] = (double)__ldcg(&a.state->status);
-    sm.scal[19] = (double)__ldcg(&a.state->breakdown);
-  }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    const double rho_new = sm.scal[10], rr = sm.scal[11], bb = sm.scal[12];
-    BicgState st;
-    st.alpha = sm.scal[13];
-    st.zeta = sm.scal[14];
-    st.rho = sm.scal[15];
-    st.iter = (int)sm.scal[16];
-    st.done = (int)sm.scal[17];
-    st.status = (int)sm.scal[18];
-    st.breakdown = (int)sm.scal[19];
-    const double bnorm = sqrt(bb);
-    const double relres = (bnorm > 0.0) ? sqrt(rr) / bnorm : 0.0;
-    int done = st.done, status = st.status;
-    double beta = 0.0;
-    if (!done) {
-      if (st.breakdown) { done = 1; status = HBX_ERR_BREAKDOWN; }
-      // NaN or Inf in b or x0 shows in b.b or r.r before the first step
-      else if (!isfinite(bb) || !isfinite(rr)) { done = 1; status = st.iter == 0 ? HBX_ERR_NONFINITE : HBX_ERR_BREAKDOWN; }
-      else if (relres < a.tol) { done = 1; status = HBX_OK; }
-      else if (!isfinite(relres)) { done = 1; status = HBX_ERR_BREAKDOWN; }
-      else if (st.iter >= a.max_iter) { done = 1; status = HBX_ERR_NOT_CONVERGED; }
-      else if (st.iter > 0) {
-        // beta = -alpha/zeta * (rh.r_new)/znormold with the reference's sign
-        // flips (HACApK_SOLVER.c:650-655, :699, :724) = (alpha/zeta) rho_new/rho_old
-        beta = (st.alpha / st.zeta) * (rho_new / st.rho);
-        if (!isfinite(beta)) { done = 1; status = HBX_ERR_BREAKDOWN; }
-      }
-    }
-    sm.scal[0] = done;
-    sm.scal[1] = status;
-    sm.scal[2] = beta;
-    sm.scal[3] = st.zeta;
-    sm.scal[4] = rho_new;
-    sm.scal[5] = relres;
-    sm.scal[6] = st.iter;
-    sm.scal[7] = bnorm;
-    if (done && blockIdx.x == 0) {
-      a.state->done = 1;
-      a.state->status = status;
-      a.state->relres = relres;
-      a.state->bnorm = bnorm;
-    }
-  }
-  __syncthreads();
-  if (sm.scal[0] != 0.0) {
-    if (threadIdx.x == kProducerWarp * 32) producer_drain(sm.full, issued0, a.timeout_ns);
-    return;
-  }
-  if (a.prof && threadIdx.x == 0) a.prof[blockIdx.x * 16 + 8] = t_start;  // stamps of working steps only
-  const double beta = sm.scal[2], zeta_prev = sm.scal[3], rho = sm.scal[4];
-  const double relres = sm.scal[5], bnorm = sm.scal[7];
-  const int iter = (int)sm.scal[6];
 
   const uint32_t K = (ci.stream_bytes + kChunkBytes - 1) >> kChunkLog;
   if (w == kProducerWarp) {
     if (lane == 0 && K > 0)
-      producer_run(ss, 2, issued0, sm.ring, sm.full, sm.empty, a.err, a.timeout_ns);
+      producer_run(ss, npass, issued0, sm.ring, sm.full, sm.empty, a.err, a.timeout_ns, &sm.rsum[4]);
     return;
   }
   if (w >= kGatherWarp0 && w < kSyncWarp) {
@@ -620,173 +644,239 @@ __global__ void __launch_bounds__(kThreads, 1) k_bicg_iter(BicgArgs a) {
     const void *z0 = kF32 ? static_cast<const void *>(a.zbu32) : static_cast<const void *>(a.zbu);
     const void *z1 =
         kF32 ? static_cast<const void *>(a.zbu32 + a.zbu_len) : static_cast<const void *>(a.zbu + a.zbu_len);
-    const GatherCtx c{a.recs + ci.rec_begin, nr, ci.nr_p + ci.nr_d, 2, x0, x1, z0, z1, a.err, a.timeout_ns};
+    const GatherCtx c{a.recs + ci.rec_begin, nr, ci.nr_p + ci.nr_d, npass, x0, x1, z0, z1, a.err, a.timeout_ns};
     gather_warp<kPrec>(c, sm, (uint32_t)(w - kGatherWarp0));
     return;
   }
   if (w == kSyncWarp) {
-    if (lane == 0) sync_warp(a.gbar, 2, kGridPass0, kGridPass1 - kGridPass0, sm, a.err, a.timeout_ns);
+    if (lane == 0) sync_warp(a.gbar, npass, kGridPass0, kGridPass1, kGridStep, sm, a.err, a.timeout_ns);
     return;
   }
-  // The two H-matvecs write separate zbu copies, so a U run of the second
-  // never reads a line of the first from L1.
-  const PassOut outs[2] = {{1.0, 0.0, nullptr, a.ap, a.zbu, kF32 ? a.zbu32 : nullptr, 0, ci.nblk_p},
-                           {1.0, 0.0, nullptr, a.at, a.zbu + a.zbu_len, kF32 ? a.zbu32 + a.zbu_len : nullptr, 1,
-                            ci.nblk_p}};
+  // The two H-matvecs of a step write separate zbu copies: a CTA may still
+  // gather the first's when another writes the second's.
   if (w == kSumWarp) {
-    sum_warp(nr, 2, ci.nblk_p, outs, sm, a.err, a.timeout_ns);
+    sum_warp(nr, npass, ci.nblk_p,
+             [&](uint32_t pass) {
+               const size_t z = (pass & 1) ? a.zbu_len : 0;
+               return PassOut{1.0, 0.0, nullptr, (pass & 1) ? a.at : a.ap, a.zbu + z, kF32 ? a.zbu32 + z : nullptr};
+             },
+             sm, a.err, a.timeout_ns);
     return;
   }
   Ring R{sm.ring, sm.full, sm.empty, 0, 0, 0, a.timeout_ns, a.err, false};
   uint32_t nb = 0;
+  bool broke = false;  // the last step broke down and formed no new partials
+  // the previous step's alpha, zeta, rho and count: scal[24..27] (identical in every CTA)
 
-  // ---- S1: p = r + beta*(p - zeta*Ap)  (p = r on the first step)
-  if (own0) {
-    c_p = (beta == 0.0) ? c_r : fma(-zeta_prev, c_ap, c_p) * beta + c_r;
-    a.p[row0] = c_p;
-    if (kF32) a.p32[row0] = (float)c_p;
-  }
-  if (beta == 0.0) {
-    for_more_rows(a.atoms, ci, [&](uint32_t r) {
-      const double v = a.r[r];
-      a.p[r] = v;
-      if (kF32) a.p32[r] = (float)v;
-    });
-  } else {
-    for_more_rows(a.atoms, ci, [&](uint32_t r) {
-      // p through L2 only: a line of p cached in L1 here could hold rows of
-      // another CTA that the gather warps read after it rewrote them
-      const double v = fma(-zeta_prev, a.ap[r], __ldcg(&a.p[r])) * beta;
-      const double pv = v + a.r[r];
-      a.p[r] = pv;
-      if (kF32) a.p32[r] = (float)pv;
-    });
-  }
-  __threadfence();
-  grid_sync(a.gbar, kGridP, a.err, a.timeout_ns, sm);
-  if (threadIdx.x == 0) signal_xready(sm, 0);  // p complete grid-wide: pass 0 may be gathered
-  stamp(1);
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    a.state->iter = iter + 1;
-    a.state->beta = beta;
-    a.state->rho = rho;
-    a.state->relres = relres;
-    a.state->bnorm = bnorm;
-    a.hist[iter] = relres;
-  }
-
-  // ---- S2: Ap = H p;  rh . Ap
-  matvec_pass<kPrec>(R, K, nr, nb, outs[0], sm, a.err, a.timeout_ns);
-  stamp(2);
-  {
-    Acc2 acc[1] = {{0, 0}};
-    named_bar(1, kConsumerThreads);
-    if (own0) {
-      c_ap = a.ap[row0];
-      dot2_add(acc[0], c_rh, c_ap);
+  for (int it = 0; it <= a.steps; ++it) {
+    const unsigned k0 = (unsigned)it * kGridStep;
+    const double l_ap = own0 ? a.ap[row0] : 0.0;
+    // ---- S0: scalars of the previous step; stop test at the top of the loop
+    // (HACApK_SOLVER.c:602-603).  Every CTA computes identical values.  (The
+    // step before has passed the grid barrier of its partials; one that broke
+    // down formed none, and those of the step before it stand.)
+    if (it == 0 && threadIdx.x == 0) {
+      sm.scal[24] = __ldcg(&a.state->alpha);
+      sm.scal[25] = __ldcg(&a.state->zeta);
+      sm.scal[26] = __ldcg(&a.state->rho);
+      sm.scal[27] = (double)__ldcg(&a.state->iter);
     }
-    for_more_rows(a.atoms, ci, [&](uint32_t r) { dot2_add(acc[0], a.rh[r], a.ap[r]); });
-    cta_partials<1>(acc, a.part, kSlotRhAp, sm);
-  }
-  grid_sync(a.gbar, kGridAlpha, a.err, a.timeout_ns, sm);
-  if (w == 0) {
-    const double zden = reduce_slot(a.part, ncta, kSlotRhAp);
-    if (lane == 0) sm.scal[8] = rho / zden;
-  }
-  named_bar(1, kConsumerThreads);
-  const double alpha = sm.scal[8];
-  stamp(3);
-
-  // ---- S3: t = r - alpha*Ap
-  if (own0) {
-    c_t = fma(-alpha, c_ap, c_r);
-    a.t[row0] = c_t;
-    if (kF32) a.t32[row0] = (float)c_t;
-  }
-  for_more_rows(a.atoms, ci, [&](uint32_t r) {
-    const double v = fma(-alpha, a.ap[r], a.r[r]);
-    a.t[r] = v;
-    if (kF32) a.t32[r] = (float)v;
-  });
-  __threadfence();
-  grid_sync(a.gbar, kGridT, a.err, a.timeout_ns, sm);
-  if (threadIdx.x == 0) signal_xready(sm, 1);  // t complete grid-wide: pass 1 may be gathered
-  stamp(4);
-
-  // ---- S4: At = H t;  At . t,  At . At
-  R.base = K;
-  matvec_pass<kPrec>(R, K, nr, nb, outs[1], sm, a.err, a.timeout_ns);
-  stamp(5);
-  {
-    Acc2 acc[2] = {{0, 0}, {0, 0}};
+    if (w == 0) {
+      const int expired = lane == 0 ? *(volatile const int *)a.err : 0;
+      double tot[3];
+      reduce_slots<3>(a.part, ncta, {kSlotRhoR, kSlotRR, kSlotBB}, tot);
+      const double rho_new = tot[0], rr = tot[1], bb = tot[2];
+      if (lane == 0) {
+        const double alpha = sm.scal[24], zeta = sm.scal[25], rho = sm.scal[26];
+        const int iter = (int)sm.scal[27];
+        const double bnorm = sqrt(bb);
+        const double relres = (bnorm > 0.0) ? sqrt(rr) / bnorm : 0.0;
+        int done = 0, status = HBX_OK;
+        double beta = 0.0;
+        if (expired) { done = 1; status = HBX_ERR_TIMEOUT; }  // a wait ran out: no more of them
+        else if (broke) { done = 1; status = HBX_ERR_BREAKDOWN; }
+        // NaN or Inf in b or x0 shows in b.b or r.r before the first step
+        else if (!isfinite(bb) || !isfinite(rr)) { done = 1; status = iter == 0 ? HBX_ERR_NONFINITE : HBX_ERR_BREAKDOWN; }
+        else if (relres < a.tol) { done = 1; status = HBX_OK; }
+        else if (!isfinite(relres)) { done = 1; status = HBX_ERR_BREAKDOWN; }
+        else if (iter >= a.max_iter) { done = 1; status = HBX_ERR_NOT_CONVERGED; }
+        else if (iter > 0) {
+          // beta = -alpha/zeta * (rh.r_new)/znormold with the reference's sign
+          // flips (HACApK_SOLVER.c:650-655, :699, :724) = (alpha/zeta) rho_new/rho_old
+          beta = (alpha / zeta) * (rho_new / rho);
+          if (!isfinite(beta)) { done = 1; status = HBX_ERR_BREAKDOWN; }
+        }
+        sm.scal[0] = done;
+        sm.scal[2] = beta;
+        sm.scal[3] = zeta;
+        sm.scal[4] = rho_new;
+        sm.scal[5] = relres;
+        sm.scal[7] = bnorm;
+        if (done && blockIdx.x == 0) {
+          a.state->status = status;
+          a.state->relres = relres;
+          a.state->bnorm = bnorm;
+          a.state->done = 1;
+        }
+      }
+    }
     named_bar(1, kConsumerThreads);
+    if (sm.scal[0] != 0.0 || it == a.steps) {
+      if (it < a.steps) {  // the launch's later passes do not follow
+        if (threadIdx.x == 0) {
+          st_release_s(&sm.rsum[4], 1u);
+          signal_xready(sm, 0x7ffffffeu);
+        }
+        named_bar(1, kConsumerThreads);
+        if (lane == 0) mbar_arrive(&sm.empty[R.released % kRingChunks]);
+      }
+      return;
+    }
+    const double beta = sm.scal[2], zeta_prev = sm.scal[3];
+    stamp(0);
+
+    // ---- S1: p = r + beta*(p - zeta*Ap)  (p = r on the first step)
     if (own0) {
-      c_at = a.at[row0];
-      dot2_add(acc[0], c_at, c_t);
-      dot2_add(acc[1], c_at, c_at);
+      c_p = (beta == 0.0) ? c_r : fma(-zeta_prev, l_ap, c_p) * beta + c_r;
+      a.p[row0] = c_p;
+      if (kF32) a.p32[row0] = (float)c_p;
+    }
+    if (beta == 0.0) {
+      for_more_rows(a.atoms, ci, [&](uint32_t r) {
+        const double v = a.r[r];
+        a.p[r] = v;
+        if (kF32) a.p32[r] = (float)v;
+      });
+    } else {
+      for_more_rows(a.atoms, ci, [&](uint32_t r) {
+        // p through L2 only: a line of p cached in L1 here could hold rows of
+        // another CTA that the gather warps read after it rewrote them
+        const double v = fma(-zeta_prev, a.ap[r], __ldcg(&a.p[r])) * beta;
+        const double pv = v + a.r[r];
+        a.p[r] = pv;
+        if (kF32) a.p32[r] = (float)pv;
+      });
+    }
+    grid_sync(a.gbar, k0 + kGridP, a.err, a.timeout_ns, sm);
+    if (threadIdx.x == 0) signal_xready(sm, 2u * it);  // p complete grid-wide: the step's first pass may be gathered
+    stamp(1);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      const int iter = (int)sm.scal[27];
+      a.state->iter = iter + 1;
+      a.state->beta = beta;
+      a.state->rho = sm.scal[4];
+      a.state->relres = sm.scal[5];
+      a.state->bnorm = sm.scal[7];
+      a.hist[iter] = sm.scal[5];
+    }
+
+    // ---- S2: Ap = H p;  rh . Ap
+    R.base = 2u * it * K;
+    matvec_pass<kPrec>(R, K, nr, nb, 2u * it, ci.nblk_p, sm, a.err, a.timeout_ns);
+    stamp(2);
+    double c_ap = 0.0;
+    {
+      Acc2 acc[1] = {{0, 0}};
+      if (own0) {
+        c_ap = a.ap[row0];
+        dot2_add(acc[0], a.rh[row0], c_ap);
+      }
+      for_more_rows(a.atoms, ci, [&](uint32_t r) { dot2_add(acc[0], a.rh[r], a.ap[r]); });
+      share_partials<1>(acc, a.part, kSlotRhAp, a.gbar, k0 + kGridAlpha, a.err, a.timeout_ns, sm);
+    }
+    if (w == 0) {
+      const double zden = reduce_slot(a.part, ncta, kSlotRhAp);
+      if (lane == 0) sm.scal[8] = sm.scal[4] / zden;
+    }
+    named_bar(1, kConsumerThreads);
+    const double alpha = sm.scal[8];
+    stamp(3);
+
+    // ---- S3: t = r - alpha*Ap
+    if (own0) {
+      c_t = fma(-alpha, c_ap, c_r);
+      a.t[row0] = c_t;
+      if (kF32) a.t32[row0] = (float)c_t;
     }
     for_more_rows(a.atoms, ci, [&](uint32_t r) {
-      const double atv = a.at[r];
-      dot2_add(acc[0], atv, a.t[r]);
-      dot2_add(acc[1], atv, atv);
+      const double v = fma(-alpha, a.ap[r], a.r[r]);
+      a.t[r] = v;
+      if (kF32) a.t32[r] = (float)v;
     });
-    cta_partials<2>(acc, a.part, kSlotAtT, sm);
-  }
-  grid_sync(a.gbar, kGridZeta, a.err, a.timeout_ns, sm);
-  if (w < 2) {  // the two sums side by side
-    const double v = reduce_slot(a.part, ncta, w == 0 ? kSlotAtT : kSlotAtAt);
-    if (lane == 0) sm.scal[10 + w] = v;
-  }
-  named_bar(1, kConsumerThreads);
-  if (w == 0) {
-    const double s3 = sm.scal[10], s4 = sm.scal[11];
-    if (lane == 0) {
-      const double zeta = (s4 != 0.0) ? s3 / s4 : 0.0;
+    grid_sync(a.gbar, k0 + kGridT, a.err, a.timeout_ns, sm);
+    if (threadIdx.x == 0) signal_xready(sm, 2u * it + 1u);  // t complete grid-wide: the second pass may be gathered
+    stamp(4);
+
+    // ---- S4: At = H t;  At . t,  At . At
+    R.base += K;
+    matvec_pass<kPrec>(R, K, nr, nb, 2u * it + 1u, ci.nblk_p, sm, a.err, a.timeout_ns);
+    stamp(5);
+    double c_at = 0.0, c_u = 0.0, c_rh = 0.0;
+    {
+      Acc2 acc[2] = {{0, 0}, {0, 0}};
+      if (own0) {
+        c_at = a.at[row0];
+        c_u = a.u[row0];
+        c_rh = a.rh[row0];
+        dot2_add(acc[0], c_at, c_t);
+        dot2_add(acc[1], c_at, c_at);
+      }
+      for_more_rows(a.atoms, ci, [&](uint32_t r) {
+        const double atv = a.at[r];
+        dot2_add(acc[0], atv, a.t[r]);
+        dot2_add(acc[1], atv, atv);
+      });
+      share_partials<2>(acc, a.part, kSlotAtT, a.gbar, k0 + kGridZeta, a.err, a.timeout_ns, sm);
+    }
+    double sums[2] = {0.0, 0.0};
+    if (w == 0) reduce_slots<2>(a.part, ncta, {kSlotAtT, kSlotAtAt}, sums);
+    if (threadIdx.x == 0) {
+      const double zeta = (sums[1] != 0.0) ? sums[0] / sums[1] : 0.0;
       sm.scal[9] = zeta;
-      const bool bad = !isfinite(alpha) || !isfinite(zeta);
+      sm.scal[24] = alpha;
+      sm.scal[25] = zeta;
+      sm.scal[26] = sm.scal[4];
+      sm.scal[27] += 1.0;
       if (blockIdx.x == 0) {
         a.state->alpha = alpha;
         a.state->zeta = zeta;
-        if (bad) a.state->breakdown = 1;
       }
     }
-  }
-  named_bar(1, kConsumerThreads);
-  const double zeta = sm.scal[9];
-  stamp(6);
+    named_bar(1, kConsumerThreads);
+    const double zeta = sm.scal[9];
+    stamp(6);
 
-  // ---- S5: u += alpha*p + zeta*t;  r = t - zeta*At;  rh . r,  r . r
-  // A breakdown (alpha or zeta not finite: r^.Ap or At.At zero or
-  // overflowing, which HACApK_SOLVER.c:650, :694 divide by unchecked) keeps
-  // u and r of the previous step; the next launch ends the solve with
-  // HBX_ERR_BREAKDOWN.
-  if (!isfinite(alpha) || !isfinite(zeta)) {
-    stamp(7);
-    return;
-  }
-  {
-    Acc2 acc[2] = {{0, 0}, {0, 0}};
-    if (own0) {
-      a.u[row0] = fma(zeta, c_t, fma(alpha, c_p, c_u));
-      const double rv = fma(-zeta, c_at, c_t);
-      a.r[row0] = rv;
-      dot2_add(acc[0], c_rh, rv);
-      dot2_add(acc[1], rv, rv);
+    // ---- S5: u += alpha*p + zeta*t;  r = t - zeta*At;  rh . r,  r . r
+    // A breakdown (alpha or zeta not finite: r^.Ap or At.At zero or
+    // overflowing, which HACApK_SOLVER.c:650, :694 divide by unchecked) keeps
+    // u and r of the previous step; the stop test then ends the solve with
+    // HBX_ERR_BREAKDOWN.
+    broke = !isfinite(alpha) || !isfinite(zeta);
+    if (!broke) {
+      Acc2 acc[2] = {{0, 0}, {0, 0}};
+      if (own0) {
+        c_u = fma(zeta, c_t, fma(alpha, c_p, c_u));
+        a.u[row0] = c_u;
+        c_r = fma(-zeta, c_at, c_t);
+        a.r[row0] = c_r;
+        dot2_add(acc[0], c_rh, c_r);
+        dot2_add(acc[1], c_r, c_r);
+      }
+      for_more_rows(a.atoms, ci, [&](uint32_t r) {
+        const double uv = fma(alpha, a.p[r], a.u[r]);
+        a.u[r] = fma(zeta, a.t[r], uv);
+        const double rv = fma(-zeta, a.at[r], a.t[r]);
+        a.r[r] = rv;
+        dot2_add(acc[0], a.rh[r], rv);
+        dot2_add(acc[1], rv, rv);
+      });
+      share_partials<2>(acc, a.part, kSlotRhoR, a.gbar, k0 + kGridEnd, a.err, a.timeout_ns, sm);
     }
-    for_more_rows(a.atoms, ci, [&](uint32_t r) {
-      const double uv = fma(alpha, a.p[r], a.u[r]);
-      a.u[r] = fma(zeta, a.t[r], uv);
-      const double rv = fma(-zeta, a.at[r], a.t[r]);
-      a.r[r] = rv;
-      dot2_add(acc[0], a.rh[r], rv);
-      dot2_add(acc[1], rv, rv);
-    });
-    cta_partials<2>(acc, a.part, kSlotRhoR, sm);
+    stamp(7);
   }
-  stamp(7);
 }
 
-// part[cta][slot] over own rows, then (block 0 of a second launch) the total.
+// A slot's partials over own rows, then (block 0 of a second launch) the total.
 #ifndef HBX_STEP_LP
 __global__ void __launch_bounds__(kThreads, 1) k_dot_partial(BicgArgs a, const double *x, const double *y, int slot) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -885,7 +975,7 @@ cudaError_t configure_step_kernels() {
   const int smem = (int)SharedLayout::bytes;
   cudaError_t e;
   if ((e = cudaFuncSetAttribute(k_bicg_setup, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
-  if ((e = cudaFuncSetAttribute(k_bicg_iter<kFP64>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
+  if ((e = cudaFuncSetAttribute(k_bicg_steps<kFP64>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
   if ((e = cudaFuncSetAttribute(k_dot_partial, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
   return configure_step_kernels_lp();
 }
@@ -895,9 +985,9 @@ cudaError_t launch_bicg_setup(const BicgArgs &a, int num_ctas, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_bicg_iter(const BicgArgs &a, int num_ctas, cudaStream_t s, int precision) {
-  if (precision != kFP64) return launch_bicg_iter_lp(a, num_ctas, s, precision);
-  return launch_coop(k_bicg_iter<kFP64>, a, num_ctas, s);
+cudaError_t launch_bicg_steps(const BicgArgs &a, int num_ctas, cudaStream_t s, int precision) {
+  if (precision != kFP64) return launch_bicg_steps_lp(a, num_ctas, s, precision);
+  return launch_coop(k_bicg_steps<kFP64>, a, num_ctas, s);
 }
 
 cudaError_t launch_dot(const BicgArgs &a, const double *x, const double *y, int slot, double *out, int num_ctas,
@@ -911,14 +1001,14 @@ cudaError_t launch_dot(const BicgArgs &a, const double *x, const double *y, int 
 cudaError_t configure_step_kernels_lp() {
   const int smem = (int)SharedLayout::bytes;
   cudaError_t e;
-  if ((e = cudaFuncSetAttribute(k_bicg_iter<kFP32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
-  if ((e = cudaFuncSetAttribute(k_bicg_iter<kBF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
+  if ((e = cudaFuncSetAttribute(k_bicg_steps<kFP32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
+  if ((e = cudaFuncSetAttribute(k_bicg_steps<kBF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
   return cudaSuccess;
 }
 
-cudaError_t launch_bicg_iter_lp(const BicgArgs &a, int num_ctas, cudaStream_t s, int precision) {
-  return precision == kBF16 ? launch_coop(k_bicg_iter<kBF16>, a, num_ctas, s)
-                            : launch_coop(k_bicg_iter<kFP32>, a, num_ctas, s);
+cudaError_t launch_bicg_steps_lp(const BicgArgs &a, int num_ctas, cudaStream_t s, int precision) {
+  return precision == kBF16 ? launch_coop(k_bicg_steps<kBF16>, a, num_ctas, s)
+                            : launch_coop(k_bicg_steps<kFP32>, a, num_ctas, s);
 }
 #endif  // HBX_STEP_TU
 

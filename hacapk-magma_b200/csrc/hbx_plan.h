@@ -61,7 +61,7 @@ namespace hbx {
 constexpr int kAtomMax = 32;       // rows per D/U block (one lane per row)
 constexpr int kSlabMax = 64;       // rows per P slab (two rows per lane)
 // Consumer warps of the product kernels (k_matvec) and of the BiCGSTAB step
-// kernel (k_bicg_iter, compiled in its own translation unit with fewer
+// kernel (k_bicg_steps, compiled in its own translation unit with fewer
 // threads, so that it keeps its registers); the planner rotates the panels of
 // consecutive runs for both counts.
 constexpr int kProductWarps = 16;

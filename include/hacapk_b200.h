@@ -173,7 +173,7 @@ typedef struct hbx_solve_opts {
   double tol;          /* stop when ||r||/||b|| < tol (checked before each step) */
   int max_iter;        /* iteration limit (param[82] in the drop-in)             */
   int verbose;         /* >0: print the residual history like the reference     */
-  int batch;           /* iterations per graph replay between host checks (0=8) */
+  int batch;           /* iterations per launch between host checks (0=8)       */
   int restart;         /* hbx_gcr: restart length m, param(87) (0 = 8; at most 64) */
   double inner_tol;    /* mixed-precision solve: relative residual reduction asked
                           of each inner solve at most (0 = 1e-6)                 */
@@ -188,8 +188,8 @@ typedef struct hbx_solve_info {
   double true_relres;  /* ||b - H u|| / ||b|| recomputed after the solve      */
   double seconds;      /* device time from r0 = b - H u0 to the last step     */
   double iter_kernel_seconds; /* device time of the iteration launches only   */
-  int iter_launches;   /* iteration-kernel launches (includes the final
-                          launches that only observe convergence)             */
+  int iter_launches;   /* steps the iteration kernels entered (includes the
+                          ones that only observe the end)                     */
   int launches;        /* all kernel launches of the solve                    */
   int outer;           /* mixed-precision solve: refinement steps (FP64 residuals) */
   int reserved[5];
