@@ -179,10 +179,10 @@ struct PassOut {
 
 // End of a block for a consumer warp: park its row sums (rows lane and
 // lane + 32) in red slot nb mod kRedSlots, once the block-sum warp has
-// emptied it, and arrive on the slot's barrier.  Returns false after a
-// timed-out wait.
-__device__ __forceinline__ bool block_end(double t0, double t1, uint32_t &nb, const Smem &sm, int *err,
-                                          uint64_t tmo) {
+// emptied it, and arrive on the slot's barrier, `arrivals` times.  Returns
+// false after a timed-out wait.
+__device__ __forceinline__ bool block_end(double t0, double t1, uint32_t nb, uint32_t arrivals, const Smem &sm,
+                                          int *err, uint64_t tmo) {
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t slot = nb % kRedSlots;
   auto free_slot = [&]() { return ld_acquire_s(sm.rsum) + kRedSlots > nb; };
@@ -191,18 +191,36 @@ __device__ __forceinline__ bool block_end(double t0, double t1, uint32_t &nb, co
     while (!__all_sync(0xffffffffu, free_slot())) {
       if (__any_sync(0xffffffffu, gtimer() - ts > tmo)) {
         if (lane == 0) atomicOr(err, kErrPipeline);
-        ++nb;
         return false;
       }
     }
   }
-  ++nb;
   double *rb = sm.red + slot * (NW * 64) + w * 64;
   rb[lane] = t0;
   rb[32 + lane] = t1;
   __syncwarp();
-  if (lane == 0) mbar_arrive(&sm.redfull[slot]);
+  if (lane == 0) mbar_arrive(&sm.redfull[slot], arrivals);
   return true;
+}
+
+// p[0], p[64], ... of N warps, added in warp order.
+template <int N>
+__device__ __forceinline__ double warp_order_sum(const double *p) {
+  double s = p[0];
+#pragma unroll
+  for (int k = 1; k < N; ++k) s += p[k * 64];
+  return s;
+}
+
+// A row's sum s of a D, DU or U block.
+__device__ __forceinline__ void put_row(const PassOut &o, uint32_t kind, uint32_t row, double s) {
+  if (kind == kRunU) {
+    o.y[row] = fma(o.alpha, s, o.y[row]);
+  } else {  // an atom's first (a merged one: only) block
+    double v = o.alpha * s;
+    if (o.beta != 0.0) v = fma(o.beta, o.yin[row], v);
+    o.y[row] = v;
+  }
 }
 
 // ---- block-sum warp: for every block end of every pass, in order, wait
@@ -211,10 +229,11 @@ __device__ __forceinline__ bool block_end(double t0, double t1, uint32_t &nb, co
 // alpha*s (the atom's D block was summed before, in this same order) --
 // then free the slot.  After the pass's last P block it signals pdone (the
 // CTA's zbu rows are complete), after the pass's last block rdone.
-template <class Outs>  // outs(pass): where that pass's sums go
+template <int kPrec, class Outs>  // outs(pass): where that pass's sums go
 __device__ __forceinline__ void sum_warp(uint32_t nr, uint32_t npass, uint32_t nblk_p, Outs outs, const Smem &sm,
                                          int *err, uint64_t tmo) {
-  const int lane = threadIdx.x & 31;
+  constexpr int kGroups = groups_of<kPrec>(), kGroupWarps = NW / kGroups;
+  const uint32_t lane = threadIdx.x & 31;
   uint32_t nb = 0;
   for (uint32_t pass = 0; pass < npass; ++pass) {
     const PassOut o = outs(pass);
@@ -240,20 +259,35 @@ __device__ __forceinline__ void sum_warp(uint32_t nr, uint32_t npass, uint32_t n
       }
       const uint32_t kind = L.flags & 0xffu;
       const double *rb = sm.red + slot * (NW * 64);
-      for (uint32_t i = lane; i < L.nrow; i += 32) {
-        double s = rb[i];
-#pragma unroll
-        for (int k = 1; k < NW; ++k) s += rb[k * 64 + i];
-        const uint32_t row = L.out + i;
+      if constexpr (kPrec == kFP64) {
+        for (uint32_t i = lane; i < L.nrow; i += 32) {
+          const double s = warp_order_sum<NW>(rb + i);
+          if (kind == kRunP) o.zbu[L.out + i] = s;
+          else put_row(o, kind, L.out + i, s);
+        }
+      } else {
+        // a block of one run has sums of that run's group alone
+        const bool single = L.flags & kFirst;
+        if (single) rb += (pass * nr + r) % kGroups * (kGroupWarps * 64);
+        auto total = [&](uint32_t i) {
+          double s = warp_order_sum<kGroupWarps>(rb + i);
+          if (!single)
+            for (int k = kGroupWarps; k < NW; ++k) s += rb[k * 64 + i];
+          return s;
+        };
         if (kind == kRunP) {
-          o.zbu[row] = s;
-          if (o.zbu32) o.zbu32[row] = (float)s;
-        } else if (kind == kRunD || kind == kRunDU) {  // an atom's first (a merged one: only) block
-          double v = o.alpha * s;
-          if (o.beta != 0.0) v = fma(o.beta, o.yin[row], v);
-          o.y[row] = v;
+          float *z = o.zbu32 + L.out;  // U runs gather the float copy alone
+          const double s0 = total(lane);
+          if (L.nrow > 32) {
+            const double s1 = total(lane + 32);
+            z[lane] = (float)s0;
+            if (lane + 32 < L.nrow) z[lane + 32] = (float)s1;
+          } else if (lane < L.nrow) {
+            z[lane] = (float)s0;
+          }
         } else {
-          o.y[row] = fma(o.alpha, s, o.y[row]);
+          const double s = total(lane);
+          if (lane < L.nrow) put_row(o, kind, L.out + lane, s);
         }
       }
       ++nb;
@@ -276,6 +310,13 @@ __device__ __forceinline__ void sum_warp(uint32_t nr, uint32_t npass, uint32_t n
 // sums for the block-sum warp.  Before it can block, a warp gives back every
 // ring chunk below the run it is about to process, so no wait holds a chunk
 // another warp needs.  nb counts the block ends over the launch.
+//
+// A run costs every warp that takes part in it some 300 instructions beside
+// its panels (the waits, the ring's bookkeeping, the parking), which bounds the
+// FP32 and BF16 kernels; there a warp has nothing to do with the other group's
+// runs, unless a block has runs of both.  (With every warp parking at every
+// block end a BiCGSTAB step took 78.2 us instead of 75.1 at 9,999 rows of leaf
+// size 15 in FP32, 71.5 instead of 69.0 in BF16, 265 instead of 258 at 81,920.)
 template <int kPrec>
 __device__ __forceinline__ void consume_pass(Ring &R, uint32_t K, uint32_t nr, uint32_t &nb, uint32_t pass,
                                              const Smem &sm, int *err, uint64_t tmo) {
@@ -288,8 +329,9 @@ __device__ __forceinline__ void consume_pass(Ring &R, uint32_t K, uint32_t nr, u
   for (uint32_t r = 0; r < nr; ++r) {
     const RunLite L = sm.lite[r];
     const uint32_t g = pass * nr + r, slot = g % kStages;
-    R.release_below(R.base + (L.pos >> kChunkLog));
-    if (kGroups == 1 || g % kGroups == grp) {  // a run of this warp's group (the other group's: parking only)
+    const bool own = kGroups == 1 || g % kGroups == grp;  // a run of this warp's group
+    if (own) {
+      R.release_below(R.base + (L.pos >> kChunkLog));
       // Every warp of the group observes every phase of the slot's barrier,
       // panels or not: a warp that skipped phases could take an older
       // completed phase for the one it waits on.
@@ -303,9 +345,13 @@ __device__ __forceinline__ void consume_pass(Ring &R, uint32_t K, uint32_t nr, u
       if (lane == 0) mbar_arrive(&sm.sempty[slot]);
     }
     if (L.flags & kLast) {
-      R.release_below(R.base + ((L.pos + 16u * L.nrow * L.npanel) >> kChunkLog));
-      if (bad) ++nb;
-      else if (!block_end(t0, t1, nb, sm, err, tmo)) bad = true;
+      // A block of one run concerns its group alone, which arrives for the others.
+      const bool single = kGroups > 1 && (L.flags & kFirst);
+      if (!single || own) {
+        R.release_below(R.base + ((L.pos + 16u * L.nrow * L.npanel) >> kChunkLog));
+        if (!bad && !block_end(t0, t1, nb, single ? kGroups : 1, sm, err, tmo)) bad = true;
+      }
+      ++nb;
       t0 = 0.0;
       t1 = 0.0;
     }
@@ -371,7 +417,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_matvec(MatvecArgs a) {
     return;
   }
   if (w == kSumWarp) {
-    sum_warp(nr, 1, ci.nblk_p,
+    sum_warp<kPrec>(nr, 1, ci.nblk_p,
              [&](uint32_t) { return PassOut{a.alpha, a.beta, a.yin, a.y, a.zbu, kF32 ? a.zbu32 : nullptr}; }, sm, a.err,
              a.timeout_ns);
     return;
@@ -655,7 +701,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_bicg_steps(BicgArgs a) {
   // The two H-matvecs of a step write separate zbu copies: a CTA may still
   // gather the first's when another writes the second's.
   if (w == kSumWarp) {
-    sum_warp(nr, npass, ci.nblk_p,
+    sum_warp<kPrec>(nr, npass, ci.nblk_p,
              [&](uint32_t pass) {
                const size_t z = (pass & 1) ? a.zbu_len : 0;
                return PassOut{1.0, 0.0, nullptr, (pass & 1) ? a.at : a.ap, a.zbu + z, kF32 ? a.zbu32 + z : nullptr};
