@@ -184,12 +184,49 @@ cudaError_t mv_launch(hbx_hmat *h, const hbx::MatvecArgs &a, cudaStream_t s) {
   return hbx::launch_matvec(a, h->num_ctas, s, h->plan.precision);
 }
 
+// Page-locked staging of short host vectors (none above kIoBytes).
+int ensure_pin(hbx_hmat *h) {
+  const size_t n = (size_t)h->plan.nd;
+  if (!h->h_pin && n * sizeof(double) <= hbx::kIoBytes)
+    HBX_CUDA(cudaHostAlloc(&h->h_pin, (2 * n + 1) * sizeof(double), cudaHostAllocDefault));
+  return HBX_OK;
+}
+
+// a (and b, or null) to the device vectors da and db, on stream s; the host
+// vectors may change once this has returned.
+int host_in(hbx_hmat *h, const double *a, double *da, const double *b, double *db, cudaStream_t s) {
+  const size_t n = (size_t)h->plan.nd, bytes = n * sizeof(double);
+  if (!h->h_pin) {
+    HBX_CUDA(cudaMemcpyAsync(da, a, bytes, cudaMemcpyHostToDevice, s));
+    if (b) HBX_CUDA(cudaMemcpyAsync(db, b, bytes, cudaMemcpyHostToDevice, s));
+    return HBX_OK;
+  }
+  std::memcpy(h->h_pin, a, bytes);
+  if (b) std::memcpy(h->h_pin + n, b, bytes);
+  HBX_CUDA(hbx::launch_copy(h->h_pin, da, b ? h->h_pin + n : nullptr, db, nullptr, nullptr, n, s));
+  return HBX_OK;
+}
+
+// The device vector da to a, and the device error word's check; waits for s.
+int host_out(hbx_hmat *h, const double *da, double *a, cudaStream_t s) {
+  const size_t n = (size_t)h->plan.nd, bytes = n * sizeof(double);
+  if (!h->h_pin) {
+    HBX_CUDA(cudaMemcpyAsync(a, da, bytes, cudaMemcpyDeviceToHost, s));
+    HBX_CUDA(cudaStreamSynchronize(s));
+    return check_device_error(h, s);
+  }
+  int *err = reinterpret_cast<int *>(h->h_pin + 2 * n);
+  HBX_CUDA(hbx::launch_copy(da, h->h_pin, nullptr, nullptr, h->d_err, err, n, s));
+  HBX_CUDA(cudaStreamSynchronize(s));
+  std::memcpy(a, h->h_pin, bytes);
+  return *err ? check_device_error(h, s) : HBX_OK;
+}
+
 int ensure_host_staging(hbx_hmat *h) {
   const size_t n = (size_t)h->plan.nd;
   if (!h->d_x) HBX_CUDA(dev_malloc(&h->d_x, n * sizeof(double)));
   if (!h->d_y) HBX_CUDA(dev_malloc(&h->d_y, n * sizeof(double)));
-  if (!h->h_pin) HBX_CUDA(cudaHostAlloc(&h->h_pin, 2 * n * sizeof(double), cudaHostAllocDefault));
-  return HBX_OK;
+  return ensure_pin(h);
 }
 
 int ensure_solver(hbx_hmat *h, int max_iter) {
@@ -700,22 +737,19 @@ int hbx_matvec_host(hbx_hmat *h, const double *zu, double *zau, int accumulate, 
   if (int rc = single_rhs(h, "hbx_matvec_host")) return rc;
   int st = ensure_host_staging(h);
   if (st != HBX_OK) return st;
-  const size_t n = (size_t)h->plan.nd, bytes = n * sizeof(double);
   cudaStream_t s = h->stream;
   const double t0 = now_s();
-  HBX_CUDA(cudaMemcpyAsync(h->d_x, zu, bytes, cudaMemcpyHostToDevice, s));
-  if (accumulate) HBX_CUDA(cudaMemcpyAsync(h->d_y, zau, bytes, cudaMemcpyHostToDevice, s));
+  if ((st = host_in(h, zu, h->d_x, accumulate ? zau : nullptr, h->d_y, s)) != HBX_OK) return st;
   HBX_CUDA(cudaEventRecord(h->ev0, s));
   HBX_CUDA(mv_launch(h, matvec_args(h, 1.0, h->d_x, accumulate ? 1.0 : 0.0, h->d_y, h->d_y), s));
   HBX_CUDA(cudaEventRecord(h->ev1, s));
-  HBX_CUDA(cudaMemcpyAsync(zau, h->d_y, bytes, cudaMemcpyDeviceToHost, s));
-  HBX_CUDA(cudaStreamSynchronize(s));
+  st = host_out(h, h->d_y, zau, s);
   const double t1 = now_s();
   float ms = 0.f;
   cudaEventElapsedTime(&ms, h->ev0, h->ev1);
   if (kernel_seconds) *kernel_seconds += ms * 1e-3;
   if (copy_seconds) *copy_seconds += (t1 - t0) - ms * 1e-3;
-  return check_device_error(h, s);
+  return st;
 }
 
 static hbx::BicgArgs bicg_args(hbx_hmat *h, const double *b, double *u, double tol, int max_iter) {

@@ -259,6 +259,15 @@ cudaError_t launch_bicg_setup(const BicgArgs &a, int num_ctas, cudaStream_t s);
 cudaError_t launch_bicg_steps(const BicgArgs &a, int num_ctas, cudaStream_t s, int precision);
 cudaError_t launch_axpy(double alpha, const double *x, double *y, size_t n, cudaStream_t s);
 cudaError_t launch_to_float(const double *x, float *y, size_t n, cudaStream_t s);
+// n doubles of a0 to b0 and (when a1 is set) of a1 to b1, and (when w is set) the
+// word *w to *wout; either side may be page-locked host memory.
+cudaError_t launch_copy(const double *a0, double *b0, const double *a1, double *b1, const int *w, int *wout, size_t n,
+                        cudaStream_t s);
+// Host vectors up to this size go through page-locked memory and the copy
+// kernel, longer ones by the runtime's copies of pageable memory.  y += H x with
+// host vectors, the runtime's copies -> this: 81 KB 134 -> 99 us, 640 KB 442 ->
+// 358, 4 MB 1,440 -> 1,300; 16 MB 5,700 -> 6,220 (one core copies the vectors).
+constexpr size_t kIoBytes = 4 << 20;
 // The slot's partials of x.y over own rows; then out[0] = the total (one block).
 cudaError_t launch_dot(const BicgArgs &a, const double *x, const double *y, int slot, double *out,
                        int num_ctas, cudaStream_t s);
@@ -323,7 +332,7 @@ struct hbx_hmat {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr, ev3 = nullptr, ev4 = nullptr, ev5 = nullptr;
   // host-vector staging
   double *d_x = nullptr, *d_y = nullptr;
-  double *h_pin = nullptr;        // pinned staging, 2*nd doubles
+  double *h_pin = nullptr;        // page-locked staging of short host vectors: 2*nd doubles and the error word
   // solver workspace
   double *d_work = nullptr;       // r, rh, p, ap, t, at, b, u  (8*nd)
   double *d_part = nullptr;

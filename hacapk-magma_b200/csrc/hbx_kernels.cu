@@ -33,6 +33,8 @@
 #include "hbx_device.cuh"
 #include "hbx_engine.h"
 
+#include <algorithm>
+
 namespace hbx {
 namespace {
 
@@ -944,6 +946,20 @@ __global__ void k_to_float(const double *x, float *y, size_t n) {
     y[i] = (float)x[i];
 }
 
+// Short host vectors to the device and back: PCIe latency bounds it.  A copy of
+// pageable memory by the runtime takes 15 us and more (81 KB); through page-locked
+// memory, read and written across PCIe by this kernel, both vectors of a call and
+// the error word take one launch each way.
+__global__ void k_copy(const double *a0, double *b0, const double *a1, double *b1, const int *w, int *wout, size_t n) {
+  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
+  for (size_t k = i; k < n; k += stride) {
+    const double v = a0[k];
+    if (a1) b1[k] = a1[k];
+    b0[k] = v;
+  }
+  if (w && i == 0) *wout = *w;
+}
+
 // y += a * x (the refinement update of the mixed-precision solve).
 __global__ void k_axpy(double a, const double *x, double *y, size_t n) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
@@ -1009,6 +1025,13 @@ cudaError_t launch_matvec(const MatvecArgs &a, int num_ctas, cudaStream_t s, int
 
 cudaError_t launch_to_float(const double *x, float *y, size_t n, cudaStream_t s) {
   k_to_float<<<296, 256, 0, s>>>(x, y, n);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_copy(const double *a0, double *b0, const double *a1, double *b1, const int *w, int *wout, size_t n,
+                        cudaStream_t s) {
+  const unsigned blocks = (unsigned)std::min<size_t>(148, (n + 255) / 256);
+  k_copy<<<std::max(1u, blocks), 256, 0, s>>>(a0, b0, a1, b1, w, wout, n);
   return cudaGetLastError();
 }
 
