@@ -789,12 +789,16 @@ static hbx::BicgArgs bicg_args(hbx_hmat *h, const double *b, double *u, double t
 }
 
 // BiCGSTAB on device vectors b, u (u: x0 in / solution out), all on h->stream.
+// Steps of one launch, at most: a CTA counts its chunks and runs over the
+// launch's passes in 32 bits (256 steps of a CTA with 1 GB of factors: 2^24).
+static constexpr int kLaunchSteps = 256;
+
 static int bicgstab_dev(hbx_hmat *h, const double *b, double *u, const hbx_solve_opts *opts, hbx_solve_info *info) {
   if (int rc = single_rhs(h, "hbx_bicgstab")) return rc;
   const double tol = opts ? opts->tol : 1e-8;
   const int max_iter = opts ? opts->max_iter : 1000;
   const int verbose = opts ? opts->verbose : 0;
-  int batch = (opts && opts->batch > 0) ? opts->batch : 8;
+  int batch = (opts && opts->batch > 0) ? std::min(opts->batch, kLaunchSteps) : 8;
   if (max_iter < 0 || !(tol >= 0.0)) return fail(HBX_ERR_INVALID, "hbx_bicgstab: bad tol or max_iter");
   int st = ensure_solver(h, max_iter);
   if (st != HBX_OK) return st;
@@ -896,8 +900,11 @@ int hbx_bicgstab_host(hbx_hmat *h, const double *b, double *u, const hbx_solve_o
 
 // Pipelined BiCGSTAB of c_hacapk_bicgstab_cax_lfmtx_pipe_ (HACApK_SOLVER_PIPE.c:144-600)
 // on device vectors, on h->stream: three products and k_pipe_init, then
-// batches of steps (k_pipe_a, v = H z, k_pipe_b, t = H w) as one captured
-// graph, the device state read back after each batch.
+// batches of steps, the device state read back after each.  FP64 engines up to
+// pipe_steps_max_rows run a batch as one launch (k_pipe_steps) and queue the
+// next while the state is read; the others run it as a captured graph of
+// k_pipe_a, v = H z, k_pipe_b, t = H w (FP32 and BF16 products convert their
+// input in a launch of its own).
 static int pipe_graph(hbx_hmat *h, const hbx::PipeVecs &v, int batch) {
   if (h->pgraph && h->pgraph_batch == batch && h->pgraph_key == v.u) return HBX_OK;
   if (h->pgraph) {
@@ -942,7 +949,7 @@ static int pipe_dev(hbx_hmat *h, const double *b, double *u, const hbx_solve_opt
   const double tol = opts ? opts->tol : 1e-8;
   const int max_iter = opts ? opts->max_iter : 1000;
   const int verbose = opts ? opts->verbose : 0;
-  const int batch = (opts && opts->batch > 0) ? opts->batch : 8;
+  const int batch = (opts && opts->batch > 0) ? std::min(opts->batch, kLaunchSteps) : 8;
   if (max_iter < 0 || !(tol >= 0.0)) return fail(HBX_ERR_INVALID, "hbx_bicgstab_pipe: bad tol or max_iter");
   const size_t n = (size_t)h->plan.nd;
   if (!h->d_pipe) HBX_CUDA(dev_malloc(&h->d_pipe, (size_t)hbx::kPipeVecs * n * sizeof(double)));
@@ -950,7 +957,7 @@ static int pipe_dev(hbx_hmat *h, const double *b, double *u, const hbx_solve_opt
     HBX_CUDA(dev_malloc(&h->d_pstate, sizeof(hbx::PipeState)));
     HBX_CUDA(cudaMemset(h->d_pstate, 0, sizeof(hbx::PipeState)));
   }
-  if (!h->h_pstate) HBX_CUDA(cudaHostAlloc(&h->h_pstate, sizeof(hbx::PipeState), cudaHostAllocDefault));
+  if (!h->h_pstate) HBX_CUDA(cudaHostAlloc(&h->h_pstate, 2 * sizeof(hbx::PipeState), cudaHostAllocDefault));
   if (!h->d_ppart) HBX_CUDA(dev_malloc(&h->d_ppart, (size_t)hbx::gcr_dot_blocks(n) * hbx::kMaxDots * 2 * sizeof(double)));
   if (h->phist_cap < max_iter + 1) {
     if (h->pgraph) {  // the captured steps write the history being replaced
@@ -973,40 +980,79 @@ static int pipe_dev(hbx_hmat *h, const double *b, double *u, const hbx_solve_opt
   HBX_CUDA(mv_launch(h, matvec_args(h, 1.0, v.r, 0.0, nullptr, v.w), s));
   HBX_CUDA(mv_launch(h, matvec_args(h, 1.0, v.w, 0.0, nullptr, v.t), s));
   HBX_CUDA(hbx::pipe_launch_init(v, n, h->d_pstate, h->d_ppart, h->d_phist, tol, max_iter, s));
-  HBX_CUDA(cudaMemcpyAsync(h->h_pstate, h->d_pstate, sizeof(hbx::PipeState), cudaMemcpyDeviceToHost, s));
-  HBX_CUDA(cudaStreamSynchronize(s));
-  const bool use_graph = !h->h_pstate->done && pipe_graph(h, v, batch) == HBX_OK;
-  int launched = 0;
+  const bool fused = h->plan.precision == hbx::kFP64 && n <= hbx::pipe_steps_max_rows(h->num_ctas);
+  long long launched = 0;  // steps
+  int launches = 0, seen = 0;
   double iter_s = 0.0;
-  while (!h->h_pstate->done && launched <= max_iter + batch) {
-    HBX_CUDA(cudaEventRecord(h->ev3, s));
-    if (use_graph) {
-      HBX_CUDA(cudaGraphLaunch(h->pgraph, s));
-    } else {
-      for (int i = 0; i < batch; ++i) {
-        hbx::MatvecArgs av = matvec_args(h, 1.0, v.z, 0.0, nullptr, v.v);
-        av.skip = &h->d_pstate->done;
-        hbx::MatvecArgs at = matvec_args(h, 1.0, v.w, 0.0, nullptr, v.t);
-        at.skip = &h->d_pstate->done;
-        HBX_CUDA(hbx::pipe_launch_a(v, n, h->d_pstate, h->d_ppart, s));
-        HBX_CUDA(mv_launch(h, av, s));
-        HBX_CUDA(hbx::pipe_launch_b(v, n, h->d_pstate, h->d_ppart, h->d_phist, s));
-        HBX_CUDA(mv_launch(h, at, s));
-      }
+  if (fused) {
+    hbx::PipeStepArgs a{};
+    a.stream = h->d_stream;
+    a.recs = h->d_recs;
+    a.ctas = h->d_ctas;
+    a.lite = h->d_lite;
+    a.zbu = h->d_zbu;
+    a.zbu_len = h->plan.zbu_len;
+    a.gbar = h->d_gbar;
+    a.err = h->d_err;
+    a.timeout_ns = h->timeout_ns;
+    a.keep_frac = h->keep_frac;
+    a.v = v;
+    a.n = n;
+    a.st = h->d_pstate;
+    a.part = h->d_ppart;
+    a.hist = h->d_phist;
+    a.steps = batch;
+    cudaEvent_t read[2] = {h->ev3, h->ev4};
+    HBX_CUDA(cudaEventRecord(h->ev5, s));
+    for (;;) {
+      const int k = launches & 1;
+      HBX_CUDA(hbx::launch_pipe_steps(a, h->num_ctas, s));
+      HBX_CUDA(cudaMemcpyAsync(&h->h_pstate[k], h->d_pstate, sizeof(hbx::PipeState), cudaMemcpyDeviceToHost, s));
+      HBX_CUDA(cudaEventRecord(read[k], s));
+      launched += batch;
+      if (launches++ == 0) continue;
+      seen = k ^ 1;
+      HBX_CUDA(cudaEventSynchronize(read[seen]));
+      if (h->h_pstate[seen].done || launched - 2 * (long long)batch > max_iter) break;
     }
-    HBX_CUDA(cudaEventRecord(h->ev4, s));
-    launched += batch;
+    float its = 0.f;
+    cudaEventElapsedTime(&its, h->ev5, read[seen]);
+    iter_s = its * 1e-3;
+  } else {
     HBX_CUDA(cudaMemcpyAsync(h->h_pstate, h->d_pstate, sizeof(hbx::PipeState), cudaMemcpyDeviceToHost, s));
     HBX_CUDA(cudaStreamSynchronize(s));
-    float bms = 0.f;
-    cudaEventElapsedTime(&bms, h->ev3, h->ev4);
-    iter_s += bms * 1e-3;
-    int derr = 0;
-    HBX_CUDA(cudaMemcpy(&derr, h->d_err, sizeof(int), cudaMemcpyDeviceToHost));
-    if (derr) break;
+    const bool use_graph = !h->h_pstate->done && pipe_graph(h, v, batch) == HBX_OK;
+    while (!h->h_pstate->done && launched <= max_iter + batch) {
+      HBX_CUDA(cudaEventRecord(h->ev3, s));
+      if (use_graph) {
+        HBX_CUDA(cudaGraphLaunch(h->pgraph, s));
+      } else {
+        for (int i = 0; i < batch; ++i) {
+          hbx::MatvecArgs av = matvec_args(h, 1.0, v.z, 0.0, nullptr, v.v);
+          av.skip = &h->d_pstate->done;
+          hbx::MatvecArgs at = matvec_args(h, 1.0, v.w, 0.0, nullptr, v.t);
+          at.skip = &h->d_pstate->done;
+          HBX_CUDA(hbx::pipe_launch_a(v, n, h->d_pstate, h->d_ppart, s));
+          HBX_CUDA(mv_launch(h, av, s));
+          HBX_CUDA(hbx::pipe_launch_b(v, n, h->d_pstate, h->d_ppart, h->d_phist, s));
+          HBX_CUDA(mv_launch(h, at, s));
+        }
+      }
+      HBX_CUDA(cudaEventRecord(h->ev4, s));
+      launched += batch;
+      HBX_CUDA(cudaMemcpyAsync(h->h_pstate, h->d_pstate, sizeof(hbx::PipeState), cudaMemcpyDeviceToHost, s));
+      HBX_CUDA(cudaStreamSynchronize(s));
+      float bms = 0.f;
+      cudaEventElapsedTime(&bms, h->ev3, h->ev4);
+      iter_s += bms * 1e-3;
+      int derr = 0;
+      HBX_CUDA(cudaMemcpy(&derr, h->d_err, sizeof(int), cudaMemcpyDeviceToHost));
+      if (derr) break;
+    }
+    launches = (int)(4 * launched);
   }
   HBX_CUDA(cudaEventRecord(h->ev1, s));
-  const hbx::PipeState S = *h->h_pstate;
+  const hbx::PipeState S = h->h_pstate[seen];
   // true residual ||b - H u||, in v.v (no longer needed)
   HBX_CUDA(mv_launch(h, matvec_args(h, -1.0, u, 1.0, b, v.v), s));
   const double *xs[1] = {v.v}, *ys[1] = {v.v};
@@ -1026,8 +1072,8 @@ static int pipe_dev(hbx_hmat *h, const double *b, double *u, const hbx_solve_opt
     info->true_relres = S.bnorm > 0 ? std::sqrt(tr2) / S.bnorm : std::sqrt(tr2);
     info->seconds = ms * 1e-3;
     info->iter_kernel_seconds = iter_s;
-    info->iter_launches = 4 * launched;
-    info->launches = 4 * launched + 7;  // 3 setup products, init, residual product, two dot kernels
+    info->iter_launches = fused ? S.step : launches;
+    info->launches = launches + 7;  // 3 setup products, init, residual product, two dot kernels
   }
   if (verbose > 0) {
     std::vector<double> hist(S.step + 1, 0.0);

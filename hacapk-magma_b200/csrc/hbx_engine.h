@@ -235,6 +235,33 @@ cudaError_t pipe_launch_init(const PipeVecs &v, size_t n, PipeState *st, double 
 cudaError_t pipe_launch_a(const PipeVecs &v, size_t n, PipeState *st, double *part, cudaStream_t s);
 cudaError_t pipe_launch_b(const PipeVecs &v, size_t n, PipeState *st, double *part, double *hist, cudaStream_t s);
 
+// FP64 engines: up to `steps` steps in one launch (k_pipe_steps, hbx_kernels.cu).
+struct PipeStepArgs {
+  const uint8_t *stream;
+  const RunRec *recs;
+  const CtaInfo *ctas;
+  const RunLite *lite;
+  double *zbu;  // [2][zbu_len]: one copy per product of a step
+  uint64_t zbu_len;
+  unsigned *gbar;
+  int *err;
+  unsigned long long timeout_ns;
+  uint32_t keep_frac;
+  PipeVecs v;
+  size_t n;
+  PipeState *st;
+  double *part, *hist;
+  int nvb;  // blocks of the dots' grid (set by the launcher)
+  int steps;
+};
+cudaError_t launch_pipe_steps(PipeStepArgs a, int num_ctas, cudaStream_t s);
+// Up to this many rows a thread of k_pipe_steps has one element (two blocks of
+// the dots' grid per CTA: 75,776 rows on 148 CTAs).  Beyond, the products are
+// most of a step and the stand-alone vector kernels, with four times the warps,
+// stream better (with several elements per thread a solve of 81,920 rows took
+// 19.6 ms either way, of 327,680 114.1 ms in k_pipe_steps and 112.2 as launches).
+inline size_t pipe_steps_max_rows(int num_ctas) { return (size_t)num_ctas * 512; }
+
 // Static scratch of hbx_matvec_noalloc (hbx_kernels.cu): 256 bytes of
 // barrier words, then room for kNoallocZbuMax zbu doubles.
 constexpr size_t kNoallocScratchBytes = size_t(1) << 20;

@@ -5,6 +5,7 @@
 //               phase, no atomics, no zeroing of zbu/zau).
 // k_bicg_setup  r = b - H u has been formed by k_matvec; sets rh = r, p = Ap = 0
 //               and the first reduction partials (HACApK_SOLVER.c:533-594).
+// k_pipe_steps  pipelined BiCGSTAB steps (hbx_pipe.cu), several in one launch.
 // k_bicg_steps  BiCGSTAB steps of HACApK_SOLVER.c:602-732, several in one
 //               launch: both H-matvecs, the vector updates and all dot
 //               products, with compensated (Dot2) partial sums reduced in a
@@ -31,6 +32,7 @@
 // complete) use a bounded grid barrier; the launch is cooperative so every
 // CTA is resident.
 #include "hbx_device.cuh"
+#include "hbx_dots.cuh"
 #include "hbx_engine.h"
 
 #include <algorithm>
@@ -39,7 +41,7 @@ namespace hbx {
 namespace {
 
 constexpr int NW = kConsumerWarps;
-[[maybe_unused]] constexpr int kConsumerThreads = NW * 32;
+constexpr int kConsumerThreads = NW * 32;
 // Consumer groups: the FP32 and BF16 product kernels split their warps into
 // kProductGroups groups taking alternate runs; the FP64 product (whose
 // summation order the drop-in's iteration counts follow, and which a CPU
@@ -383,6 +385,25 @@ __device__ __forceinline__ uint32_t keep_bytes(uint32_t stream_bytes, uint32_t k
   return r > 0xffffffffull ? 0xffffffffu : (uint32_t)r;
 }
 
+// Grid-barrier instance k of the launch for this CTA, by one whole warp.
+__device__ __forceinline__ void arrive_and_wait(unsigned *gbar, unsigned k, int *err, uint64_t timeout_ns,
+                                                const Smem &sm) {
+  const unsigned target = grid_target(sm.rsum[1], k, gridDim.x);
+  if ((threadIdx.x & 31) == 0) grid_arrive(gbar, target);
+  __syncwarp();
+  if (!grid_wait_warp(gbar, target, timeout_ns) && (threadIdx.x & 31) == 0) atomicOr(err, kErrGridBarrier);
+}
+
+// Full grid barrier (instance k of the launch) among the consumer warps of
+// every CTA: what their threads wrote before it is read after it (bar.sync,
+// then the arriving thread's release; no fence of their own).
+__device__ __forceinline__ void grid_sync(unsigned *gbar, unsigned k, int *err, uint64_t timeout_ns, const Smem &sm) {
+  named_bar(1, kConsumerThreads);
+  if (threadIdx.x < 32) arrive_and_wait(gbar, k, err, timeout_ns, sm);
+  named_bar(1, kConsumerThreads);
+}
+
+
 // kPrec: storage precision of the factors; FP32 and BF16 engines gather the
 // float copies of the vectors.
 #ifndef HBX_STEP_TU
@@ -431,6 +452,273 @@ __global__ void __launch_bounds__(kThreads, 1) k_matvec(MatvecArgs a) {
   if (a.prof && threadIdx.x == 0) {
     a.prof[blockIdx.x * 16 + 0] = t_start;
     a.prof[blockIdx.x * 16 + 5] = gtimer();
+  }
+}
+
+// ---------------------------------------------------------- pipelined BiCGSTAB
+// Grid-barrier instances of one pipelined step, in order: z and the y.q, y.y
+// partials complete, zbu of v = H z, v, then w and its five partials, zbu of
+// t = H w, t.
+enum : unsigned {
+  kGridZ = 0, kGridPassV = 1, kGridV = 2, kGridW = 3, kGridPassT = 4, kGridT2 = 5, kGridPipeStep = 6
+};
+// Partials of dot j: slots [kPipeSlot + j][dot_blocks] of 16-byte pairs.
+constexpr int kPipeSlotA = 0, kPipeSlotB = 2;
+
+// The block partials of K dots in hbx_dots.cuh's order (blocks of kDotThreads
+// threads, an element per thread): eight consumer warps stand for block `vb`,
+// so the totals are those of the stand-alone kernels bit for bit.
+template <int K>
+__device__ __forceinline__ void pipe_partials(const PipeStepArgs &a, int slot0, uint32_t vb, Acc2 (&acc)[K], const Smem &sm) {
+  static_assert(NW == 2 * kDotThreads / 32, "two blocks of the dots' grid per CTA");
+  constexpr int kBlockWarps = kDotThreads / 32;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, wb = w % kBlockWarps;
+  double *sc = sm.red + w / kBlockWarps * (kBlockWarps * K * 2);  // free: every warp has waited for the block-sum warp
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    acc[k] = warp_merge(acc[k]);
+    if (lane == 0) {
+      sc[(wb * K + k) * 2 + 0] = acc[k].s;
+      sc[(wb * K + k) * 2 + 1] = acc[k].c;
+    }
+  }
+  named_bar(1, kConsumerThreads);
+  if (wb == 0 && lane < K && vb < (uint32_t)a.nvb) {
+    Acc2 t{sc[lane * 2], sc[lane * 2 + 1]};
+    for (int q = 1; q < kBlockWarps; ++q) t = acc2_merge(t, Acc2{sc[(q * K + lane) * 2], sc[(q * K + lane) * 2 + 1]});
+    reinterpret_cast<double2 *>(a.part)[(size_t)(slot0 + lane) * a.nvb + vb] = make_double2(t.s, t.c);
+  }
+}
+
+// pair_total of hbx_dots.cuh over a slot's partials (a whole warp), the loads
+// of five chunks of 32 under way together.
+__device__ __forceinline__ double pipe_total(const PipeStepArgs &a, int slot) {
+  constexpr int kBatch = 5;
+  const int lane = threadIdx.x & 31;
+  const double2 *part = reinterpret_cast<const double2 *>(a.part) + (size_t)slot * a.nvb;
+  Acc2 t{0.0, 0.0};
+  for (int b0 = 0; b0 < a.nvb; b0 += 32 * kBatch) {
+    Acc2 v[kBatch];
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k) {
+      const int b = b0 + 32 * k + lane;
+      v[k] = Acc2{0.0, 0.0};
+      if (b < a.nvb) {
+        const double2 x = __ldcg(part + b);
+        v[k] = Acc2{x.x, x.y};
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k)
+      if (b0 + 32 * k < a.nvb) t = acc2_merge(t, warp_merge(v[k]));
+  }
+  return t.s + t.c;
+}
+
+// Up to a.steps pipelined BiCGSTAB steps (the arithmetic and the summation
+// order of k_pipe_a, k_matvec, k_pipe_b, k_matvec: hbx_pipe.cu).  As four
+// launches a step paid four launch boundaries, two products with a cold ring
+// and two tickets on which the last block started its totals; here six grid
+// barriers take their place, the ring runs on through the vector work, and no
+// graph is captured for a new u.  An element is always the same thread's, so of
+// the vectors only v and t (written by rows), z and w (gathered) cross CTAs.
+// The early end of a launch is k_bicg_steps'.  Solves to 1e-8, launches -> this:
+// N = 320 430 -> 306 us, 1,280 715 -> 571, 5,120 1,250 -> 1,050, 6,001 (leaf size
+// 32, ragged) 1,814 -> 1,527, 20,480 3,660 -> 3,410 (60 products of 265 MB at 6.55
+// TB/s: 2,430; the six barriers of a step and the vector work: some 20 us).
+__global__ void __launch_bounds__(kThreads, 1) k_pipe_steps(const __grid_constant__ PipeStepArgs a) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  if (*(volatile const int *)&a.st->done) return;  // an earlier launch ended the solve
+  const CtaInfo ci = a.ctas[blockIdx.x];
+  const uint32_t nr = ci.nr_p + ci.nr_d + ci.nr_u;
+  const Smem sm = cta_smem(smem_raw, a.lite + ci.rec_begin, nr);
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t npass = 2u * (uint32_t)a.steps;
+  const StreamSrc ss{a.stream + ci.stream_off, ci.stream_bytes, keep_bytes(ci.stream_bytes, a.keep_frac)};
+  uint32_t issued0 = 0;
+  if (threadIdx.x == kProducerWarp * 32) issued0 = producer_start(ss, npass, sm.ring, sm.full, sm.empty);
+  init_cta(sm, a.lite + ci.rec_begin, nr, a.gbar, NW);
+  const uint32_t K = (ci.stream_bytes + kChunkBytes - 1) >> kChunkLog;
+  if (w == kProducerWarp) {
+    if (lane == 0 && K > 0)
+      producer_run(ss, npass, issued0, sm.ring, sm.full, sm.empty, a.err, a.timeout_ns, &sm.rsum[4]);
+    return;
+  }
+  const PipeVecs &v = a.v;
+  if (w >= kGatherWarp0 && w < kSyncWarp) {
+    const GatherCtx c{a.recs + ci.rec_begin, nr, ci.nr_p + ci.nr_d, npass, v.z, v.w, a.zbu, a.zbu + a.zbu_len, a.err,
+                      a.timeout_ns};
+    gather_warp<kFP64>(c, sm, (uint32_t)(w - kGatherWarp0));
+    return;
+  }
+  if (w == kSyncWarp) {
+    if (lane == 0) sync_warp(a.gbar, npass, kGridPassV, kGridPassT, kGridPipeStep, sm, a.err, a.timeout_ns);
+    return;
+  }
+  if (w == kSumWarp) {
+    sum_warp<kFP64>(nr, npass, ci.nblk_p,
+                    [&](uint32_t pass) {
+                      return PassOut{1.0, 0.0, nullptr, (pass & 1) ? v.t : v.v, a.zbu + ((pass & 1) ? a.zbu_len : 0),
+                                     nullptr};
+                    },
+                    sm, a.err, a.timeout_ns);
+    return;
+  }
+  // scal: alpha, beta, zeta, r.r0, done, steps taken; [8..12] the five totals
+  enum { kAlpha = 0, kBeta, kZeta, kZnorm, kDone, kStep, kTot = 8 };
+  Ring R{sm.ring, sm.full, sm.empty, 0, 0, 0, a.timeout_ns, a.err, false};
+  uint32_t nb = 0;
+  if (threadIdx.x == 0) {
+    sm.scal[kAlpha] = __ldcg(&a.st->alpha);
+    sm.scal[kBeta] = __ldcg(&a.st->beta);
+    sm.scal[kZeta] = __ldcg(&a.st->zeta);
+    sm.scal[kZnorm] = __ldcg(&a.st->znorm);
+    sm.scal[kStep] = (double)__ldcg(&a.st->step);  // (state is written after the first grid barrier)
+    sm.scal[kDone] = *(volatile const int *)a.err ? 1.0 : 0.0;  // an earlier wait ran out
+  }
+  named_bar(1, kConsumerThreads);
+  // The launch's later passes do not follow: wake the warps that wait for one.
+  auto stop = [&]() {
+    if (threadIdx.x == 0) {
+      st_release_s(&sm.rsum[4], 1u);
+      signal_xready(sm, 0x7ffffffeu);
+    }
+    named_bar(1, kConsumerThreads);
+    if (lane == 0) mbar_arrive(&sm.empty[R.released % kRingChunks]);
+  };
+  auto finish = [&](int status) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      a.st->status = status;
+      a.st->done = 1;
+    }
+  };
+  if (sm.scal[kDone] != 0.0) {
+    // done stays unset: a CTA that has yet to start must come this way too
+    stop();
+    return;
+  }
+  auto mul = [](double x, double y) { return __dmul_rn(x, y); };
+  auto add = [](double x, double y) { return __dadd_rn(x, y); };
+
+  // One product per turn, its call in one place: the loop over the panels keeps
+  // the registers that it has in k_matvec when little else is live.  (Called in
+  // two places, or as a function, it spilled inside the runs: 81,920 rows 21.7 and
+  // 22.6 ms instead of 19.6.)
+  for (uint32_t pass = 0; pass < npass; ++pass) {
+    const unsigned k0 = (pass >> 1) * kGridPipeStep;
+    // (volatile: kept live through the product, the element's index and
+    // addresses spill inside the loop over the panels)
+    uint32_t tid;
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid));
+    const uint32_t vb = blockIdx.x + (tid >= kConsumerThreads / 2 ? gridDim.x : 0u);
+    const uint32_t i = vb * kDotThreads + tid % kDotThreads;
+    const bool own = i < (uint32_t)a.n;
+    if ((pass & 1u) == 0) {
+      if (pass > 0) grid_sync(a.gbar, k0 - kGridPipeStep + kGridT2, a.err, a.timeout_ns, sm);
+      // p, s, z (copies on the first step), q, y; y.q, y.y.  (Reading ahead of
+      // the barrier gained nothing: the values spilled.)
+      Acc2 acc[2] = {{0.0, 0.0}, {0.0, 0.0}};
+      if (own) {
+        const double alpha = sm.scal[kAlpha], beta = sm.scal[kBeta], nzeta = -sm.scal[kZeta], t = __ldcg(&v.t[i]);
+        const double r = __ldcg(&v.r[i]), wv = __ldcg(&v.w[i]), vv = __ldcg(&v.v[i]);
+        double p = __ldcg(&v.p[i]), s = __ldcg(&v.s[i]), z = __ldcg(&v.z[i]);
+        if (sm.scal[kStep] == 0.0) {
+          p = r, s = wv, z = t;
+        } else {
+          p = add(mul(beta, add(p, mul(nzeta, s))), r);
+          s = add(mul(beta, add(s, mul(nzeta, z))), wv);
+          z = add(mul(beta, add(z, mul(nzeta, vv))), t);
+        }
+        const double q = add(r, mul(-alpha, s)), y = add(wv, mul(-alpha, z));
+        v.z[i] = z;
+        v.p[i] = p;
+        v.s[i] = s;
+        v.q[i] = q;
+        v.y[i] = y;
+        dot2_add(acc[0], y, q);
+        dot2_add(acc[1], y, y);
+      }
+      pipe_partials<2>(a, kPipeSlotA, vb, acc, sm);
+      grid_sync(a.gbar, k0 + kGridZ, a.err, a.timeout_ns, sm);
+      if (threadIdx.x == 0) signal_xready(sm, pass);
+      // zeta while the gathers start; a zeta that is not finite ends the solve
+      // after this product, before u changes
+      if (w < 2) {
+        const double d = pipe_total(a, kPipeSlotA + w);
+        if (lane == 0) sm.scal[kTot + w] = d;
+      }
+    } else {
+      grid_sync(a.gbar, k0 + kGridV, a.err, a.timeout_ns, sm);
+      const double alpha = sm.scal[kAlpha], zeta = __ddiv_rn(sm.scal[kTot], sm.scal[kTot + 1]);
+      if (blockIdx.x == 0 && threadIdx.x == 0) a.st->zeta = zeta;
+      if (!isfinite(zeta)) {  // y = 0 (HACApK_SOLVER_PIPE.c:433 divides unchecked)
+        finish(HBX_ERR_BREAKDOWN);
+        stop();
+        return;
+      }
+      // u, r, w; r.r0, w.r0, s.r0, z.r0, r.r
+      Acc2 acc[5] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
+      if (own) {
+        const double q = __ldcg(&v.q[i]), y = __ldcg(&v.y[i]), r0 = __ldcg(&v.r0[i]), t = __ldcg(&v.t[i]);
+        const double p = __ldcg(&v.p[i]), s = __ldcg(&v.s[i]), z = __ldcg(&v.z[i]), u = __ldcg(&v.u[i]);
+        const double wv = add(mul(-zeta, add(t, mul(-alpha, __ldcg(&v.v[i])))), y);
+        const double r = add(q, mul(-zeta, y));
+        v.w[i] = wv;
+        v.r[i] = r;
+        v.u[i] = add(add(u, mul(alpha, p)), mul(zeta, q));
+        dot2_add(acc[0], r, r0);
+        dot2_add(acc[1], wv, r0);
+        dot2_add(acc[2], s, r0);
+        dot2_add(acc[3], z, r0);
+        dot2_add(acc[4], r, r);
+      }
+      pipe_partials<5>(a, kPipeSlotB, vb, acc, sm);
+      grid_sync(a.gbar, k0 + kGridW, a.err, a.timeout_ns, sm);
+      if (w < 5) {
+        const double d = pipe_total(a, kPipeSlotB + w);
+        if (lane == 0) sm.scal[kTot + w] = d;
+      }
+      named_bar(1, kConsumerThreads);
+      if (threadIdx.x == 0) {
+        const int step = (int)sm.scal[kStep] + 1;
+        const double znorm = sm.scal[kTot];
+        const double beta = mul(__ddiv_rn(alpha, zeta), __ddiv_rn(znorm, sm.scal[kZnorm]));
+        const double den =
+            __dsub_rn(add(sm.scal[kTot + 1], mul(beta, sm.scal[kTot + 2])), mul(mul(beta, zeta), sm.scal[kTot + 3]));
+        const double alpha_new = __ddiv_rn(znorm, den);
+        const double bnorm = __ldcg(&a.st->bnorm);
+        const double rel = bnorm > 0.0 ? __ddiv_rn(__dsqrt_rn(sm.scal[kTot + 4]), bnorm) : 0.0;
+        int done = 1, status = HBX_OK;
+        if (*(volatile const int *)a.err) status = HBX_ERR_TIMEOUT;  // a wait ran out: no more of them
+        else if (rel < __ldcg(&a.st->tol)) status = HBX_OK;
+        else if (!isfinite(rel) || !isfinite(alpha_new) || !isfinite(beta)) status = HBX_ERR_BREAKDOWN;
+        else if (step >= __ldcg(&a.st->max_iter)) status = HBX_ERR_NOT_CONVERGED;
+        else done = 0;
+        sm.scal[kAlpha] = alpha_new;
+        sm.scal[kBeta] = beta;
+        sm.scal[kZeta] = zeta;
+        sm.scal[kZnorm] = znorm;
+        sm.scal[kDone] = done;
+        sm.scal[kStep] = (double)step;
+        if (blockIdx.x == 0) {
+          a.st->znorm = znorm;
+          a.st->beta = beta;
+          a.st->alpha = alpha_new;
+          a.st->relres = rel;
+          a.st->step = step;
+          a.hist[step] = rel;
+          if (done) finish(status);
+        }
+      }
+      named_bar(1, kConsumerThreads);
+      if (sm.scal[kDone] != 0.0) {
+        stop();
+        return;
+      }
+      if (threadIdx.x == 0) signal_xready(sm, pass);
+    }
+    R.base = pass * K;
+    matvec_pass<kFP64>(R, K, nr, nb, pass, ci.nblk_p, sm, a.err, a.timeout_ns);  // v = H z, then t = H w
   }
 }
 
@@ -556,24 +844,6 @@ __device__ __forceinline__ void reduce_slots(const double *part, int ncta, const
 enum : unsigned {
   kGridP = 0, kGridPass0 = 1, kGridAlpha = 2, kGridT = 3, kGridPass1 = 4, kGridZeta = 5, kGridEnd = 6, kGridStep = 7
 };
-
-// Grid-barrier instance k of the launch for this CTA, by one whole warp.
-__device__ __forceinline__ void arrive_and_wait(unsigned *gbar, unsigned k, int *err, uint64_t timeout_ns,
-                                                const Smem &sm) {
-  const unsigned target = grid_target(sm.rsum[1], k, gridDim.x);
-  if ((threadIdx.x & 31) == 0) grid_arrive(gbar, target);
-  __syncwarp();
-  if (!grid_wait_warp(gbar, target, timeout_ns) && (threadIdx.x & 31) == 0) atomicOr(err, kErrGridBarrier);
-}
-
-// Full grid barrier (instance k of the launch) among the consumer warps of
-// every CTA: what their threads wrote before it is read after it (bar.sync,
-// then the arriving thread's release; no fence of their own).
-__device__ __forceinline__ void grid_sync(unsigned *gbar, unsigned k, int *err, uint64_t timeout_ns, const Smem &sm) {
-  named_bar(1, kConsumerThreads);
-  if (threadIdx.x < 32) arrive_and_wait(gbar, k, err, timeout_ns, sm);
-  named_bar(1, kConsumerThreads);
-}
 
 // The CTA's compensated partials of NSL dots to slots slot0 + k, then
 // grid-barrier instance `inst`, all in warp 0 after one barrier of the CTA: the
@@ -995,6 +1265,7 @@ cudaError_t configure_kernels() {
   const int smem = (int)SharedLayout::bytes;
   cudaError_t e;
   if ((e = cudaFuncSetAttribute(k_matvec<kFP64>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
+  if ((e = cudaFuncSetAttribute(k_pipe_steps, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
   if ((e = cudaFuncSetAttribute(k_matvec<kFP32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
   if ((e = cudaFuncSetAttribute(k_matvec<kBF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
   return configure_step_kernels();
@@ -1021,6 +1292,11 @@ static cudaError_t launch_coop(void (*kern)(Args), const Args &a, int num_ctas, 
 cudaError_t launch_matvec(const MatvecArgs &a, int num_ctas, cudaStream_t s, int precision) {
   if (precision == kBF16) return launch_coop(k_matvec<kBF16>, a, num_ctas, s);
   return precision == kFP32 ? launch_coop(k_matvec<kFP32>, a, num_ctas, s) : launch_coop(k_matvec<kFP64>, a, num_ctas, s);
+}
+
+cudaError_t launch_pipe_steps(PipeStepArgs a, int num_ctas, cudaStream_t s) {
+  a.nvb = dot_blocks(a.n);
+  return launch_coop(k_pipe_steps, a, num_ctas, s);
 }
 
 cudaError_t launch_to_float(const double *x, float *y, size_t n, cudaStream_t s) {

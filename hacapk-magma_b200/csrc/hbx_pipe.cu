@@ -9,7 +9,9 @@
 // count, done/status) stays on the device, so a batch of steps
 //   k_pipe_a, k_matvec(v = A z), k_pipe_b, k_matvec(t = A w)
 // is captured once as a CUDA graph; after `done` is set every later kernel of
-// the batch returns at once (the products through MatvecArgs::skip).
+// the batch returns at once (the products through MatvecArgs::skip).  FP64
+// engines up to pipe_steps_max_rows take the same steps in k_pipe_steps
+// (hbx_kernels.cu), with the same bits.
 //
 // The element-wise roundings follow the reference's BLAS-1 calls (daxpy
 // y = y + a x, dlascl x = c x), written with __dmul_rn / __dadd_rn so that no
