@@ -920,7 +920,10 @@ template <int kPrec>
 __global__ void __launch_bounds__(kThreads, 1) k_bicg_steps(BicgArgs a) {
   constexpr bool kF32 = kPrec != kFP64;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  if (*(volatile const int *)&a.state->done) return;  // an earlier launch ended the solve (or its waits ran out)
+  // An earlier launch ended the solve (or its waits ran out).  The first CTA may
+  // end it in this launch before another has started, so a CTA's threads decide
+  // together.
+  if (__syncthreads_or(*(volatile const int *)&a.state->done)) return;
   const CtaInfo ci = a.ctas[blockIdx.x];
   const uint32_t nr = ci.nr_p + ci.nr_d + ci.nr_u;
   const Smem sm = cta_smem(smem_raw, a.lite + ci.rec_begin, nr);
