@@ -273,7 +273,7 @@ def run_ours(args, world, rank, local):
             "kernel": "k_bicg_steps (per BiCGSTAB step: 2 H-matvecs + vector updates + dots)",
             "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": achieved / peak, "peak_kind": peak_kind,
-            "traffic": ncu_traffic("k_bicg_iter"),
+            "traffic": ncu_traffic("k_bicg_steps"),
             "alg_bytes_per_launch": bytes_iter,
             "avg_launch_us": per_iter_s * 1e6,
         },
