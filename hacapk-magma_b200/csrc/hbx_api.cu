@@ -53,6 +53,14 @@ cudaError_t dev_malloc(void *p, size_t bytes) {
     if (e_ != cudaSuccess) return cuda_fail(e_, #call); \
   } while (0)
 
+// A table of the engine's to the device, in place when the call returns.  (A
+// plain copy of pageable memory may return with its last part under way on the
+// default stream, which the solves' streams do not wait for.)
+cudaError_t upload(hbx_hmat *h, void *dst, const void *src, size_t bytes) {
+  cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, h->stream);
+  return e == cudaSuccess ? cudaStreamSynchronize(h->stream) : e;
+}
+
 double now_s() {
   return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
 }
@@ -296,8 +304,8 @@ int hbx_create_batch(const stc_HACApK_leafmtxp *const *st, const int *nd, int co
   cudaError_t e;
   if ((e = dev_malloc(&h->d_inst_off, (count + 1) * sizeof(int))) != cudaSuccess ||
       (e = dev_malloc(&h->d_rinst, rinst.size() * sizeof(int))) != cudaSuccess ||
-      (e = cudaMemcpy(h->d_inst_off, cl.off.data(), (count + 1) * sizeof(int), cudaMemcpyHostToDevice)) != cudaSuccess ||
-      (e = cudaMemcpy(h->d_rinst, rinst.data(), rinst.size() * sizeof(int), cudaMemcpyHostToDevice)) != cudaSuccess) {
+      (e = upload(h, h->d_inst_off, cl.off.data(), (count + 1) * sizeof(int))) != cudaSuccess ||
+      (e = upload(h, h->d_rinst, rinst.data(), rinst.size() * sizeof(int))) != cudaSuccess) {
     free_engine(h);
     return cuda_fail(e, "hbx_create_batch: instance tables");
   }
@@ -308,10 +316,8 @@ int hbx_create_batch(const stc_HACApK_leafmtxp *const *st, const int *nd, int co
     if ((e = dev_malloc(&h->d_chunk_inst, cinst.size() * sizeof(uint32_t))) != cudaSuccess ||
         (e = dev_malloc(&h->d_chunk_base, cbase.size() * sizeof(uint32_t))) != cudaSuccess ||
         (e = dev_malloc(&h->d_inst_pre, (count + 1) * sizeof(int))) != cudaSuccess ||
-        (e = cudaMemcpy(h->d_chunk_inst, cinst.data(), cinst.size() * sizeof(uint32_t), cudaMemcpyHostToDevice)) !=
-            cudaSuccess ||
-        (e = cudaMemcpy(h->d_chunk_base, cbase.data(), cbase.size() * sizeof(uint32_t), cudaMemcpyHostToDevice)) !=
-            cudaSuccess) {
+        (e = upload(h, h->d_chunk_inst, cinst.data(), cinst.size() * sizeof(uint32_t))) != cudaSuccess ||
+        (e = upload(h, h->d_chunk_base, cbase.data(), cbase.size() * sizeof(uint32_t))) != cudaSuccess) {
       free_engine(h);
       return cuda_fail(e, "hbx_create_batch: chunk table");
     }
@@ -955,7 +961,7 @@ static int pipe_dev(hbx_hmat *h, const double *b, double *u, const hbx_solve_opt
   if (!h->d_pipe) HBX_CUDA(dev_malloc(&h->d_pipe, (size_t)hbx::kPipeVecs * n * sizeof(double)));
   if (!h->d_pstate) {
     HBX_CUDA(dev_malloc(&h->d_pstate, sizeof(hbx::PipeState)));
-    HBX_CUDA(cudaMemset(h->d_pstate, 0, sizeof(hbx::PipeState)));
+    HBX_CUDA(cudaMemsetAsync(h->d_pstate, 0, sizeof(hbx::PipeState), h->stream));
   }
   if (!h->h_pstate) HBX_CUDA(cudaHostAlloc(&h->h_pstate, 2 * sizeof(hbx::PipeState), cudaHostAllocDefault));
   if (!h->d_ppart) HBX_CUDA(dev_malloc(&h->d_ppart, (size_t)hbx::gcr_dot_blocks(n) * hbx::kMaxDots * 2 * sizeof(double)));
@@ -1184,7 +1190,7 @@ static int gcr_dev(hbx_hmat *h, const double *b, double *u, const hbx_solve_opts
   }
   if (!h->d_gcrs) {
     HBX_CUDA(dev_malloc(&h->d_gcrs, sizeof(hbx::GcrState)));
-    HBX_CUDA(cudaMemset(h->d_gcrs, 0, sizeof(hbx::GcrState)));
+    HBX_CUDA(cudaMemsetAsync(h->d_gcrs, 0, sizeof(hbx::GcrState), h->stream));
   }
   if (!h->h_gcrs) HBX_CUDA(cudaHostAlloc(&h->h_gcrs, sizeof(hbx::GcrState), cudaHostAllocDefault));
   if (!h->d_gcrpart)
@@ -1474,12 +1480,7 @@ int ensure_mr_workspace(hbx_hmat *hm) {
   if (!hm->d_mrpart)
     HBX_CUDA(dev_malloc(&hm->d_mrpart, (size_t)hbx::mr_row_blocks(hm->plan.nd) * 2 * hbx::kNrhs * sizeof(double)));
   if (!hm->d_mrsc) HBX_CUDA(dev_malloc(&hm->d_mrsc, hbx::kNrhs * sizeof(hbx::MrScal)));
-  if (!hm->d_mrint) {
-    int *d = nullptr;
-    HBX_CUDA(dev_malloc(&d, (2 + hbx::kNrhs) * sizeof(int)));
-    hm->d_mrint = d;
-    HBX_CUDA(cudaMemset(d, 0, (2 + hbx::kNrhs) * sizeof(int)));
-  }
+  if (!hm->d_mrint) HBX_CUDA(dev_malloc(&hm->d_mrint, (2 + hbx::kNrhs) * sizeof(int)));
   if (!hm->d_mrdbl) HBX_CUDA(dev_malloc(&hm->d_mrdbl, 2 * hbx::kNrhs * sizeof(double)));
   if (!hm->h_mrpin) HBX_CUDA(cudaMallocHost(&hm->h_mrpin, sizeof(MrPinned)));
   return HBX_OK;
@@ -1506,7 +1507,7 @@ int ensure_mm64(hbx_hmat *h, bool &have) {
       return HBX_OK;
     }
     h->d_mm64 = d;
-    HBX_CUDA(cudaMemcpy(d, p.data(), p.size() * sizeof(hbx::Mm64Unit), cudaMemcpyHostToDevice));
+    HBX_CUDA(upload(h, d, p.data(), p.size() * sizeof(hbx::Mm64Unit)));
   }
   if ((!h->d_mm64_next && dev_malloc(&h->d_mm64_next, 2 * sizeof(unsigned)) != cudaSuccess) ||
       (!h->d_mm64_zbu &&
@@ -1592,6 +1593,8 @@ int hbx_bicgstab_multi(hbx_hmat *h, hbx_hmat *hm, const double *B, double *U, co
   bool have_mm64 = false;
   if ((reinterpret_cast<uintptr_t>(U) & 15) == 0 && (st = ensure_mm64(h, have_mm64)) != HBX_OK) return st;
   HBX_CUDA(cudaEventRecord(hm->ev0, s));
+  // any_active, the mask and the reductions' ticket, whatever an earlier solve left
+  HBX_CUDA(cudaMemsetAsync(hm->d_mrint, 0, (2 + hbx::kNrhs) * sizeof(int), s));
   if ((st = norms(B)) != HBX_OK) return st;
   double bnorm[hbx::kNrhs], relres[hbx::kNrhs];
   int done[hbx::kNrhs], status[hbx::kNrhs], iters[hbx::kNrhs];
@@ -1770,20 +1773,15 @@ int ensure_bt_workspace(hbx_hmat *h, int count) {
     const int off[2] = {0, h->plan.nd};
     if (!h->d_inst_off) HBX_CUDA(dev_malloc(&h->d_inst_off, 2 * sizeof(int)));
     if (!h->d_rinst) HBX_CUDA(dev_malloc(&h->d_rinst, n * sizeof(int)));
-    HBX_CUDA(cudaMemcpy(h->d_inst_off, off, 2 * sizeof(int), cudaMemcpyHostToDevice));
-    HBX_CUDA(cudaMemset(h->d_rinst, 0, n * sizeof(int)));
+    HBX_CUDA(cudaMemsetAsync(h->d_rinst, 0, n * sizeof(int), h->stream));
+    HBX_CUDA(upload(h, h->d_inst_off, off, 2 * sizeof(int)));  // (waits for the clear too)
     h->inst_off.assign(off, off + 2);
   }
   if (!h->d_btv) HBX_CUDA(dev_malloc(&h->d_btv, 6 * n * sizeof(double)));
   if (!h->d_btsc) HBX_CUDA(dev_malloc(&h->d_btsc, count * sizeof(hbx::MrScal)));
   if (!h->d_btdbl) HBX_CUDA(dev_malloc(&h->d_btdbl, 3 * (size_t)count * sizeof(double)));
   if (!h->h_btany) HBX_CUDA(cudaMallocHost(&h->h_btany, 2 * sizeof(int)));
-  if (!h->d_btflags) {
-    hbx::BtFlags *f = nullptr;
-    HBX_CUDA(dev_malloc(&f, sizeof(hbx::BtFlags)));
-    h->d_btflags = f;
-    HBX_CUDA(cudaMemset(f, 0, sizeof(hbx::BtFlags)));
-  }
+  if (!h->d_btflags) HBX_CUDA(dev_malloc(&h->d_btflags, sizeof(hbx::BtFlags)));
   return HBX_OK;
 }
 
@@ -1802,6 +1800,7 @@ static int batch_dev(hbx_hmat *h, const double *b, double *u, double tol, const 
   double *r = h->d_btv, *rh = r + n, *p = rh + n, *ap = p + n, *t = ap + n, *at = t + n;
   double *bnorm = h->d_btdbl, *tnorm = bnorm + count;
   HBX_CUDA(cudaEventRecord(h->ev0, s));
+  HBX_CUDA(cudaMemsetAsync(h->d_btflags, 0, sizeof(hbx::BtFlags), s));  // whatever an earlier solve left
   // r = b - H u, rh = r, p = r; the stop test of every instance
   HBX_CUDA(mv_launch(h, matvec_args(h, -1.0, u, 1.0, b, r), s));
   hbx::BtStep a{};

@@ -1,0 +1,123 @@
+"""The engine's host code on the CPU, its object files linked with a stand-in
+for the CUDA runtime (tests/emu/fake_cuda.cpp: launches do nothing, every call
+is logged with its stream, any call can be made to fail)."""
+import ctypes as C
+import glob
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from conftest import ROOT, sphere
+
+PKG = os.path.join(ROOT, "hacapk-magma_b200")
+
+
+@pytest.fixture(scope="module")
+def fake(build_libs):
+    from hacapk_b200 import abi
+    emu = os.path.join(ROOT, "tests", "emu")
+    lib = os.path.join(emu, "_build", "libfakecuda.so")
+    os.makedirs(os.path.dirname(lib), exist_ok=True)
+    objs = sorted(glob.glob(os.path.join(PKG, "_build", "hbx_*.o")))
+    subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-I/usr/local/cuda/include", "-o", lib,
+                    os.path.join(emu, "fake_cuda.cpp"), *objs, "-fopenmp",
+                    f"-Wl,--version-script={os.path.join(emu, 'fake_cuda.map')}"], check=True)
+    L = abi._load(lib, abi.ENGINE_SYMBOLS)
+    L.fake_fail.argtypes = [C.c_char_p, C.c_int, C.c_int]
+    L.fake_op.argtypes = [C.c_int, C.POINTER(C.c_ulonglong), C.POINTER(C.c_int)]
+    L.fake_op.restype = C.c_char_p
+    return L
+
+
+@pytest.fixture
+def engine(fake, monkeypatch):
+    """The Engine class on the stand-in library."""
+    from hacapk_b200 import abi
+    from hacapk_b200.engine import Engine
+    monkeypatch.setattr(abi, "engine_lib", lambda: fake)
+    fake.fake_clear()
+    return Engine
+
+
+def _ops(L):
+    """(call, stream, complete on return) of every logged operation."""
+    out = []
+    for i in range(L.fake_ops()):
+        s, w = C.c_ulonglong(), C.c_int()
+        out.append((L.fake_op(i, C.byref(s), C.byref(w)).decode(), s.value, w.value))
+    return out
+
+
+DEVICE_WORK = ("launch", "cudaMemcpy", "cudaMemcpyAsync", "cudaMemset", "cudaMemsetAsync")
+
+
+def _unordered(ops, streams):
+    """Operations that a launch on one of `streams` (none of them ordered after
+    the default stream) may overtake: queued elsewhere, and neither complete on
+    return nor waited for by the host before the call's end."""
+    bad, waiting = [], {}
+    for what, s, done in ops:
+        if what in ("cudaStreamSynchronize", "cudaDeviceSynchronize"):
+            for k in [s] if what == "cudaStreamSynchronize" else list(waiting):
+                waiting.pop(k, None)
+        elif what == "launch" and s in streams:
+            bad += [x for k, v in waiting.items() if k != s for x in v]
+        elif what in DEVICE_WORK:
+            if done:  # and with it all that its stream held
+                waiting.pop(s, None)
+            else:
+                waiting.setdefault(s, []).append((what, s))
+    return bad
+
+
+USER = 0xbeef0  # a stream of the caller's
+
+
+@pytest.mark.parametrize("call", ["batch", "batch_host", "plain_batch", "batch_refined", "multi", "multi_host",
+                                  "multi_unaligned", "pipe", "gcr", "bicgstab"])
+def test_first_solves_queue_nothing_on_another_stream(engine, fake, call):
+    """A solver's first call on a new engine prepares its workspace.  All of it
+    is queued on the solve's own stream, or complete before the solve's first
+    launch: a non-blocking stream does not wait for the default one, where a
+    clear queued behind the caller's own work would land in the middle of the
+    solve."""
+    H = sphere(2)
+    n = H.nd
+    b = np.ones(n)
+    if "batch" in call and call != "plain_batch":
+        E, low = engine.batch([H, H]), engine.batch([H, H], precision=1)
+    else:
+        E, low = engine(H.st, n), engine(H.st, n, precision=1)
+    n = E.nd
+    M = engine(H.st, H.nd, precision=1, nrhs=64) if call.startswith("multi") else None
+    buf = np.zeros((2 * n + 1) * 64)
+    p = buf.ctypes.data + (-buf.ctypes.data) % 16
+    create = _ops(fake)
+    fake.fake_clear()
+    if call in ("batch", "plain_batch"):
+        E.bicgstab_batch_dev(p, p + 8 * n, stream=USER, check=False)
+    elif call == "batch_host":
+        E.bicgstab_batch_host(np.ones(n))
+    elif call == "batch_refined":
+        E.bicgstab_batch_refined_host(low, np.ones(n))
+    elif call == "multi":
+        E.bicgstab_multi_dev(M, p, p + 8 * 64 * n, stream=USER, check=False)
+    elif call == "multi_unaligned":
+        E.bicgstab_multi_dev(M, p, p + 8 * 64 * n + 8, stream=USER, check=False)
+    elif call == "multi_host":
+        E.bicgstab_multi_host(M, np.ones((n, 64)))
+    elif call == "pipe":
+        E.bicgstab_pipe_host(b, check=False, max_iter=8)
+    elif call == "gcr":
+        E.gcr_host(b, check=False, max_iter=8)
+    else:
+        E.bicgstab_host(b, check=False, max_iter=8)
+    ops = _ops(fake)
+    streams = {s for what, s, _ in ops if what == "launch"}
+    assert streams and 0 not in streams
+    assert _unordered(create + ops, streams) == []
+    for X in (E, low, M):
+        if X is not None:
+            X.close()
