@@ -528,7 +528,9 @@ __device__ __forceinline__ double pipe_total(const PipeStepArgs &a, int slot) {
 // TB/s: 2,430; the six barriers of a step and the vector work: some 20 us).
 __global__ void __launch_bounds__(kThreads, 1) k_pipe_steps(const __grid_constant__ PipeStepArgs a) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  if (*(volatile const int *)&a.st->done) return;  // an earlier launch ended the solve
+  // An earlier launch ended the solve.  (A CTA's threads decide together, as in
+  // k_bicg_steps: where waits run out the first CTA may end it in this launch.)
+  if (__syncthreads_or(*(volatile const int *)&a.st->done)) return;
   const CtaInfo ci = a.ctas[blockIdx.x];
   const uint32_t nr = ci.nr_p + ci.nr_d + ci.nr_u;
   const Smem sm = cta_smem(smem_raw, a.lite + ci.rec_begin, nr);
