@@ -1019,7 +1019,8 @@ static int pipe_dev(hbx_hmat *h, const double *b, double *u, const hbx_solve_opt
       if (launches++ == 0) continue;
       seen = k ^ 1;
       HBX_CUDA(cudaEventSynchronize(read[seen]));
-      if (h->h_pstate[seen].done || launched - 2 * (long long)batch > max_iter) break;
+      const hbx::PipeState &S = h->h_pstate[seen];
+      if (S.done || S.expired || launched - 2 * (long long)batch > max_iter) break;
     }
     float its = 0.f;
     cudaEventElapsedTime(&its, h->ev5, read[seen]);

@@ -223,7 +223,7 @@ struct PipeState {
   double alpha, beta, zeta, znorm, bnorm, relres, tol;
   int step, max_iter, done, status;
   unsigned ticket;  // last-block counter of the fused reductions
-  int pad;
+  int expired;      // a launch of k_pipe_steps found the error word set and did nothing
 };
 struct PipeVecs {
   const double *b;

@@ -596,6 +596,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_pipe_steps(const __grid_constan
   };
   if (sm.scal[kDone] != 0.0) {
     // done stays unset: a CTA that has yet to start must come this way too
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.st->expired = 1;
     stop();
     return;
   }

@@ -71,6 +71,7 @@ __global__ void __launch_bounds__(kDotThreads) k_pipe_init(PipeVecs v, size_t n,
   st->zeta = 0.0;
   st->step = 0;
   st->done = 0;
+  st->expired = 0;
   st->status = HBX_OK;
   const double rel = bnorm > 0.0 ? sqrt(rr) / bnorm : 0.0;
   st->relres = rel;

@@ -28,3 +28,18 @@ def test_expired_wait_ends_the_solve(gpu, build_libs, monkeypatch, solver, preci
     assert [i1[k] for k in ("status", "iterations", "relres")] == [i0[k] for k in ("status", "iterations", "relres")]
     assert np.array_equal(u0, u1)
     E.close()
+
+
+@pytest.mark.parametrize("solver,precision", SOLVES)
+def test_expired_wait_ends_the_solve_at_once(gpu, build_libs, monkeypatch, solver, precision):
+    """A large step limit queues no more launches than the steps under way."""
+    from hacapk_b200.engine import Engine
+    monkeypatch.setenv("HBX_TIMEOUT_MS", "100")
+    H = sphere(3)
+    E = Engine(H.st, H.nd, precision=precision)
+    b = np.random.default_rng(1).standard_normal(H.nd)
+    assert E.lib.hbx_debug_stall_next_barrier(E._h) == 0
+    _, i = getattr(E, solver)(b, tol=1e-6, max_iter=4000, batch=8, check=False)
+    assert i["status"] == 4
+    assert i["launches"] <= 2 * 4 * 8 + 7  # two batches of steps, four launches a step at most, and the ends
+    E.close()
