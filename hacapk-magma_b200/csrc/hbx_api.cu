@@ -472,6 +472,7 @@ static int create_engine(const stc_HACApK_leafmtxp *st, int nd, const hbx_option
     if (P.total_bytes >= ((uint64_t)32 << 20))
       e = hbx::pack_on_device(st, P, h->d_recs, h->d_ctas, h->d_stream, dev_malloc);
     if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
       std::vector<uint8_t> host(P.total_bytes);
       hbx::pack_plan(st, P, host.data());
       e = cudaMemcpy(h->d_stream, host.data(), P.total_bytes, cudaMemcpyHostToDevice);

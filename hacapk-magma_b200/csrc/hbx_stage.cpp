@@ -53,18 +53,16 @@ void touch_pages(double *host, uint64_t words) {
 
 }  // namespace
 
-cudaError_t Stager::open() {
-  if (!s_) {
-    cudaError_t e = cudaStreamCreate(&s_);  // a blocking stream: after the default stream's work
-    if (e != cudaSuccess) return e;
-  }
+bool Stager::open() {
+  cudaError_t e = cudaSuccess;
+  if (!s_) e = cudaStreamCreate(&s_);  // a blocking stream: after the default stream's work
   for (int k = 0; k < 2; ++k) {
-    cudaError_t e = cudaSuccess;
-    if (!buf_[k]) e = cudaHostAlloc(reinterpret_cast<void **>(&buf_[k]), kBufWords * sizeof(double), cudaHostAllocDefault);
+    if (e == cudaSuccess && !buf_[k])
+      e = cudaHostAlloc(reinterpret_cast<void **>(&buf_[k]), kBufWords * sizeof(double), cudaHostAllocDefault);
     if (e == cudaSuccess && !done_[k]) e = cudaEventCreateWithFlags(&done_[k], cudaEventDisableTiming);
-    if (e != cudaSuccess) return e;
   }
-  return cudaSuccess;
+  if (e != cudaSuccess) cudaGetLastError();  // the plain copies do without: no error is left for the next launch
+  return e == cudaSuccess;
 }
 
 Stager::~Stager() {
@@ -84,7 +82,12 @@ cudaError_t Stager::to_device(const std::vector<HostPiece> &pieces, uint64_t tot
     move_words<true>(pieces, 0, total, one.get());
     return cudaMemcpy(dev, one.get(), total * sizeof(double), cudaMemcpyHostToDevice);
   }
-  cudaError_t e = open();
+  cudaError_t e = cudaSuccess;
+  if (!open()) {
+    for (const HostPiece &p : pieces)
+      if (e == cudaSuccess) e = cudaMemcpy(dev + p.at, p.host, p.words * sizeof(double), cudaMemcpyHostToDevice);
+    return e;
+  }
   int k = 0;
   for (uint64_t w = 0; w < total && e == cudaSuccess; w += kBufWords, ++k) {
     const uint64_t n = std::min(kBufWords, total - w);
@@ -104,8 +107,13 @@ cudaError_t Stager::to_host(const std::vector<HostPiece> &pieces, uint64_t total
     touch_pages(pieces[0].host, total);
     return cudaMemcpy(pieces[0].host, dev, total * sizeof(double), cudaMemcpyDeviceToHost);
   }
-  cudaError_t e = open();
+  cudaError_t e = cudaSuccess;
   for (const HostPiece &p : pieces) touch_pages(p.host, p.words);
+  if (!open()) {
+    for (const HostPiece &p : pieces)
+      if (e == cudaSuccess) e = cudaMemcpy(p.host, dev + p.at, p.words * sizeof(double), cudaMemcpyDeviceToHost);
+    return e;
+  }
   const uint64_t nbuf = (total + kBufWords - 1) / kBufWords;
   for (uint64_t k = 0; k <= nbuf && e == cudaSuccess; ++k) {
     if (k < nbuf) {  // the transfer of buffer k runs while buffer k - 1 is spread

@@ -22,9 +22,9 @@ struct HostPiece {
 
 // Copies between a device image (total words) and host pieces, sorted by `at`
 // and tiling the image, ordered after the work on the device's default stream;
-// both return once the host side and the device side are complete.  The
-// page-locked buffers are taken by the first large copy and given back with
-// the object.
+// both return once the host side and the device side are complete (a plain copy
+// to the device: for work on the default stream).  The page-locked buffers are
+// taken by the first large copy and given back with the object.
 class Stager {
  public:
   Stager() = default;
@@ -35,7 +35,7 @@ class Stager {
   cudaError_t to_host(const std::vector<HostPiece> &pieces, uint64_t total, const double *dev);
 
  private:
-  cudaError_t open();
+  bool open();  // false where the system refuses the buffers: plain copies then
   double *buf_[2] = {nullptr, nullptr};
   cudaEvent_t done_[2] = {nullptr, nullptr};
   cudaStream_t s_ = nullptr;

@@ -121,3 +121,39 @@ def test_first_solves_queue_nothing_on_another_stream(engine, fake, call):
     for X in (E, low, M):
         if X is not None:
             X.close()
+
+
+def _big_dense(n=2100):
+    """One dense leaf of 35 MB: packed on the device, through the page-locked buffers."""
+    import test_plan as tp
+    P, keep = tp._custom([(2, 0, 1, n, 1, n, np.ones(n * n))], n)
+    return P, keep, n
+
+
+NO_MEMORY = 2  # cudaErrorMemoryAllocation
+REFUSALS = [("cudaHostAlloc", 0), ("cudaHostAlloc", 1), ("cudaEventCreate", 0), ("cudaStreamCreate", 0)]
+
+
+@pytest.mark.parametrize("what,nth", REFUSALS)
+def test_create_without_page_locked_memory(engine, fake, what, nth):
+    """The device packing goes on with plain copies where page-locked memory (or
+    a stream or event) is refused, and leaves no error behind for the next
+    launch to report."""
+    P, keep, n = _big_dense()
+    # the engine's own stream and events come before the packing's
+    first = {"cudaHostAlloc": 0, "cudaEventCreate": 6, "cudaStreamCreate": 1}[what]
+    fake.fake_fail(what.encode(), first + nth, NO_MEMORY)
+    E = engine(C.pointer(P), n)
+    assert fake.fake_last_error() == 0
+    E.close()
+
+
+@pytest.mark.parametrize("what,nth", REFUSALS)
+def test_fill_without_page_locked_memory(fake, engine, what, nth):
+    """The same for the leaves' copy from the device."""
+    from hacapk_b200 import hmatrix
+    first = {"cudaHostAlloc": 0, "cudaEventCreate": 0, "cudaStreamCreate": 6}[what]  # after the fill's own streams
+    fake.fake_fail(what.encode(), first + nth, NO_MEMORY)
+    H = hmatrix.HostHMatrix(hmatrix.icosphere(4), leaf_size=3000, eta=2.0, aca_eps=1e-5, fill="gpu")
+    assert fake.fake_last_error() == 0
+    H.close()
