@@ -27,6 +27,7 @@ int fail(int status, const std::string &msg) {
 }
 
 int cuda_fail(cudaError_t e, const char *what) {
+  cudaGetLastError();  // reported here, not by the next launch as well
   return fail(e == cudaErrorMemoryAllocation ? HBX_ERR_NOMEM : HBX_ERR_CUDA,
               std::string(what) + ": " + cudaGetErrorString(e));
 }

@@ -3,15 +3,18 @@
 //
 // Device memory is host memory, copies and clears are done at once, and a
 // kernel launch does nothing.  What the tests look at: on which stream every
-// operation was queued and whether the host waited for it (fake_log), and what
-// the engine does when one of these calls fails (fake_fail).
+// operation was queued and whether the host waited for it (fake_op), and what
+// the engine does when one of these calls (fake_fail) or a host allocation of
+// its own (fake_fail_new) fails.
 #include <cuda_runtime_api.h>
 
+#include <atomic>
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -28,17 +31,23 @@ std::map<std::string, int> g_fail;  // call -> the n-th one from now fails (0: t
 std::map<std::string, cudaError_t> g_fail_code;
 thread_local cudaError_t g_last = cudaSuccess;
 uintptr_t g_next = 0x1000;
+std::atomic<long> g_fail_new{-1};  // the n-th operator new from now fails (0: the next)
+thread_local bool t_own = false;   // the log's own allocations do not count
 
 // Logs the call; its error when a test asked for one.
 cudaError_t op(const char *what, cudaStream_t s = nullptr, int waits = 0) {
   std::lock_guard<std::mutex> lock(g_mu);
+  t_own = true;
+  cudaError_t e = cudaSuccess;
   auto it = g_fail.find(what);
   if (it != g_fail.end() && it->second-- == 0) {
     g_fail.erase(it);
-    return g_last = g_fail_code[what];
+    e = g_last = g_fail_code[what];
+  } else {
+    g_ops.push_back(Op{what, (uintptr_t)s, waits});
   }
-  g_ops.push_back(Op{what, (uintptr_t)s, waits});
-  return cudaSuccess;
+  t_own = false;
+  return e;
 }
 template <class T>
 cudaError_t handle(const char *what, T *out) {
@@ -54,6 +63,14 @@ cudaError_t alloc(const char *what, void **p, size_t n) {
 }
 
 }  // namespace
+
+void *operator new(size_t n) {
+  if (!t_own && g_fail_new.load() >= 0 && g_fail_new.fetch_sub(1) == 0) throw std::bad_alloc();
+  if (void *p = std::malloc(n ? n : 1)) return p;
+  throw std::bad_alloc();
+}
+void operator delete(void *p) noexcept { std::free(p); }
+void operator delete(void *p, size_t) noexcept { std::free(p); }
 
 extern "C" {
 
@@ -76,6 +93,8 @@ const char *fake_op(int i, unsigned long long *stream, int *waits) {
   return g_ops[(size_t)i].what.c_str();
 }
 int fake_last_error() { return g_last; }
+// The n-th host allocation from now fails; -1: none.  Returns the count still to go.
+int fake_fail_new(int n) { return (int)g_fail_new.exchange(n); }
 
 // ---- the runtime ----------------------------------------------------------------
 cudaError_t cudaMalloc(void **p, size_t n) { return alloc("cudaMalloc", p, n); }

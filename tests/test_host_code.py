@@ -5,6 +5,7 @@ import ctypes as C
 import glob
 import os
 import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -14,21 +15,27 @@ from conftest import ROOT, sphere
 PKG = os.path.join(ROOT, "hacapk-magma_b200")
 
 
-@pytest.fixture(scope="module")
-def fake(build_libs):
+EMU = os.path.join(ROOT, "tests", "emu")
+LIB = os.path.join(EMU, "_build", "libfakecuda.so")
+
+
+def _load():
     from hacapk_b200 import abi
-    emu = os.path.join(ROOT, "tests", "emu")
-    lib = os.path.join(emu, "_build", "libfakecuda.so")
-    os.makedirs(os.path.dirname(lib), exist_ok=True)
-    objs = sorted(glob.glob(os.path.join(PKG, "_build", "hbx_*.o")))
-    subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-I/usr/local/cuda/include", "-o", lib,
-                    os.path.join(emu, "fake_cuda.cpp"), *objs, "-fopenmp",
-                    f"-Wl,--version-script={os.path.join(emu, 'fake_cuda.map')}"], check=True)
-    L = abi._load(lib, abi.ENGINE_SYMBOLS)
+    L = abi._load(LIB, abi.ENGINE_SYMBOLS)
     L.fake_fail.argtypes = [C.c_char_p, C.c_int, C.c_int]
     L.fake_op.argtypes = [C.c_int, C.POINTER(C.c_ulonglong), C.POINTER(C.c_int)]
     L.fake_op.restype = C.c_char_p
     return L
+
+
+@pytest.fixture(scope="module")
+def fake(build_libs):
+    os.makedirs(os.path.dirname(LIB), exist_ok=True)
+    objs = sorted(glob.glob(os.path.join(PKG, "_build", "hbx_*.o")))
+    subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-I/usr/local/cuda/include", "-o", LIB,
+                    os.path.join(EMU, "fake_cuda.cpp"), *objs, "-fopenmp",
+                    f"-Wl,--version-script={os.path.join(EMU, 'fake_cuda.map')}"], check=True)
+    return _load()
 
 
 @pytest.fixture
@@ -157,3 +164,18 @@ def test_fill_without_page_locked_memory(fake, engine, what, nth):
     H = hmatrix.HostHMatrix(hmatrix.icosphere(4), leaf_size=3000, eta=2.0, aca_eps=1e-5, fill="gpu")
     assert fake.fake_last_error() == 0
     H.close()
+
+
+def test_a_reported_error_is_reported_once(engine, fake):
+    """The runtime keeps a failed call's error until it is asked for: the next
+    call's first launch must not report it again."""
+    from hacapk_b200.engine import HbxError
+    H = sphere(2)
+    E = engine(H.st, H.nd)
+    fake.fake_fail(b"cudaMalloc", 0, NO_MEMORY)
+    with pytest.raises(HbxError) as ei:
+        E.matvec_host(np.ones(H.nd))
+    assert ei.value.status == 2
+    E.matvec_host(np.ones(H.nd))
+    E.close()
+
