@@ -1490,27 +1490,37 @@ int ensure_mr_workspace(hbx_hmat *hm) {
 }
 
 // What the FP64 product with kNrhs right-hand sides on `h` needs; false when
-// it does not fit on the device (the caller then takes one product per
-// right-hand side).
+// it does not fit on the host or the device (the caller then takes one product
+// per right-hand side).  The unit table is published once it is in place.
 int ensure_mm64(hbx_hmat *h, bool &have) {
   have = false;
   if (!h->d_mm64) {
-    std::vector<hbx::RunLite> lite((size_t)h->num_runs);
-    if (h->num_runs > 0)
-      HBX_CUDA(cudaMemcpy(lite.data(), h->d_lite, lite.size() * sizeof(hbx::RunLite), cudaMemcpyDeviceToHost));
     std::vector<hbx::Mm64Unit> p, rest;
-    hbx::mm64_units(h->plan.ctas, lite, p, rest);
-    h->mm64_p = (uint32_t)p.size();
-    h->mm64_rest = (uint32_t)rest.size();
-    p.insert(p.end(), rest.begin(), rest.end());
+    size_t np = 0;
+    try {
+      std::vector<hbx::RunLite> lite((size_t)h->num_runs);
+      if (h->num_runs > 0)
+        HBX_CUDA(cudaMemcpy(lite.data(), h->d_lite, lite.size() * sizeof(hbx::RunLite), cudaMemcpyDeviceToHost));
+      hbx::mm64_units(h->plan.ctas, lite, p, rest);
+      np = p.size();
+      p.insert(p.end(), rest.begin(), rest.end());
+    } catch (...) {  // no exception leaves a C entry
+      return HBX_OK;
+    }
     HBX_CUDA(hbx::configure_mm64());
     hbx::Mm64Unit *d = nullptr;
     if (dev_malloc(&d, std::max<size_t>(1, p.size()) * sizeof(hbx::Mm64Unit)) != cudaSuccess) {
       cudaGetLastError();
       return HBX_OK;
     }
+    cudaError_t e = upload(h, d, p.data(), p.size() * sizeof(hbx::Mm64Unit));
+    if (e != cudaSuccess) {
+      cudaFree(d);
+      return cuda_fail(e, "multi-RHS product units");
+    }
     h->d_mm64 = d;
-    HBX_CUDA(upload(h, d, p.data(), p.size() * sizeof(hbx::Mm64Unit)));
+    h->mm64_p = (uint32_t)np;
+    h->mm64_rest = (uint32_t)(p.size() - np);
   }
   if ((!h->d_mm64_next && dev_malloc(&h->d_mm64_next, 2 * sizeof(unsigned)) != cudaSuccess) ||
       (!h->d_mm64_zbu &&

@@ -179,3 +179,58 @@ def test_a_reported_error_is_reported_once(engine, fake):
     E.matvec_host(np.ones(H.nd))
     E.close()
 
+
+def _multi(engine):
+    H = sphere(2)
+    E, M = engine(H.st, H.nd), engine(H.st, H.nd, precision=1, nrhs=64)
+    buf = np.zeros((2 * H.nd + 1) * 64)
+    p = buf.ctypes.data + (-buf.ctypes.data) % 16
+    return E, M, buf, lambda: E.bicgstab_multi_dev(M, p, p + 8 * 64 * H.nd, stream=USER)
+
+
+def test_unit_table_is_published_once_it_is_on_the_device(engine, fake):
+    """A failed upload of the multi-RHS product's units leaves no table behind:
+    the next solve uploads it."""
+    from hacapk_b200.engine import HbxError
+
+    def uploads():
+        return sum(what == "cudaMemcpyAsync" and s != USER for what, s, _ in _ops(fake))
+    E, M, buf, solve = _multi(engine)
+    fake.fake_clear()
+    fake.fake_fail(b"cudaMemcpyAsync", 0, 1)  # the first of the call
+    with pytest.raises(HbxError):
+        solve()
+    assert uploads() == 0
+    solve()
+    assert uploads() == 1
+    solve()  # kept
+    assert uploads() == 1
+    for X in (E, M):
+        X.close()
+
+
+def _fail_allocations():
+    """In a child: every host allocation of a first multi-RHS solve fails once."""
+    import test_host_code as t
+    from hacapk_b200 import abi
+    from hacapk_b200.engine import Engine
+    L = t._load()
+    abi.engine_lib = lambda: L
+    for n in range(100000):
+        E, M, buf, solve = t._multi(Engine)
+        L.fake_fail_new(n)
+        solve()  # an exception that leaves the C entry ends this process
+        left = L.fake_fail_new(-1)
+        E.close()
+        M.close()
+        if left >= 0:
+            print(f"{n} allocations")
+            return
+
+
+def test_no_exception_leaves_the_multi_rhs_solve(fake):
+    code = "import conftest, test_host_code as t; t._fail_allocations()"
+    r = subprocess.run([sys.executable, "-c", code], cwd=os.path.dirname(os.path.abspath(__file__)),
+                       capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, (r.returncode, r.stderr[-500:])
+    assert int(r.stdout.split()[0]) > 5
