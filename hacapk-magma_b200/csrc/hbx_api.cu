@@ -122,6 +122,7 @@ void free_engine(hbx_hmat *h) {
   cudaFree(h->d_btsc);
   cudaFree(h->d_btdbl);
   cudaFree(h->d_btflags);
+  cudaFree(const_cast<hbx::BtCta *>(h->btgrid.map));
   if (h->h_btany) cudaFreeHost(h->h_btany);
   if (h->h_pin) cudaFreeHost(h->h_pin);
   if (h->h_back) cudaFreeHost(h->h_back);
@@ -1770,13 +1771,6 @@ cudaError_t bt_matvec(void *ctx, const double *x, double *y, cudaStream_t s) {
   return hbx::launch_matvec(a, h->num_ctas, s, h->plan.precision);
 }
 
-// CTAs per instance of the vector kernels, by the largest instance.
-int bt_cluster_of(const hbx_hmat *h) {
-  int most = 0;
-  for (size_t k = 0; k + 1 < h->inst_off.size(); ++k) most = std::max(most, h->inst_off[k + 1] - h->inst_off[k]);
-  return hbx::bt_cluster(most);
-}
-
 // A plain engine is one instance.  Its tables are published (inst_off set)
 // only once both are on the device, and each work buffer is tested on its
 // own, so a call after a failed allocation never runs on a null pointer.
@@ -1789,6 +1783,23 @@ int ensure_bt_workspace(hbx_hmat *h, int count) {
     HBX_CUDA(cudaMemsetAsync(h->d_rinst, 0, n * sizeof(int), h->stream));
     HBX_CUDA(upload(h, h->d_inst_off, off, 2 * sizeof(int)));  // (waits for the clear too)
     h->inst_off.assign(off, off + 2);
+  }
+  if (!h->btgrid.map) {
+    std::vector<hbx::BtCta> map;
+    int cluster = 1;
+    try {
+      cluster = hbx::bt_map(h->inst_off, map);
+    } catch (...) {
+      return fail(HBX_ERR_NOMEM, "host memory for the batch vector kernels' CTAs");
+    }
+    hbx::BtCta *d = nullptr;
+    HBX_CUDA(dev_malloc(&d, map.size() * sizeof(hbx::BtCta)));
+    cudaError_t e = upload(h, d, map.data(), map.size() * sizeof(hbx::BtCta));
+    if (e != cudaSuccess) {
+      cudaFree(d);
+      return cuda_fail(e, "batch vector kernels' CTAs");
+    }
+    h->btgrid = hbx::BtGrid{d, (int)map.size(), cluster};
   }
   if (!h->d_btv) HBX_CUDA(dev_malloc(&h->d_btv, 6 * n * sizeof(double)));
   if (!h->d_btsc) HBX_CUDA(dev_malloc(&h->d_btsc, count * sizeof(hbx::MrScal)));
@@ -1819,7 +1830,7 @@ static int batch_dev(hbx_hmat *h, const double *b, double *u, double tol, const 
   hbx::BtStep a{};
   a.count = count;
   a.max_iter = max_iter;
-  a.cluster = bt_cluster_of(h);
+  a.grid = h->btgrid;
   a.off = h->d_inst_off;
   a.sc = h->d_btsc;
   a.flags = h->d_btflags;
@@ -1860,7 +1871,7 @@ static int batch_dev(hbx_hmat *h, const double *b, double *u, double tol, const 
   if (true_res) {
     // the true residual of every instance: ||b - H u|| / ||b||
     HBX_CUDA(mv_launch(h, matvec_args(h, -1.0, u, 1.0, b, r), s));
-    HBX_CUDA(hbx::bt_launch_norms(count, a.cluster, h->d_inst_off, r, tnorm, s));
+    HBX_CUDA(hbx::bt_launch_norms(a.grid, h->d_inst_off, r, tnorm, s));
     launches += 2;
   }
   std::vector<hbx::MrScal> sc(count);
@@ -1931,18 +1942,17 @@ static int batch_refined_dev(hbx_hmat *h, hbx_hmat *hl, const double *b, double 
   double *d_itol = reinterpret_cast<double *>(reinterpret_cast<char *>(h->d_rflag) +
                                               ((size_t)count * sizeof(int) + 15) / 16 * 16);
   double *dots = h->d_btdbl + 2 * (size_t)count;  // [count]: per-instance norms of the outer loop
-  const int cluster = bt_cluster_of(h);
   cudaEventRecord(h->ev2, s);
   std::vector<double> bb(count), rr(count), rel(count, 0.0), itol(count);
   std::vector<int> flag(count), inner(count, 0), status(count, HBX_ERR_NOT_CONVERGED), outer_k(count, 0);
-  HBX_CUDA(hbx::bt_launch_norms(count, cluster, h->d_inst_off, b, dots, s));
+  HBX_CUDA(hbx::bt_launch_norms(h->btgrid, h->d_inst_off, b, dots, s));
   HBX_CUDA(cudaMemcpyAsync(bb.data(), dots, count * sizeof(double), cudaMemcpyDeviceToHost, s));
   HBX_CUDA(cudaStreamSynchronize(s));
   std::vector<hbx_solve_info> ii(count);
   int outer = 0, launches = 1;
   for (;;) {
     HBX_CUDA(mv_launch(h, matvec_args(h, -1.0, u, 1.0, b, r), s));
-    HBX_CUDA(hbx::bt_launch_norms(count, cluster, h->d_inst_off, r, dots, s));
+    HBX_CUDA(hbx::bt_launch_norms(h->btgrid, h->d_inst_off, r, dots, s));
     HBX_CUDA(cudaMemcpyAsync(rr.data(), dots, count * sizeof(double), cudaMemcpyDeviceToHost, s));
     HBX_CUDA(cudaStreamSynchronize(s));
     launches += 2;

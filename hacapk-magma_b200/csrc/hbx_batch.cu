@@ -7,17 +7,23 @@
 // HACApK_SOLVER.c:631 does.  A finished instance keeps u and r, and its p and
 // t are zero so its rows of the block-diagonal products are zero.
 //
-// An instance's dots need its rows alone, so a cluster of CTAs takes an
+// An instance's dots need its rows alone, so a group of CTAs takes an
 // instance and goes from the product to the next product's input in one
 // launch: k_bt_mid forms alpha and t, k_bt_end zeta, u, r, beta and p, the
 // float copy of t or p that an FP32 or BF16 product reads included.  Two
 // launches and two products a step; what bounds them is their chain of
 // reductions (one or two, through the cluster's shared memory), and the
-// cluster's size (1 to 8 CTAs by the largest instance) keeps a row or a few
-// per thread.  The step of 24 bodies of 320 to 5,120 rows took 17 launches
-// beside the products before (dots, scalars, updates, float copies, prefix
-// counts: 40 us, and the host could not launch them fast enough); these two
-// take 12.
+// group's size (1, 2, 4 or 8 CTAs by the instance's own rows) keeps at most four
+// rows per thread up to 16,384 rows.  The step of 24 bodies of 320 to 5,120
+// rows took 17 launches beside the products before (dots, scalars, updates,
+// float copies, prefix counts: 40 us, and the host could not launch them fast
+// enough); these two take 12.
+//
+// The launch's clusters are of the largest group's size, and smaller groups
+// share one (the groups lie in descending size, so none straddles two).  A
+// cluster barrier then takes in more than its group, and a group that has
+// returned no longer counts: no group waits for anything but the others' next
+// barrier or end.
 //
 // Dot products are compensated (Dot2), as the single-body solver's: each
 // thread in row order, a warp butterfly, the CTA's warps in order, the
@@ -37,35 +43,41 @@ namespace {
 namespace cg = cooperative_groups;
 
 constexpr int kBt = 512;       // threads of a CTA
-constexpr int kBtRows = 4096;  // rows of the largest instance per 2x of cluster: about 4 to 8 a thread
+constexpr int kBtRows = 2048;  // rows that a CTA takes before its instance gets twice as many CTAs: 4 a thread
 constexpr int kMaxCluster = 8;
 
-// The rows of the calling thread: its instance's, in turn over the cluster.
+// The calling CTA's place and the rows of the calling thread: its instance's,
+// in turn over the group's CTAs.
 struct Rows {
-  int k;        // instance
-  int i0, i1;   // first and end row of the instance
+  int k;        // instance (-1: a CTA past the last group)
+  int size, rank, base;  // CTAs of the group, this one's place, the first one's rank in the cluster
+  int i1;       // end row of the instance
   int first, step;
 };
-__device__ __forceinline__ Rows my_rows(const int *off, unsigned nrank, unsigned rank) {
-  Rows R;
-  R.k = blockIdx.x / nrank;
-  R.i0 = off[R.k];
-  R.i1 = off[R.k + 1];
-  R.first = R.i0 + (int)(rank * kBt + threadIdx.x);
-  R.step = (int)nrank * kBt;
+__device__ __forceinline__ Rows my_rows(const BtCta *map, const int *off) {
+  const BtCta c = map[blockIdx.x];
+  Rows R{c.k, c.size, c.rank, c.base, 0, 0, kBt};
+  if (c.k < 0) return R;
+  R.i1 = off[c.k + 1];
+  R.first = off[c.k] + c.rank * kBt + (int)threadIdx.x;
+  R.step = c.size * kBt;
   return R;
 }
+__device__ __forceinline__ void group_sync(const Rows &R, cg::cluster_group &cl) {
+  if (R.size > 1) cl.sync();
+  else __syncthreads();
+}
 
-// tot[q]: the sums of acc[q] over the cluster, the same in every thread.
-// `sh` is written again only after another cluster barrier.
+// tot[q]: the sums of acc[q] over the group, the same in every thread.
+// `sh` is written again only after another group_sync.
 template <int NQ>
 struct ClusterSums {
   Acc2 warp[kBt / 32][NQ];
   Acc2 cta[NQ];
 };
 template <int NQ>
-__device__ __forceinline__ void cluster_totals(cg::cluster_group &cl, const Acc2 (&acc)[NQ], ClusterSums<NQ> &sh,
-                                               double (&tot)[NQ]) {
+__device__ __forceinline__ void group_totals(const Rows &R, cg::cluster_group &cl, const Acc2 (&acc)[NQ],
+                                             ClusterSums<NQ> &sh, double (&tot)[NQ]) {
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
   for (int q = 0; q < NQ; ++q) {
@@ -78,12 +90,11 @@ __device__ __forceinline__ void cluster_totals(cg::cluster_group &cl, const Acc2
     for (int k = 1; k < kBt / 32; ++k) t = acc2_merge(t, sh.warp[k][threadIdx.x]);
     sh.cta[threadIdx.x] = t;
   }
-  cl.sync();
-  const unsigned n = cl.num_blocks();
+  group_sync(R, cl);
 #pragma unroll
   for (int q = 0; q < NQ; ++q) {
-    Acc2 t = *cl.map_shared_rank(&sh.cta[q], 0);
-    for (unsigned c = 1; c < n; ++c) t = acc2_merge(t, *cl.map_shared_rank(&sh.cta[q], c));
+    Acc2 t = *cl.map_shared_rank(&sh.cta[q], R.base);
+    for (int c = 1; c < R.size; ++c) t = acc2_merge(t, *cl.map_shared_rank(&sh.cta[q], R.base + c));
     tot[q] = t.s + t.c;
   }
 }
@@ -131,16 +142,17 @@ __device__ __forceinline__ void count_active(int count, const MrScal *s, int *pr
 }
 
 // out[k] = x . x over the rows of instance k
-__global__ void __launch_bounds__(kBt) k_bt_norms(const int *off, const double *x, double *out) {
+__global__ void __launch_bounds__(kBt) k_bt_norms(const BtCta *map, const int *off, const double *x, double *out) {
   cg::cluster_group cl = cg::this_cluster();
   __shared__ ClusterSums<1> sh;
-  const Rows R = my_rows(off, cl.num_blocks(), cl.block_rank());
+  const Rows R = my_rows(map, off);
+  if (R.k < 0) return;
   Acc2 acc[1] = {{0.0, 0.0}};
   for (int i = R.first; i < R.i1; i += R.step) dot2_add(acc[0], x[i], x[i]);
   double tot[1];
-  cluster_totals<1>(cl, acc, sh, tot);
-  if (cl.block_rank() == 0 && threadIdx.x == 0) out[R.k] = tot[0];
-  cl.sync();  // every CTA has read the others' sums
+  group_totals<1>(R, cl, acc, sh, tot);
+  if (R.rank == 0 && threadIdx.x == 0) out[R.k] = tot[0];
+  group_sync(R, cl);  // every CTA has read the others' sums
 }
 
 // Start of the solve, r = b - H u formed: rh = r, p = r, the stop test; an
@@ -148,7 +160,11 @@ __global__ void __launch_bounds__(kBt) k_bt_norms(const int *off, const double *
 __global__ void __launch_bounds__(kBt) k_bt_init(BtStep a, const double *b, double tol, const double *rtol) {
   cg::cluster_group cl = cg::this_cluster();
   __shared__ ClusterSums<2> sh;
-  const Rows R = my_rows(a.off, cl.num_blocks(), cl.block_rank());
+  const Rows R = my_rows(a.grid.map, a.off);
+  if (R.k < 0) {
+    count_active(a.count, a.sc, a.pre, a.flags);
+    return;
+  }
   Acc2 acc[2] = {{0.0, 0.0}, {0.0, 0.0}};
   for (int i = R.first; i < R.i1; i += R.step) {
     const double rv = a.r[i], bv = b[i];
@@ -157,7 +173,7 @@ __global__ void __launch_bounds__(kBt) k_bt_init(BtStep a, const double *b, doub
     dot2_add(acc[1], bv, bv);
   }
   double tot[2];
-  cluster_totals<2>(cl, acc, sh, tot);
+  group_totals<2>(R, cl, acc, sh, tot);
   const double rr = tot[0], bn = std::sqrt(tot[1]);
   MrScal q{};
   q.rho = rr;
@@ -175,11 +191,11 @@ __global__ void __launch_bounds__(kBt) k_bt_init(BtStep a, const double *b, doub
     if (a.x32) a.x32[i] = (float)pv;
     if (!q.active) a.t[i] = 0.0;
   }
-  if (cl.block_rank() == 0 && threadIdx.x == 0) {
+  if (R.rank == 0 && threadIdx.x == 0) {
     a.bnorm[R.k] = bn;
     a.sc[R.k] = q;
   }
-  cl.sync();
+  group_sync(R, cl);
   count_active(a.count, a.sc, a.pre, a.flags);
 }
 
@@ -188,14 +204,15 @@ __global__ void __launch_bounds__(kBt) k_bt_mid(BtStep a) {
   cg::cluster_group cl = cg::this_cluster();
   __shared__ ClusterSums<1> sh;
   if (*(volatile const int *)&a.flags->done) return;
-  const Rows R = my_rows(a.off, cl.num_blocks(), cl.block_rank());
+  const Rows R = my_rows(a.grid.map, a.off);
+  if (R.k < 0) return;
   MrScal &S = a.sc[R.k];
-  if (!S.active) return;  // the same in the whole cluster
+  if (!S.active) return;  // the same in the whole group
   const double rho = S.rho;
   Acc2 acc[1] = {{0.0, 0.0}};
   for (int i = R.first; i < R.i1; i += R.step) dot2_add(acc[0], a.rh[i], a.ap[i]);
   double tot[1];
-  cluster_totals<1>(cl, acc, sh, tot);
+  group_totals<1>(R, cl, acc, sh, tot);
   const double alpha = rho / tot[0];
   const bool bad = tot[0] == 0.0 || !isfinite(alpha);
   for (int i = R.first; i < R.i1; i += R.step) {
@@ -204,8 +221,8 @@ __global__ void __launch_bounds__(kBt) k_bt_mid(BtStep a) {
     if (a.x32) a.x32[i] = (float)tv;
     if (bad) a.p[i] = 0.0;
   }
-  cl.sync();  // the others' sums and S are read
-  if (cl.block_rank() == 0 && threadIdx.x == 0) {
+  group_sync(R, cl);  // the others' sums and S are read
+  if (R.rank == 0 && threadIdx.x == 0) {
     if (bad) {
       S.active = 0;
       S.status = HBX_ERR_BREAKDOWN;
@@ -224,8 +241,9 @@ __global__ void __launch_bounds__(kBt) k_bt_end(BtStep a) {
   cg::cluster_group cl = cg::this_cluster();
   __shared__ ClusterSums<2> sh, sh2;
   if (*(volatile const int *)&a.flags->done) return;
-  const Rows R = my_rows(a.off, cl.num_blocks(), cl.block_rank());
-  MrScal q = a.sc[R.k];
+  const Rows R = my_rows(a.grid.map, a.off);
+  MrScal q{};
+  if (R.k >= 0) q = a.sc[R.k];
   if (q.active) {
     Acc2 acc[2] = {{0.0, 0.0}, {0.0, 0.0}};
     for (int i = R.first; i < R.i1; i += R.step) {
@@ -234,7 +252,7 @@ __global__ void __launch_bounds__(kBt) k_bt_end(BtStep a) {
       dot2_add(acc[1], av, av);
     }
     double tot[2];
-    cluster_totals<2>(cl, acc, sh, tot);
+    group_totals<2>(R, cl, acc, sh, tot);
     const double zeta = tot[1] != 0.0 ? tot[0] / tot[1] : 0.0;
     bool run = isfinite(zeta);
     if (!run) {
@@ -250,7 +268,7 @@ __global__ void __launch_bounds__(kBt) k_bt_end(BtStep a) {
         dot2_add(acc[0], a.rh[i], rv);
         dot2_add(acc[1], rv, rv);
       }
-      cluster_totals<2>(cl, acc, sh2, tot);
+      group_totals<2>(R, cl, acc, sh2, tot);
       const double rho_new = tot[0], rr = tot[1], bn = a.bnorm[R.k];
       q.iters += 1;
       q.rr = rr;
@@ -281,8 +299,8 @@ __global__ void __launch_bounds__(kBt) k_bt_end(BtStep a) {
       if (a.x32) a.x32[i] = (float)pv;
       if (!run) a.t[i] = 0.0;
     }
-    cl.sync();  // the others' sums and scalars are read
-    if (cl.block_rank() == 0 && threadIdx.x == 0) a.sc[R.k] = q;
+    group_sync(R, cl);  // the others' sums and scalars are read
+    if (R.rank == 0 && threadIdx.x == 0) a.sc[R.k] = q;
   }
   count_active(a.count, a.sc, a.pre, a.flags);
 }
@@ -294,9 +312,9 @@ __global__ void k_bt_mask(size_t n, const int *rinst, const int *flag, double *r
 }
 
 template <class... P, class... A>
-cudaError_t launch_clusters(void (*kern)(P...), int count, int cluster, cudaStream_t s, A... args) {
+cudaError_t launch_clusters(void (*kern)(P...), int ctas, int cluster, cudaStream_t s, A... args) {
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)(count * cluster));
+  cfg.gridDim = dim3((unsigned)ctas);
   cfg.blockDim = dim3(kBt);
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
@@ -311,18 +329,36 @@ cudaError_t launch_clusters(void (*kern)(P...), int count, int cluster, cudaStre
 
 }  // namespace
 
-int bt_cluster(int max_rows) {
-  int c = 1;
-  while (c < kMaxCluster && max_rows > c * kBtRows / 2) c *= 2;
-  return c;
+// Each instance's group by its own rows: with every group sized by the largest
+// instance, a step of 1,000 bodies of 320 rows beside one of 20,480 took 773 us,
+// more than the 17 launches (580); this way it takes 533 where those take 622
+// (another draw of the bodies).  One body of 1,280 rows alone 90 -> 61 us a step,
+// 20,480 183 -> 139, 81,920 534 -> 464, 327,680 (80 rows a thread) 2,142 -> 2,038.
+int bt_map(const std::vector<int> &off, std::vector<BtCta> &map) {
+  const int count = (int)off.size() - 1;
+  auto size_of = [&](int k) {
+    int c = 1;
+    while (c < kMaxCluster && off[k + 1] - off[k] > c * kBtRows) c *= 2;
+    return c;
+  };
+  int cluster = 1;
+  for (int k = 0; k < count; ++k) cluster = std::max(cluster, size_of(k));
+  map.clear();
+  for (int c = cluster; c > 0; c /= 2)
+    for (int k = 0; k < count; ++k)
+      if (size_of(k) == c)
+        for (int r = 0; r < c; ++r)
+          map.push_back(BtCta{k, (uint8_t)c, (uint8_t)r, (uint8_t)((map.size() - r) % cluster), 0});
+  while (map.size() % cluster) map.push_back(BtCta{-1, 1, 0, 0, 0});
+  return cluster;
 }
 
-cudaError_t bt_launch_norms(int count, int cluster, const int *off, const double *x, double *out, cudaStream_t s) {
-  return launch_clusters(k_bt_norms, count, cluster, s, off, x, out);
+cudaError_t bt_launch_norms(const BtGrid &g, const int *off, const double *x, double *out, cudaStream_t s) {
+  return launch_clusters(k_bt_norms, g.ctas, g.cluster, s, g.map, off, x, out);
 }
 
 cudaError_t bt_launch_init(const BtStep &a, const double *b, double tol, const double *rtol, cudaStream_t s) {
-  return launch_clusters(k_bt_init, a.count, a.cluster, s, a, b, tol, rtol);
+  return launch_clusters(k_bt_init, a.grid.ctas, a.grid.cluster, s, a, b, tol, rtol);
 }
 
 cudaError_t bt_launch_mask(size_t n, const int *rinst, const int *flag, double *r, cudaStream_t s) {
@@ -333,9 +369,9 @@ cudaError_t bt_launch_mask(size_t n, const int *rinst, const int *flag, double *
 cudaError_t bt_launch_step(const BtStep &a, cudaStream_t s) {
   cudaError_t e;
   if ((e = a.matvec(a.ctx, a.p, a.ap, s)) != cudaSuccess) return e;
-  if ((e = launch_clusters(k_bt_mid, a.count, a.cluster, s, a)) != cudaSuccess) return e;
+  if ((e = launch_clusters(k_bt_mid, a.grid.ctas, a.grid.cluster, s, a)) != cudaSuccess) return e;
   if ((e = a.matvec(a.ctx, a.t, a.at, s)) != cudaSuccess) return e;
-  return launch_clusters(k_bt_end, a.count, a.cluster, s, a);
+  return launch_clusters(k_bt_end, a.grid.ctas, a.grid.cluster, s, a);
 }
 
 }  // namespace hbx

@@ -172,8 +172,17 @@ struct BtFlags {
   int any, done;    // some instance runs; none does (MatvecArgs::skip)
   unsigned ticket;  // last-block counter, zero between launches
 };
+struct BtCta {  // a CTA of the vector kernels
+  int k;                           // its instance (-1: none)
+  uint8_t size, rank, base, pad;   // CTAs of the instance, this one's place, the first one's rank in the cluster
+};
+struct BtGrid {
+  const BtCta *map;  // on the device
+  int ctas, cluster;
+};
 struct BtStep {
-  int count, max_iter, cluster;  // cluster: CTAs per instance (bt_cluster)
+  int count, max_iter;
+  BtGrid grid;
   const int *off;                // instance row offsets [count + 1]
   MrScal *sc;
   BtFlags *flags;
@@ -183,8 +192,9 @@ struct BtStep {
   cudaError_t (*matvec)(void *ctx, const double *x, double *y, cudaStream_t s);
   void *ctx;
 };
-int bt_cluster(int max_rows);
-cudaError_t bt_launch_norms(int count, int cluster, const int *off, const double *x, double *out, cudaStream_t s);
+// The CTAs of the instances at rows off[k]..off[k + 1]; returns the cluster size.
+int bt_map(const std::vector<int> &off, std::vector<BtCta> &map);
+cudaError_t bt_launch_norms(const BtGrid &g, const int *off, const double *x, double *out, cudaStream_t s);
 cudaError_t bt_launch_init(const BtStep &a, const double *b, double tol, const double *rtol, cudaStream_t s);
 cudaError_t bt_launch_mask(size_t n, const int *rinst, const int *flag, double *r, cudaStream_t s);
 cudaError_t bt_launch_step(const BtStep &a, cudaStream_t s);
@@ -339,6 +349,7 @@ struct hbx_hmat {
   hbx::MrScal *d_btsc = nullptr;
   double *d_btdbl = nullptr;    // bnorm [count], true norms [count], norms of the outer loop [count]
   hbx::BtFlags *d_btflags = nullptr;
+  hbx::BtGrid btgrid{};         // the vector kernels' CTAs
   int *h_btany = nullptr;       // page-locked: any_active after the last two batches of steps
   hbx::Plan plan;
   uint8_t *d_stream = nullptr;
