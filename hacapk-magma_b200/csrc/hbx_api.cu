@@ -232,11 +232,17 @@ int host_out(hbx_hmat *h, const double *da, double *a, cudaStream_t s) {
   return *err ? check_device_error(h, s) : HBX_OK;
 }
 
-int ensure_host_staging(hbx_hmat *h) {
+// Two device vectors for a call's host vectors (the products' and the batch solves').
+int ensure_host_vectors(hbx_hmat *h) {
   const size_t n = (size_t)h->plan.nd;
   if (!h->d_x) HBX_CUDA(dev_malloc(&h->d_x, n * sizeof(double)));
   if (!h->d_y) HBX_CUDA(dev_malloc(&h->d_y, n * sizeof(double)));
-  return ensure_pin(h);
+  return HBX_OK;
+}
+
+int ensure_host_staging(hbx_hmat *h) {
+  const int st = ensure_host_vectors(h);
+  return st != HBX_OK ? st : ensure_pin(h);
 }
 
 int ensure_solver(hbx_hmat *h, int max_iter) {
@@ -2026,10 +2032,10 @@ int hbx_bicgstab_batch_refined(hbx_hmat *h, hbx_hmat *hl, const double *b, doubl
 int hbx_bicgstab_batch_refined_host(hbx_hmat *h, hbx_hmat *hl, const double *b, double *u, const hbx_solve_opts *opts,
                                     hbx_solve_info *info) {
   if (!h || !hl || !b || !u) return fail(HBX_ERR_INVALID, "hbx_bicgstab_batch_refined_host: NULL argument");
-  int st = ensure_solver(h, 0);
+  int st = ensure_host_vectors(h);
   if (st != HBX_OK) return st;
-  const size_t n = (size_t)h->plan.nd, bytes = n * sizeof(double);
-  double *db = h->d_work + 6 * n, *du = h->d_work + 7 * n;
+  const size_t bytes = (size_t)h->plan.nd * sizeof(double);
+  double *db = h->d_x, *du = h->d_y;
   cudaStream_t s = h->stream;
   HBX_CUDA(cudaMemcpyAsync(db, b, bytes, cudaMemcpyHostToDevice, s));
   HBX_CUDA(cudaMemcpyAsync(du, u, bytes, cudaMemcpyHostToDevice, s));
@@ -2043,10 +2049,10 @@ int hbx_bicgstab_batch_refined_host(hbx_hmat *h, hbx_hmat *hl, const double *b, 
 int hbx_bicgstab_batch_host(hbx_hmat *h, const double *b, double *u, const hbx_solve_opts *opts,
                             hbx_solve_info *info) {
   if (!h || !b || !u) return fail(HBX_ERR_INVALID, "hbx_bicgstab_batch_host: NULL argument");
-  int st = ensure_solver(h, 0);
+  int st = ensure_host_vectors(h);
   if (st != HBX_OK) return st;
-  const size_t n = (size_t)h->plan.nd, bytes = n * sizeof(double);
-  double *db = h->d_work + 6 * n, *du = h->d_work + 7 * n;
+  const size_t bytes = (size_t)h->plan.nd * sizeof(double);
+  double *db = h->d_x, *du = h->d_y;
   cudaStream_t s = h->stream;
   HBX_CUDA(cudaMemcpyAsync(db, b, bytes, cudaMemcpyHostToDevice, s));
   HBX_CUDA(cudaMemcpyAsync(du, u, bytes, cudaMemcpyHostToDevice, s));

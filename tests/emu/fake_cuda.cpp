@@ -55,6 +55,7 @@ cudaError_t handle(const char *what, T *out) {
   if (e == cudaSuccess) *out = (T)(g_next += 16);
   return e;
 }
+std::map<void *, size_t> g_device;  // live device allocations
 cudaError_t alloc(const char *what, void **p, size_t n) {
   cudaError_t e = op(what);
   if (e != cudaSuccess) return e;
@@ -92,15 +93,32 @@ const char *fake_op(int i, unsigned long long *stream, int *waits) {
   *waits = g_ops[(size_t)i].waits;
   return g_ops[(size_t)i].what.c_str();
 }
+long long fake_device_bytes() {  // device memory held now
+  long long n = 0;
+  for (const auto &a : g_device) n += (long long)a.second;
+  return n;
+}
 int fake_last_error() { return g_last; }
 // The n-th host allocation from now fails; -1: none.  Returns the count still to go.
 int fake_fail_new(int n) { return (int)g_fail_new.exchange(n); }
 
 // ---- the runtime ----------------------------------------------------------------
-cudaError_t cudaMalloc(void **p, size_t n) { return alloc("cudaMalloc", p, n); }
+cudaError_t cudaMalloc(void **p, size_t n) {
+  cudaError_t e = alloc("cudaMalloc", p, n);
+  std::lock_guard<std::mutex> lock(g_mu);
+  t_own = true;
+  if (e == cudaSuccess) g_device[*p] = n;
+  t_own = false;
+  return e;
+}
 cudaError_t cudaMallocHost(void **p, size_t n) { return alloc("cudaMallocHost", p, n); }
 cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) { return alloc("cudaHostAlloc", p, n); }
-cudaError_t cudaFree(void *p) { std::free(p); return cudaSuccess; }
+cudaError_t cudaFree(void *p) {
+  std::lock_guard<std::mutex> lock(g_mu);
+  g_device.erase(p);
+  std::free(p);
+  return cudaSuccess;
+}
 cudaError_t cudaFreeHost(void *p) { std::free(p); return cudaSuccess; }
 // A plain copy to the device may return with its last part under way; one to the host is complete.
 cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind k) {

@@ -25,6 +25,7 @@ def _load():
     L.fake_fail.argtypes = [C.c_char_p, C.c_int, C.c_int]
     L.fake_op.argtypes = [C.c_int, C.POINTER(C.c_ulonglong), C.POINTER(C.c_int)]
     L.fake_op.restype = C.c_char_p
+    L.fake_device_bytes.restype = C.c_longlong
     return L
 
 
@@ -234,3 +235,26 @@ def test_no_exception_leaves_the_multi_rhs_solve(fake):
                        capture_output=True, text=True, timeout=600)
     assert r.returncode == 0, (r.returncode, r.stderr[-500:])
     assert int(r.stdout.split()[0]) > 5
+
+
+@pytest.mark.parametrize("refined", [False, True])
+def test_batch_host_solve_holds_two_vectors_of_its_own(engine, fake, refined):
+    """The host-vector form of a batch solve holds b and u on the device beside
+    what the device-vector form holds, and no other solver's workspace."""
+    H = sphere(2)
+    held = []
+    for host in (False, True):
+        E, low = engine.batch([H, H]), engine.batch([H, H], precision=1)
+        before = fake.fake_device_bytes()
+        b = np.ones(2 * E.nd)
+        if host:
+            E.bicgstab_batch_refined_host(low, b[:E.nd]) if refined else E.bicgstab_batch_host(b[:E.nd])
+        elif refined:
+            E.bicgstab_batch_refined_dev(low, b.ctypes.data, b.ctypes.data + 8 * E.nd)
+        else:
+            E.bicgstab_batch_dev(b.ctypes.data, b.ctypes.data + 8 * E.nd)
+        held.append(fake.fake_device_bytes() - before)
+        nd = E.nd
+        E.close()
+        low.close()
+    assert held[1] - held[0] == 2 * 8 * nd
