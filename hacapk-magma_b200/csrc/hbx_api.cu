@@ -444,8 +444,10 @@ static int create_engine(const stc_HACApK_leafmtxp *st, int nd, const hbx_option
     return bail(cuda_fail(e, "cudaMalloc(lite)"));
   if ((e = dev_malloc(&h->d_atoms, std::max<size_t>(1, P.atoms.size()) * sizeof(hbx::Atom))) != cudaSuccess)
     return bail(cuda_fail(e, "cudaMalloc(atoms)"));
-  // zbu twice: the two H-matvecs of a BiCGSTAB step write separate copies
-  if ((e = dev_malloc(&h->d_zbu, 2 * std::max<uint64_t>(1, P.zbu_len) * sizeof(double))) != cudaSuccess)
+  // zbu twice: the two H-matvecs of a BiCGSTAB step write separate copies (the
+  // FP32 and BF16 engines' in d_f32, in float; a multi-RHS engine's in d_zbum)
+  if (prec == hbx::kFP64 &&
+      (e = dev_malloc(&h->d_zbu, 2 * std::max<uint64_t>(1, P.zbu_len) * sizeof(double))) != cudaSuccess)
     return bail(cuda_fail(e, "cudaMalloc(zbu)"));
   if (P.precision != hbx::kFP64 &&
       (e = dev_malloc(&h->d_f32, (3 * (size_t)nd + 2 * std::max<uint64_t>(1, P.zbu_len)) * sizeof(float))) !=
@@ -493,7 +495,7 @@ static int create_engine(const stc_HACApK_leafmtxp *st, int nd, const hbx_option
     return bail(cuda_fail(e, "multi-RHS columns"));
   cudaMemset(h->d_gbar, 0, 4 * sizeof(unsigned));
   cudaMemset(h->d_err, 0, sizeof(int));
-  cudaMemset(h->d_zbu, 0, 2 * std::max<uint64_t>(1, P.zbu_len) * sizeof(double));
+  if (h->d_zbu) cudaMemset(h->d_zbu, 0, 2 * std::max<uint64_t>(1, P.zbu_len) * sizeof(double));
   if ((e = cudaDeviceSynchronize()) != cudaSuccess) return bail(cuda_fail(e, "hbx_create sync"));
   // host copies of the records and the packing tables are no longer needed
   h->num_runs = (long long)P.recs.size();

@@ -98,6 +98,11 @@ long long fake_device_bytes() {  // device memory held now
   for (const auto &a : g_device) n += (long long)a.second;
   return n;
 }
+int fake_device_blocks(long long bytes) {  // device allocations of this size held now
+  int n = 0;
+  for (const auto &a : g_device) n += a.second == (size_t)bytes;
+  return n;
+}
 int fake_last_error() { return g_last; }
 // The n-th host allocation from now fails; -1: none.  Returns the count still to go.
 int fake_fail_new(int n) { return (int)g_fail_new.exchange(n); }

@@ -26,6 +26,7 @@ def _load():
     L.fake_op.argtypes = [C.c_int, C.POINTER(C.c_ulonglong), C.POINTER(C.c_int)]
     L.fake_op.restype = C.c_char_p
     L.fake_device_bytes.restype = C.c_longlong
+    L.fake_device_blocks.argtypes = [C.c_longlong]
     return L
 
 
@@ -258,3 +259,13 @@ def test_batch_host_solve_holds_two_vectors_of_its_own(engine, fake, refined):
         E.close()
         low.close()
     assert held[1] - held[0] == 2 * 8 * nd
+
+
+@pytest.mark.parametrize("precision,nrhs", [(0, 0), (1, 0), (2, 0), (1, 64)])
+def test_only_fp64_engines_hold_zbu_in_doubles(engine, fake, precision, nrhs):
+    """The other engines' V^T x segments are floats, in a buffer of their own."""
+    H = sphere(3)
+    E = engine(H.st, H.nd, precision=precision, nrhs=nrhs)
+    assert E.info["zbu_len"] > 0
+    assert fake.fake_device_blocks(2 * 8 * E.info["zbu_len"]) == (1 if precision == 0 else 0)
+    E.close()
