@@ -703,7 +703,10 @@ int hbx_fill_leaves(const double *xyz, int nond, const int *face2node, int nofc,
   long long retried = 0;
   double t_aca = 0.0;
   bool dense_launched = false;
-  constexpr int kBigLeaf = 4096;  // leaves of this many rows and columns make batches of their own
+  // Leaves of this many rows and columns make batches of their own.  (All in one
+  // batch is no faster: the 81,920-triangle sphere 148 ms this way, 145 to 188
+  // that way, 327,680 triangles 620 and 604.)
+  constexpr int kBigLeaf = 4096;
   DevBuf d_work, d_mask, d_jobs;
   size_t work_cap = 0, mask_cap = 0, jobs_cap = 0;
   auto ensure = [&](DevBuf &b, size_t &cap, size_t bytes) -> cudaError_t {
@@ -757,10 +760,16 @@ int hbx_fill_leaves(const double *xyz, int nond, const int *face2node, int nofc,
       std::vector<AcaJob> grouped(jobs.size());
       for (size_t q = 0; q < jobs.size(); ++q) grouped[at[q]] = jobs[q];
       const double tb = now_s();
+      const size_t held = work_cap;
       if ((e = ensure(d_jobs, jobs_cap, jobs.size() * sizeof(AcaJob))) != cudaSuccess ||
           (e = ensure(d_work, work_cap, (size_t)wd * 8)) != cudaSuccess ||
           (e = ensure(d_mask, mask_cap, (size_t)wm * 4)) != cudaSuccess)
         return e == cudaErrorMemoryAllocation ? HBX_ERR_NOMEM : HBX_ERR_CUDA;
+      // A leaf that stops in a column or row below the threshold goes on to read
+      // the other vector of that term, which it never set.  New memory may hold
+      // another allocation's words (NaN among them: non-finite factors in 4,097
+      // leaves of a 20,480-triangle sphere); cleared, the ranks are the host fill's.
+      if (work_cap != held && (e = cudaMemset(d_work.p, 0, work_cap)) != cudaSuccess) return HBX_ERR_CUDA;
       cudaMemcpy(d_jobs.p, grouped.data(), grouped.size() * sizeof(AcaJob), cudaMemcpyHostToDevice);
       for (int c = kTeams - 1; c >= 0; --c) {  // the longest leaves start first
         const int n = first[c + 1] - first[c];

@@ -24,6 +24,8 @@ struct Op {
   std::string what;
   uintptr_t stream;
   int waits;  // 1: complete when the call returns
+  const void *at;  // the memory that an allocation gave or a clear wrote ...
+  size_t bytes;    // ... and its size
 };
 std::mutex g_mu;
 std::vector<Op> g_ops;
@@ -35,7 +37,7 @@ std::atomic<long> g_fail_new{-1};  // the n-th operator new from now fails (0: t
 thread_local bool t_own = false;   // the log's own allocations do not count
 
 // Logs the call; its error when a test asked for one.
-cudaError_t op(const char *what, cudaStream_t s = nullptr, int waits = 0) {
+cudaError_t op(const char *what, cudaStream_t s = nullptr, int waits = 0, const void *at = nullptr, size_t bytes = 0) {
   std::lock_guard<std::mutex> lock(g_mu);
   t_own = true;
   cudaError_t e = cudaSuccess;
@@ -44,7 +46,7 @@ cudaError_t op(const char *what, cudaStream_t s = nullptr, int waits = 0) {
     g_fail.erase(it);
     e = g_last = g_fail_code[what];
   } else {
-    g_ops.push_back(Op{what, (uintptr_t)s, waits});
+    g_ops.push_back(Op{what, (uintptr_t)s, waits, at, bytes});
   }
   t_own = false;
   return e;
@@ -93,6 +95,10 @@ const char *fake_op(int i, unsigned long long *stream, int *waits) {
   *waits = g_ops[(size_t)i].waits;
   return g_ops[(size_t)i].what.c_str();
 }
+const void *fake_op_memory(int i, unsigned long long *bytes) {
+  *bytes = g_ops[(size_t)i].bytes;
+  return g_ops[(size_t)i].at;
+}
 long long fake_device_bytes() {  // device memory held now
   long long n = 0;
   for (const auto &a : g_device) n += (long long)a.second;
@@ -112,7 +118,11 @@ cudaError_t cudaMalloc(void **p, size_t n) {
   cudaError_t e = alloc("cudaMalloc", p, n);
   std::lock_guard<std::mutex> lock(g_mu);
   t_own = true;
-  if (e == cudaSuccess) g_device[*p] = n;
+  if (e == cudaSuccess) {
+    g_device[*p] = n;
+    g_ops.back().at = *p;
+    g_ops.back().bytes = n;
+  }
   t_own = false;
   return e;
 }
@@ -137,12 +147,12 @@ cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cu
   return e;
 }
 cudaError_t cudaMemset(void *d, int v, size_t n) {
-  cudaError_t e = op("cudaMemset");
+  cudaError_t e = op("cudaMemset", nullptr, 0, d, n);
   if (e == cudaSuccess && n) std::memset(d, v, n);
   return e;
 }
 cudaError_t cudaMemsetAsync(void *d, int v, size_t n, cudaStream_t st) {
-  cudaError_t e = op("cudaMemsetAsync", st);
+  cudaError_t e = op("cudaMemsetAsync", st, 0, d, n);
   if (e == cudaSuccess && n) std::memset(d, v, n);
   return e;
 }

@@ -27,6 +27,8 @@ def _load():
     L.fake_op.restype = C.c_char_p
     L.fake_device_bytes.restype = C.c_longlong
     L.fake_device_blocks.argtypes = [C.c_longlong]
+    L.fake_op_memory.argtypes = [C.c_int, C.POINTER(C.c_ulonglong)]
+    L.fake_op_memory.restype = C.c_void_p
     return L
 
 
@@ -269,3 +271,20 @@ def test_only_fp64_engines_hold_zbu_in_doubles(engine, fake, precision, nrhs):
     assert E.info["zbu_len"] > 0
     assert fake.fake_device_blocks(2 * 8 * E.info["zbu_len"]) == (1 if precision == 0 else 0)
     E.close()
+
+
+def test_fill_workspace_is_cleared_before_the_kernels(fake, engine):
+    """ACA+ reads a column of its workspace that it never set when it stops in
+    one, so the workspace must not hold what another allocation left there."""
+    from hacapk_b200 import hmatrix
+    H = hmatrix.HostHMatrix(hmatrix.icosphere(3), leaf_size=32, eta=2.0, aca_eps=1e-5, fill="gpu")
+    mem = []
+    for i in range(fake.fake_ops()):
+        n = C.c_ulonglong()
+        mem.append((fake.fake_op_memory(i, C.byref(n)), n.value))
+    names = [what for what, _, _ in _ops(fake)]
+    mallocs = [i for i, w in enumerate(names) if w == "cudaMalloc"]
+    work = max(mallocs, key=lambda i: mem[i][1])  # the largest by far: U and V of every leaf at 64 columns
+    launch = next(i for i in range(work, len(names)) if names[i] == "launch")
+    assert [i for i in range(work, launch) if names[i] == "cudaMemset" and mem[i] == mem[work]]
+    H.close()
