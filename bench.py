@@ -693,6 +693,23 @@ def profile_matmat(args):
     print(json.dumps({"profile_matmat": True, "stream_bytes": E.info["stream_bytes"]}), flush=True)
 
 
+def profile_solves(args):
+    """One pipelined and one BiCGSTAB solve on the C1 workload from a zero
+    guess, device vectors, nothing timed: the command the ncu summary of
+    k_bicg_steps and k_pipe_steps is taken from."""
+    import torch
+    from hacapk_b200 import configs
+    from hacapk_b200.engine import Engine
+    H, b_h = configs.c1(args.level)
+    E = Engine(H.st, H.nd)
+    b = torch.from_numpy(b_h).cuda()
+    out = {}
+    for name, solve in (("pipelined", E.bicgstab_pipe_dev), ("bicgstab", E.bicgstab_dev)):
+        u = torch.zeros_like(b)
+        out[name] = solve(b.data_ptr(), u.data_ptr(), tol=args.tol, max_iter=args.max_iter)["iterations"]
+    print(json.dumps({"profile_solves": out, "stream_bytes": E.info["stream_bytes"]}), flush=True)
+
+
 def cpu_baseline(H, b, args):
     """The compiled reference CPU H-matvec (HACApK_MAGMA.c:5-57, one thread as
     written) inside the BiCGSTAB of HACApK_SOLVER.c:254-417: one full solve."""
@@ -784,6 +801,8 @@ def main():
     ap.add_argument("--form", default="", help="with --forms-only: only this form (e.g. solvers_c1)")
     ap.add_argument("--profile-matmat", action="store_true",
                     help="only run five 64-RHS tensor-core products (a short command for ncu)")
+    ap.add_argument("--profile-solves", action="store_true",
+                    help="only run one pipelined and one BiCGSTAB solve on C1 (a short command for ncu)")
     ap.add_argument("--profile-products", type=int, default=0,
                     help="only run a few FP64/FP32/BF16 products on C2 at this level (a short command for ncu)")
     ap.add_argument("--precision-level", type=int, default=0,
@@ -791,6 +810,9 @@ def main():
     args = ap.parse_args()
     if args.profile_matmat:
         profile_matmat(args)
+        return
+    if args.profile_solves:
+        profile_solves(args)
         return
     if args.profile_products > 0:
         profile_products(args)
