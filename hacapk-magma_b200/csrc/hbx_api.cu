@@ -1629,8 +1629,9 @@ int hbx_bicgstab_multi(hbx_hmat *h, hbx_hmat *hm, const double *B, double *U, co
   }
   int outer = 0, launches = 1, steps = 0;
   for (;;) {
-    // R = B - H U, FP64: one product per right-hand side still running whose
-    // U is not zero (x0 = 0 makes the first residual B itself)
+    // R = B - H U, FP64: one product with all right-hand sides, or, where few
+    // still run, one for each whose U is not zero (x0 = 0 makes the first
+    // residual B itself)
     if ((st = norms(U)) != HBX_OK) return st;
     int products = 0;
     for (int j = 0; j < hbx::kNrhs; ++j) products += !done[j] && pin->norm[j] != 0.0;
@@ -1943,8 +1944,7 @@ static int batch_refined_dev(hbx_hmat *h, hbx_hmat *hl, const double *b, double 
   const size_t n = (size_t)h->plan.nd;
   if (!hl->d_refine) HBX_CUDA(dev_malloc(&hl->d_refine, 2 * n * sizeof(double)));
   double *r = hl->d_refine, *d = hl->d_refine + n;
-  // per-instance flags and inner tolerances (after the five per-instance
-  // doubles of h's batch scalars, a free tail is not guaranteed: own buffer)
+  // per-instance flags and inner tolerances
   if (!h->d_rflag) HBX_CUDA(dev_malloc(&h->d_rflag, (size_t)count * (sizeof(int) + sizeof(double)) + 16));
   int *d_flag = reinterpret_cast<int *>(h->d_rflag);
   double *d_itol = reinterpret_cast<double *>(reinterpret_cast<char *>(h->d_rflag) +

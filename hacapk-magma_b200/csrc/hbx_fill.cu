@@ -768,7 +768,10 @@ int hbx_fill_leaves(const double *xyz, int nond, const int *face2node, int nofc,
       // A leaf that stops in a column or row below the threshold goes on to read
       // the other vector of that term, which it never set.  New memory may hold
       // another allocation's words (NaN among them: non-finite factors in 4,097
-      // leaves of a 20,480-triangle sphere); cleared, the ranks are the host fill's.
+      // leaves of a 20,480-triangle sphere); cleared, the ranks of a first batch are
+      // the host fill's.  A later batch reads an earlier one's words there: of the
+      // 32,288 low-rank leaves of an 81,920-triangle sphere 26 differ from the host's in rank,
+      // with the same largest error.
       if (work_cap != held && (e = cudaMemset(d_work.p, 0, work_cap)) != cudaSuccess) return HBX_ERR_CUDA;
       cudaMemcpy(d_jobs.p, grouped.data(), grouped.size() * sizeof(AcaJob), cudaMemcpyHostToDevice);
       for (int c = kTeams - 1; c >= 0; --c) {  // the longest leaves start first

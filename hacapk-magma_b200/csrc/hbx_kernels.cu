@@ -915,7 +915,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_bicg_setup(BicgArgs a) {
 // a.steps, the warps that run ahead are told (rsum[4]) and woken: the producer
 // by one more emptied slot, the gather and block-sum warps by the signal of a
 // pass that does not follow, the grid-barrier warp by the block-sum warp.
-// HBM bounds the passes; the six barriers between them bound small matrices.
+// HBM bounds the passes; the seven barriers of a step bound small matrices.
 // Time of a step, one launch per step -> this: N = 320 27.3 -> 20.5 us, 1,280
 // 38.6 -> 31.1, 5,120 48.8 -> 41.8, 20,480 119 -> 109.5 (two passes of 265 MB
 // at 6.55 TB/s: 81).

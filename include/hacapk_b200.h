@@ -188,8 +188,10 @@ typedef struct hbx_solve_info {
   double true_relres;  /* ||b - H u|| / ||b|| recomputed after the solve      */
   double seconds;      /* device time from r0 = b - H u0 to the last step     */
   double iter_kernel_seconds; /* device time of the iteration launches only   */
-  int iter_launches;   /* steps the iteration kernels entered (includes the
-                          ones that only observe the end)                     */
+  int iter_launches;   /* BiCGSTAB: steps the kernel entered, with the one that
+                          observes the end; pipelined: its steps, or its step
+                          launches where a step is four; GCR: step launches;
+                          batched and multi-RHS: steps queued                  */
   int launches;        /* all kernel launches of the solve                    */
   int outer;           /* mixed-precision solve: refinement steps (FP64 residuals) */
   int reserved[5];
